@@ -29,7 +29,6 @@ constexpr int kLanes = 4;            // neighbour-list slots per chunk (nb_idx)
 constexpr int kLanesSR = 1;          // threads per particle in the SR pair kernel (lists of a few pairs)
 constexpr int kLanesLR = 4;          // threads per particle in the LR pair kernel
 constexpr int kThreadsLR = 512;      // threads per LR block (its kBlock particles in kBlock * 4 / 512 passes)
-constexpr int kIntPer = 1;           // particles per thread in the integrator
 
 // neighbour slot k of particle p: chunks of four slots per particle, chunk-major,
 // so the four threads of a particle read 16 contiguous bytes and a warp 128
@@ -54,6 +53,10 @@ struct RepParams {
     double kappa;                // inverse Debye length of the screened Coulomb term (0: unscreened, the reference)
     float kappaf;
     double mass[10], k1[10], k2[10], sigma[10], vcap[10];
+    int vcut[10];                // high word of sqrt(0.33 / vcap): smaller velocity components cannot reach the cap
+    float hf;                    // h in FP32
+    // floor(x qinv) by integers (fix_position): qinv 2^k in 64 bits, the high word of 2 L, and the shifts
+    struct { unsigned long long q; unsigned hi2l; int sh, fb; } qx[3];
     double k2fix[10], k2sig[10];  // K2 * 2^-32 (fixed-point force to velocity), K2 * sigma (noise)
     // pair tables, 1..45 (E:2908-2938); dm = D_LJ - 1.5852
     float dlj2[46], dm[46], flj[46], elj[46], d2min[46], qclb[46];

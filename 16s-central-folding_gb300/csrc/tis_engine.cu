@@ -370,7 +370,8 @@ int valid_replica(Group *h, int r)
 }  // namespace
 
 
-static int grp_create(const tis_system *const *systems, int n_replicas, const tis_run_params &prm, int base, Group **out)
+static int grp_create(const tis_system *const *systems, int n_replicas, const tis_run_params &prm, int base, int total_blocks,
+                      Group **out)
 {
     Group *h = new Group();
     h->prm = prm;
@@ -443,6 +444,18 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
             R.hbox[k] = 0.5 * L;
             R.qinv[k] = 4294967296.0 / L;
             R.qstep[k] = (float)(L / 4294967296.0);
+            {
+                int e2l, eq;  // 2 L < 2^e2l, qinv < 2^eq
+                std::frexp(2.0 * L, &e2l);
+                std::frexp(R.qinv[k], &eq);
+                uint64_t bits;
+                const double l2 = 2.0 * L;
+                memcpy(&bits, &l2, 8);
+                R.qx[k].q = (unsigned long long)std::ldexp(R.qinv[k], 64 - eq);
+                R.qx[k].hi2l = (unsigned)(bits >> 32);
+                R.qx[k].sh = 1022 + e2l;
+                R.qx[k].fb = 64 - eq - e2l - 1;
+            }
             R.mc[k] = (int)(L / (rc + prm.skin));  // E:1484-1490
             if (R.mc[k] < 1) return bail(fail(TIS_ERR_ARG, "replica %d: box smaller than the LR list radius", base + r));
             R.lcell[k] = L / R.mc[k];
@@ -460,6 +473,7 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
         R.lr_interval = prm.lr_interval;
         R.T = T;
         R.h = hstep;
+        R.hf = (float)hstep;
         R.lB = lB;
         R.kappa = (debye > 0.0 && std::isfinite(debye)) ? 1.0 / debye : 0.0;
         R.kappaf = (float)R.kappa;
@@ -480,6 +494,12 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
             R.k2[t] = (1.0 - R.k1[t]) / visc;
             R.sigma[t] = sqrt(2.0 * visc * T / hstep);
             R.vcap[t] = m / (300.0 * T);
+            {
+                const double vc = sqrt(0.33 / R.vcap[t]);
+                uint64_t bits;
+                memcpy(&bits, &vc, 8);
+                R.vcut[t] = (vc > 0 && std::isfinite(vc)) ? (int)(bits >> 32) : 0;
+            }
             R.k2fix[t] = R.k2[t] / tis::kFixScale;
             R.k2sig[t] = R.k2[t] * R.sigma[t];
         }
@@ -713,6 +733,7 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, prm.device);
         d.search_warps = std::max(4, sms * 4);  // one block of 4 warps per SM: rebuilds are rare
         d.sm_count = std::max(1, sms);
+        d.wide = total_blocks <= 4 * d.sm_count;
         int nc_max = 1;
         for (auto &Q : rp) nc_max = std::max(nc_max, Q.nc);
         d.nc_max = nc_max;
@@ -1627,11 +1648,14 @@ int tis_create(const tis_system *const *systems, int n_replicas, const tis_run_p
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming) != cudaSuccess)
         return bail(fail(TIS_ERR_CUDA, "cudaStreamCreate/cudaEventCreate failed"));
+    int total_blocks = 0;  // particle blocks of the whole handle
+    for (int r = 0; r < n_replicas; ++r)
+        if (systems[r]) total_blocks += (int)((scalar_i64(systems[r], "n_particles", 0) + tis::kBlock - 1) / tis::kBlock);
     for (int k = 0; k < G; ++k) {
         // replicas [first, last) in group k: sizes differ by at most one
         const int first = (int)((int64_t)n_replicas * k / G), last = (int)((int64_t)n_replicas * (k + 1) / G);
         Group *g = nullptr;
-        const int rc = grp_create(systems + first, last - first, prm, first, &g);
+        const int rc = grp_create(systems + first, last - first, prm, first, total_blocks, &g);
         if (rc) return bail(rc);
         h->groups.push_back(g);
         cudaEvent_t e;

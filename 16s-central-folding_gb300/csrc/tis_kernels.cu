@@ -626,13 +626,54 @@ __device__ inline double total_force(const Dev &d, int p, int c)
     return (double)t * (1.0 / kFixScale);
 }
 
+// (double)v by integer operations while v fits the 53 bits of a double's significand
+// (GB300 has 64-bit conversions and FP64 arithmetic at 1/64 of its integer rate)
+__device__ __forceinline__ double fix_to_double(long long v)
+{
+    const unsigned long long m = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
+    if (m >> 53) return (double)v;
+    const int z = __clzll((long long)m);  // 11 .. 64
+    unsigned long long b = ((m << z) << 1) >> 12;  // the significand below its leading one
+    b |= (unsigned long long)(unsigned)(1086 - z) << 52;
+    if (m == 0) b = 0;
+    return __longlong_as_double((long long)(b | ((unsigned long long)v & 0x8000000000000000ull)));
+}
+
+// floor(x qinv) modulo 2^32 of axis c, as __double2ll_rd(x * qinv[c]) gives it.  For
+// 0 <= x < 2 L by integers: X = x 2^(63 - B) (2 L <= 2^B) times qinv 2^k, of which the
+// high word has fb = k - B - 1 fraction bits (28 to 30).  It lies below the exact product
+// by less than 2^-26; the FP64 product is rounded by at most 2^-21, which can only move
+// its floor when the fraction lies within 2^-20 of one: those, and other x, take the FP64 form.
+__device__ __forceinline__ int fix_position(const RepParams *R, int c, double x)
+{
+    const int hi = __double2hiint(x);
+    if ((unsigned)hi < R->qx[c].hi2l) {
+        const int s = R->qx[c].sh - (hi >> 20);
+        const unsigned long long m = ((unsigned long long)(unsigned)((hi & 0xfffff) | 0x100000) << 32 | (unsigned)__double2loint(x)) << 10;
+        const unsigned long long v = __umul64hi(s < 64 ? m >> s : 0ull, R->qx[c].q);
+        const int fb = R->qx[c].fb;
+        const unsigned fr = (unsigned)v & ((1u << fb) - 1u);
+        if (fr < (1u << fb) - (1u << (fb - 20))) return (int)(unsigned)(v >> fb);
+    }
+    return (int)(unsigned)__double2ll_rd(x * R->qinv[c]);
+}
+
+// x as a float, its significand cut to 24 bits (0 below 2^-126, huge from 2^128 on)
+__device__ __forceinline__ float cut_to_float(double x)
+{
+    const int hi = __double2hiint(x), a = hi & 0x7fffffff;
+    const int f = __funnelshift_l((unsigned)__double2loint(x), (unsigned)(a - 0x38000000), 3);
+    const float m = a < 0x38100000 ? 0.0f : a >= 0x47f00000 ? 3.0e38f : __int_as_float(f);
+    return hi < 0 ? -m : m;
+}
+
 // leap_frog_move_atom (E:570-642) with the noise of full_forces (E:2612-2622).
 // FP64 mode follows the reference's operation order.  Mixed mode evaluates the
 // same update v' = K1 v + K2 (f + g sigma) as K1 v + (K2 2^-32) f_fix + (K2 sigma) g
 // with fused multiply-adds, and x' = x + (x - x_old) + (v' - v) h; the velocity
 // cap m v'^2 / (300 T) > 1 uses the precomputed m / (300 T) in both modes.
 template <bool D>
-__device__ inline void leap_frog(const Dev &d, const RepParams *R, int r, int p, double xn[3], double vn[3])
+__device__ inline void leap_frog(const Dev &d, const RepParams *R, int r, int p, double xn[3], double vn[3], float2 *e2 = nullptr)
 {
     const int t = d.q[p].w & 0xff;
     const double v0[3] = {d.vx[p], d.vy[p], d.vz[p]};
@@ -651,19 +692,38 @@ __device__ inline void leap_frog(const Dev &d, const RepParams *R, int r, int p,
         const double k1 = R->k1[t], kf = R->k2fix[t], kg = d.noise == 0 ? R->k2sig[t] : 0.0;
         for (int c = 0; c < 3; ++c) {
             const long long fx = (long long)(__ldcg(d.f + c * d.P + p) + __ldcg(d.flr + c * d.P + p));
-            vn[c] = fma(kg, g[k + 1000 * c], fma(kf, (double)fx, k1 * v0[c]));
+            vn[c] = fma(kg, g[k + 1000 * c], fma(kf, fix_to_double(fx), k1 * v0[c]));
         }
     }
-    double vsq = R->vcap[t] * (vn[0] * vn[0] + vn[1] * vn[1] + vn[2] * vn[2]);
-    if (vsq > 1.0) {
-        vsq = 1.0 / sqrt(vsq);
-        for (int c = 0; c < 3; ++c) vn[c] *= vsq;
+    // a component below sqrt(0.33 / vcap) each (vcut: that value's high word) cannot reach
+    // the cap; a runaway or NaN component has a larger high word and takes the FP64 test
+    const int hv = max(max(__double2hiint(vn[0]) & 0x7fffffff, __double2hiint(vn[1]) & 0x7fffffff),
+                       __double2hiint(vn[2]) & 0x7fffffff);
+    if (hv >= R->vcut[t]) {
+        double vsq = R->vcap[t] * (vn[0] * vn[0] + vn[1] * vn[1] + vn[2] * vn[2]);
+        if (vsq > 1.0) {
+            vsq = 1.0 / sqrt(vsq);
+            for (int c = 0; c < 3; ++c) vn[c] *= vsq;
+        }
     }
     if (D) {
         for (int c = 0; c < 3; ++c)
             xn[c] = __dadd_rn(__dsub_rn(__dmul_rn(2.0, x0[c]), o0[c]), __dmul_rn(__dsub_rn(vn[c], v0[c]), R->h));
     } else {
         for (int c = 0; c < 3; ++c) xn[c] = fma(vn[c] - v0[c], R->h, x0[c] + (x0[c] - o0[c]));
+    }
+    if (e2) {
+        // |x' - x|^2 in FP32, good to 1e-5 unless its two parts cancel (or it all but
+        // vanishes): then nothing (x) and an upper bound (y)
+        const float h = R->hf;
+        float s = 0.0f, parts = 0.0f;
+        for (int c = 0; c < 3; ++c) {
+            const float a = cut_to_float(x0[c] - o0[c]), b = cut_to_float(vn[c] - v0[c]) * h, e = a + b;
+            s += e * e;
+            parts += a * a + b * b;
+        }
+        const bool bad = s < 1.0e-30f || parts > 64.0f * s;
+        *e2 = make_float2(bad ? 0.0f : s, bad ? 2.1f * parts + 1.0e-30f : s);
     }
 }
 
@@ -1218,16 +1278,19 @@ __device__ void write_frame(const Dev &d, int r, long long klok, int tid, int nt
 
 // move_rigid_units for particle p of replica r (leap-frog, the recentring shift
 // sh, the ions' periodic wrap, the new fixed-point position, its force sum zeroed);
-// bits: max |x - x_old|^2 as bit pattern, err: flags
+// xn, xo: its new position and the old one, moved alike; est: leap_frog's estimate of
+// |xn - xo|^2.  False for a padding slot.
 template <bool D>
-__device__ __forceinline__ void integrate_particle(const Dev &d, const RepParams *R, int r, int p, const double sh[3],
-                                                   unsigned long long &bits, int &err)
+__device__ __forceinline__ bool move_particle(const Dev &d, const RepParams *R, int r, int p, const double sh[3],
+                                              double xn[3], double xo[3], float2 *est, int &err)
 {
     const int4 qp = d.q[p];
-    if (!((qp.w >> 16) & 1)) return;
-    double xn[3], vn[3];
-    leap_frog<D>(d, R, r, p, xn, vn);
-    double xo[3] = {d.x[p], d.y[p], d.z[p]};
+    if (!((qp.w >> 16) & 1)) return false;
+    double vn[3];
+    leap_frog<D>(d, R, r, p, xn, vn, est);
+    xo[0] = d.x[p];
+    xo[1] = d.y[p];
+    xo[2] = d.z[p];
     for (int c = 0; c < 3; ++c) {
         xn[c] = xn[c] + sh[c];
         xo[c] = xo[c] + sh[c];
@@ -1238,12 +1301,6 @@ __device__ __forceinline__ void integrate_particle(const Dev &d, const RepParams
             if (above(xn[c], R->box[c])) { xn[c] -= R->box[c]; xo[c] -= R->box[c]; }
         }
     }
-    double e2 = 0.0;
-    for (int c = 0; c < 3; ++c) {
-        const double e = xn[c] - xo[c];
-        e2 += e * e;
-    }
-    bits = max(bits, (unsigned long long)__double_as_longlong(e2));
     // a runaway or non-finite particle (|x| or |v| component >= 2^20) stops the run
     bool ok = true;
     for (int c = 0; c < 3; ++c) ok = ok && bounded(xn[c]) && bounded(vn[c]);
@@ -1254,49 +1311,66 @@ __device__ __forceinline__ void integrate_particle(const Dev &d, const RepParams
     d.f[p] = 0ull;  // consumed: the next step's force kernels accumulate from zero
     d.f[d.P + p] = 0ull;
     d.f[2 * d.P + p] = 0ull;
-    int4 q = qp;  // floor(x L / 2^32) modulo 2^32, one rounding conversion per axis
-    q.x = (int)(unsigned)__double2ll_rd(xn[0] * R->qinv[0]);
-    q.y = (int)(unsigned)__double2ll_rd(xn[1] * R->qinv[1]);
-    q.z = (int)(unsigned)__double2ll_rd(xn[2] * R->qinv[2]);
+    int4 q = qp;
+    q.x = fix_position(R, 0, xn[0]);
+    q.y = fix_position(R, 1, xn[1]);
+    q.z = fix_position(R, 2, xn[2]);
     d.q[p] = q;
+    return true;
 }
 
-// move_rigid_units (E:2660-2731) of one particle per thread: leap-frog, the
-// recentring shift, the periodic wrap of the ions; the replica's last block to
-// finish runs the skin check
-// kIntPer particles per thread, kBlock / kIntPer threads per block of kBlock particles
-template <bool D>
-__global__ void __launch_bounds__(kBlock / kIntPer) k_integrate(Dev d)
+// |xn - xo|^2 as a bit pattern (non-negative doubles order as integers)
+__device__ __forceinline__ unsigned long long shift_bits(const double xn[3], const double xo[3])
+{
+    double e2 = 0.0;
+    for (int c = 0; c < 3; ++c) {
+        const double e = xn[c] - xo[c];
+        e2 += e * e;
+    }
+    return (unsigned long long)__double_as_longlong(e2);
+}
+
+// move_rigid_units (E:2660-2731) of one particle per thread, T threads per block: leap-frog,
+// the recentring shift, the periodic wrap of the ions; the replica's last block to
+// finish runs the skin check.
+// Bound by the FP64 pipe (a warp instruction takes it 16 cycles or more, 64 issue slots):
+// everything but the update itself runs on integers or FP32.  Of the largest
+// displacement, which check_shifts needs exactly, an FP32 estimate finds the block's
+// candidates and only those form it in FP64.  Measured (one launch for all replicas): 64
+// replicas, 344,903 particles, 51.3 -> 38.9 us; 16 replicas, 782,384 particles, 96 -> 70 us.
+// Handles of few particles for the GPU (Dev::wide) take blocks of 64 threads, so that the
+// FP64 work spreads over more SMs; with more they would only add blocks to schedule.
+template <bool D, int T>
+__global__ void __launch_bounds__(T) k_integrate(Dev d)
 {
     wait_prior_grid();
-    const int r = d.blk_rep[blockIdx.x];
+    const int p = blockIdx.x * T + threadIdx.x;
+    const int r = d.blk_rep[blockIdx.x * T / kBlock];
     const RepParams *R = d.rp + r;
-    __shared__ unsigned long long s_max;
-    if (threadIdx.x == 0) s_max = 0ull;
+    __shared__ int s_est;
+    __shared__ int s_last;
+    if (threadIdx.x == 0) s_est = 0;
     __syncthreads();
     const double sh[3] = {d.shift[3 * r], d.shift[3 * r + 1], d.shift[3 * r + 2]};
-    unsigned long long bits = 0ull;  // max |x - x_old|^2 of the thread's particles (non-negative doubles order as integers)
     int err = 0;
-#pragma unroll
-    for (int j = 0; j < kIntPer; ++j)
-        integrate_particle<D>(d, R, r, blockIdx.x * kBlock + j * (kBlock / kIntPer) + threadIdx.x, sh, bits, err);
-    // check_shifts (E:1745-1762): max |x - x_old|^2 over the block
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long b = __shfl_down_sync(kFull, bits, o);
-        bits = b > bits ? b : bits;
-    }
-    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, bits);
+    float2 est = make_float2(0.0f, 0.0f);
+    double xn[3], xo[3];
+    const bool on = move_particle<D>(d, R, r, p, sh, xn, xo, &est, err);
+    // check_shifts (E:1745-1762): max |x - x_old|^2 over the block (a NaN estimate orders above all)
+    const int wm = __reduce_max_sync(kFull, on ? __float_as_int(est.x) & 0x7fffffff : 0);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_est, wm);
     __syncthreads();
-    __shared__ int s_last;
+    // within 512 units in the last place, 3e-5 to 6e-5, of the block's largest estimate
+    if (on && (__float_as_int(est.y) & 0x7fffffff) >= s_est - 512) atomicMax(&d.rs[r].maxd2, shift_bits(xn, xo));
+    if (err) atomicOr(&d.rs[r].err, err);
+    __syncthreads();
     if (threadIdx.x == 0) {
-        atomicMax(&d.rs[r].maxd2, s_max);
         __threadfence();
         // the replica's last block to finish runs the skin check for it
         const unsigned done = atomicAdd(&d.rs[r].blocks_done, 1u);
-        s_last = (done == (unsigned)(R->npad / kBlock) - 1u);
+        s_last = (done == (unsigned)(R->npad / T) - 1u);
         if (s_last) d.rs[r].blocks_done = 0u;
     }
-    if (err) atomicOr(&d.rs[r].err, err);
     __syncthreads();
     if (s_last) {
         __threadfence();
@@ -1317,17 +1391,21 @@ __device__ void control_step(const Dev &d, int r)
     const RepParams *R = d.rp + r;
     RepState *S = d.rs + r;
     if (threadIdx.x == 0) {
-        const double d2 = __longlong_as_double((long long)atomicExch(&S->maxd2, 0ull));
+        const double d2 = __longlong_as_double((long long)__ldcg(&S->maxd2));  // every block of the step has added its own
+        const long long kl = __ldcg(&S->klok) + 1;
+        const double e2 = __ldcg(&S->e2st_acc), e3 = __ldcg(&S->e3st_acc);
+        double progress = __ldcg(&S->progress);
         const double sh = sqrt(d2);
-        S->progress += (sh + sh);
-        S->klok += 1;
-        int reb = S->progress > R->skin;
-        if (reb) S->progress = 0.0;
+        progress += (sh + sh);
+        const int reb = progress > R->skin;
+        if (reb) progress = 0.0;
+        S->maxd2 = 0ull;
+        S->progress = progress;
+        S->klok = kl;
         S->rebuild = reb;
-        const long long kn = S->klok + 1;
-        S->lr_now = (R->lr_interval <= 1) || (kn % R->lr_interval == 1) || (S->progress == 0.0);
-        S->e2st = S->e2st_acc;  // stacking energies of the step just finished (E2_STACK, E3_STACK)
-        S->e3st = S->e3st_acc;
+        S->lr_now = (R->lr_interval <= 1) || ((kl + 1) % R->lr_interval == 1) || (progress == 0.0);
+        S->e2st = e2;  // stacking energies of the step just finished (E2_STACK, E3_STACK)
+        S->e3st = e3;
         S->e2st_acc = 0.0;
         S->e3st_acc = 0.0;
     }
@@ -1832,7 +1910,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_step_fused(Dev d, int step
             const double sh[3] = {s_shift[0], s_shift[1], s_shift[2]};
             unsigned long long bits = 0ull;
             const int i1 = min(npad, (rank + 1) * per);
-            for (int i = rank * per + tid; i < i1; i += kFusedThreads) integrate_particle<D>(d, R, r, p0 + i, sh, bits, err);
+            for (int i = rank * per + tid; i < i1; i += kFusedThreads) {
+                double xn[3], xo[3];
+                if (move_particle<D>(d, R, r, p0 + i, sh, xn, xo, nullptr, err)) bits = max(bits, shift_bits(xn, xo));
+            }
             for (int o = 16; o > 0; o >>= 1) {
                 const unsigned long long b = __shfl_down_sync(kFull, bits, o);
                 bits = b > bits ? b : bits;
@@ -2101,8 +2182,13 @@ void launch_shift(const Dev &d, cudaStream_t s)
 
 void launch_move(const Dev &d, cudaStream_t s)
 {
-    if (d.fp64) launch_pdl(k_integrate<true>, d.nblk, kBlock / kIntPer, 0, s, d);
-    else launch_pdl(k_integrate<false>, d.nblk, kBlock / kIntPer, 0, s, d);
+    if (d.wide) {
+        if (d.fp64) launch_pdl(k_integrate<true, 64>, d.P / 64, 64, 0, s, d);
+        else launch_pdl(k_integrate<false, 64>, d.P / 64, 64, 0, s, d);
+    } else {
+        if (d.fp64) launch_pdl(k_integrate<true, kBlock>, d.nblk, kBlock, 0, s, d);
+        else launch_pdl(k_integrate<false, kBlock>, d.nblk, kBlock, 0, s, d);
+    }
 }
 
 void launch_integrate(const Dev &d, cudaStream_t s)

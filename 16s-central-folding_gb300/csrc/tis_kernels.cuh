@@ -69,6 +69,7 @@ struct Dev {
     int cidx_max, cpos_max;         // largest per-replica ca_cidx and hb_cpos lengths
     int hb_smem;                // dynamic shared bytes of the H-bond kernel (0: its arrays stay in global scratch)
     double *eterm;              // R x kNE (per-term energies, compute_forces only)
+    int wide;                   // 1: few particles for the GPU: blocks of fewer particles each
     double *shift;              // R x 3, recentring shift of the current step (adjust_box)
     const int *cell_rep;        // replica of every cell
     int *hb_rec;                // when not null: 1 per H-bond candidate formed after the step's Monte Carlo, else 0
