@@ -658,6 +658,12 @@ __global__ void __launch_bounds__(kBlock) k_adj_record(Dev d, AdjDev a)
     }
     if (blockIdx.x == 0)
         for (int r = threadIdx.x; r < d.R; r += blockDim.x) a.rlr[r] = d.rs[r].lr_now;
+    // the step's Gaussians, from where its Monte Carlo left their start (RepState::pending)
+    for (int i = p; i < d.R * kNoise; i += gridDim.x * kBlock) {
+        const int r = i / kNoise;
+        const unsigned drawn = d.rs[r].pending ? d.rs[r].pending - 1u : 0u;
+        a.rg[i] = d.gnoise[(size_t)r * kNoiseStride + (drawn <= kNoiseSpare ? drawn : kNoise + kNoiseSpare) + i % kNoise];
+    }
 }
 
 // nine packed host-order arrays (replicas end to end, n values each) <-> nine

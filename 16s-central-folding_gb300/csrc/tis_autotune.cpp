@@ -157,9 +157,6 @@ extern "C" int tis_autotune(const tis_system *const *systems, int n_replicas, co
         if (g >= 1 && g <= n_replicas) groups.push_back(g);
     tune(&tis_run_params::groups, groups);
     tune(&tis_run_params::graph_steps, {25, 50, 100, 200});
-    tune(&tis_run_params::lanes_sr, {1, 2, 4});
-    tune(&tis_run_params::lanes_lr, {2, 4, 8});
-    tune(&tis_run_params::groups, groups);  // again: the best grouping moves with the launch shapes
     tune(&tis_run_params::fused_ctas, {0, 1, 2, 4});
     *best = p;
     if (rate) *rate = cur;

@@ -17,6 +17,12 @@ namespace tis {
 
 constexpr int kBlock = 128;          // particles per block; replicas are padded to it
 constexpr int kNoise = 3000;         // shared Gaussians per step (E:2598)
+// Gaussians of one replica in memory: those of the step and kNoiseSpare more, made beside
+// the H-bond Monte Carlo that decides where in them the step's start, and a second place
+// for a step whose Monte Carlo draws more than kNoiseSpare numbers
+constexpr int kNoiseSpare = 128;
+constexpr int kNoiseStride = 2 * kNoise + kNoiseSpare;
+constexpr int kForceThreads = 512;   // threads of a force block
 constexpr int kNE = 11;              // energies vector (tis_energy_index)
 constexpr double kSig0 = 1.5852;     // LJ length scale (E:749-821)
 constexpr double kFixScale = 4294967296.0;   // 2^32 fixed-point units per kcal/mol/A
@@ -26,9 +32,6 @@ constexpr int kExcl = 8;             // bonded (1-2, 1-3) partners stored per pa
 constexpr int kExclShift = 30;       // SR list entry: partner | (exclusion multiplicity << 30)
 constexpr int kIdxMask = (1 << kExclShift) - 1;
 constexpr int kLanes = 4;            // neighbour-list slots per chunk (nb_idx)
-constexpr int kLanesSR = 1;          // threads per particle in the SR pair kernel (lists of a few pairs)
-constexpr int kLanesLR = 4;          // threads per particle in the LR pair kernel
-constexpr int kThreadsLR = 512;      // threads per LR block (its kBlock particles in kBlock * 4 / 512 passes)
 
 // neighbour slot k of particle p: chunks of four slots per particle, chunk-major,
 // so the four threads of a particle read 16 contiguous bytes and a warp 128
@@ -78,7 +81,7 @@ struct RepState {
     double e2hb, e3hb, e2st, e3st;
     double e2st_acc, e3st_acc;   // stacking energies being summed in the current step
     unsigned blocks_done;        // integrator blocks finished this step (the last one runs the skin check)
-    unsigned pad_;
+    unsigned pending;            // 1 + the Monte Carlo draws of the step in flight, which control_step books with its Gaussians (0: none)
 };
 
 // ---- Philox-4x32-10 (Salmon et al., SC'11) --------------------------------
@@ -158,7 +161,8 @@ __host__ __device__ inline int pick_index(uint32_t v, int n)
 // Monte Carlo (E:2290-2300).  Decided in FP32 when u lies outside a margin around the
 // FP32 estimate that covers its rounding (relative 1e-6 + 4e-7 |x|); else in FP64 as
 // written.  Identical to the FP64 test for every input.
-__device__ inline bool accept_move(uint32_t v, double ea, double eb, double T, float inv_t)
+template <class E>
+__device__ inline bool accept_move(uint32_t v, E ea, E eb, double T, float inv_t)
 {
     const float x = (float)(ea - eb) * inv_t;
     const float ef = expf(x);
@@ -166,7 +170,7 @@ __device__ inline bool accept_move(uint32_t v, double ea, double eb, double T, f
     const float m = 1.0e-6f + 4.0e-7f * fabsf(x);
     if (uf < ef * (1.0f - m)) return true;
     if (uf > ef * (1.0f + m)) return false;
-    return u31_ratio(v) < exp((ea - eb) / T);
+    return u31_ratio(v) < exp(((double)ea - (double)eb) / T);
 }
 
 // sqrt(-2 ln u) for u = v / (2^31-1), accurate in FP32 over the whole range.
@@ -180,22 +184,29 @@ __device__ inline float bm_radius(uint32_t v)
 }
 
 // ---- fixed point ----------------------------------------------------------
-// round(v * 2^32) as int64 from 32-bit conversions only (64-bit conversions run
-// on GB300's narrow FP64 pipe).  For |v| < 0.5 the product fits int32 and is
-// rounded to nearest; for |v| >= 0.5, v is a multiple of 2^-24, so the split
-// v = floor(v) + frac is exact and frac * 2^32 is an exact integer below 2^32.
-// The result equals __float2ll_rn(v * 2^32) for every |v| < kFixLimit.
+// round(v * 2^32) as int64 from 32-bit operations only (64-bit conversions run on
+// GB300's narrow FP64 pipe), equal to __float2ll_rn(v * 2^32) for every |v| < kFixLimit.
+// Below 2^21 without a branch: adding and subtracting 1.5 x 2^23 leaves the nearest
+// integer h (ties to even), v - h is exact and at most 1/2 in size, and (v - h) 2^32
+// rounds to an int32; only v - h = +1/2 exactly gives 2^31, which saturates to INT_MAX,
+// a value no other FP32 product reaches, and gets its missing unit back.  From 2^21 on
+// the split floor + fraction is exact.
 __device__ inline long long to_fix(float v, int &err)
 {
-    if (!(fabsf(v) < kFixLimit)) {
-        if (v != v) { err |= kErrNonFinite; return 0; }
-        err |= kErrNonFinite;
-        v = v > 0 ? kFixLimit : -kFixLimit;
+    if (!(fabsf(v) < 2097152.0f)) {
+        if (!(fabsf(v) < kFixLimit)) {
+            err |= kErrNonFinite;
+            if (v != v) return 0;
+            v = v > 0 ? kFixLimit : -kFixLimit;
+        }
+        const float hi = floorf(v);
+        const unsigned lo = __float2uint_rz((v - hi) * kFixScaleF);
+        return (long long)((unsigned long long)(long long)__float2int_rz(hi) << 32) + (long long)lo;
     }
-    if (fabsf(v) < 0.5f) return (long long)__float2int_rn(v * kFixScaleF);
-    const float hi = floorf(v);
-    const unsigned lo = __float2uint_rz((v - hi) * kFixScaleF);
-    return (long long)((unsigned long long)(long long)__float2int_rz(hi) << 32) + (long long)lo;
+    const float t = v + 12582912.0f;
+    const int hi = __float_as_int(t) - 0x4b400000;
+    const int lo = __float2int_rn((v - (t - 12582912.0f)) * kFixScaleF);
+    return (long long)((unsigned long long)(long long)hi << 32) + (long long)lo + (lo == 0x7fffffff ? 1 : 0);
 }
 
 __device__ inline void atomic_add_fix(unsigned long long *a, long long v)

@@ -109,8 +109,6 @@ struct Group {
     int R = 0, P = 0, C = 0, nblk = 0;
     tis_run_params prm{};
     cudaStream_t stream = nullptr;
-    cudaStream_t side[3] = {nullptr, nullptr, nullptr};  // concurrent force branches
-    cudaEvent_t fork = nullptr, join[3] = {nullptr, nullptr, nullptr};
     std::vector<void *> owned;
     std::vector<RepHost> rep;
     tis::Dev dev{};
@@ -143,11 +141,6 @@ struct Group {
         for (void *p : owned) cudaFree(p);
         if (h_rs) cudaFreeHost(h_rs);
         if (h_peaks) cudaFreeHost(h_peaks);
-        for (int k = 0; k < 3; ++k) {
-            if (side[k]) cudaStreamDestroy(side[k]);
-            if (join[k]) cudaEventDestroy(join[k]);
-        }
-        if (fork) cudaEventDestroy(fork);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -303,9 +296,6 @@ int populate(Group *h)
     }
 }
 
-// deterministic_forces_MPI (E:2524-2586): the four force kernels are independent
-// (fixed-point atomics into one sum, the LR sum kept apart), so they run as
-// concurrent branches joined before the integrator
 // in-step profiling (tis_profile_in_step): an event recorded on s before stage k of
 // the step being captured (begin) or after it; no-op otherwise.  Event pair k of a
 // step sits at pev[2 * (step * TIS_N_STAGES + k)].
@@ -318,44 +308,31 @@ void mark(Group *h, cudaStream_t s, int k, bool begin)
                              cudaEventRecordExternal);
 }
 
+// deterministic_forces_MPI (E:2524-2586) in one launch: fixed-point atomics into one sum, the
+// LR sum kept apart.  make_noise: the step's Gaussians and recentring shifts too (launch_move
+// follows)
 void enqueue_forces(Group *h, bool make_noise)
 {
-    cudaEventRecord(h->fork, h->stream);
-    for (int k = 0; k < 3; ++k) cudaStreamWaitEvent(h->side[k], h->fork, 0);
-    mark(h, h->side[0], 1, true);
-    tis::launch_pair_lr(h->dev, h->side[0], false, false);
-    mark(h, h->side[0], 1, false);
-    mark(h, h->side[1], 2, true);
-    tis::launch_topology(h->dev, h->side[1], 4 | 8, false, false, true);
-    mark(h, h->side[1], 2, false);
-    mark(h, h->side[2], 3, true);
-    tis::launch_topology(h->dev, h->side[2], 16, false, make_noise, true);
-    mark(h, h->side[2], 3, false);
     mark(h, h->stream, 0, true);
-    tis::launch_pair_sr(h->dev, h->stream, false, true);
+    tis::launch_forces(h->dev, h->stream, make_noise, make_noise);
     mark(h, h->stream, 0, false);
-    for (int k = 0; k < 3; ++k) {
-        cudaEventRecord(h->join[k], h->side[k]);
-        cudaStreamWaitEvent(h->stream, h->join[k], 0);
-    }
 }
 
 void enqueue_step(Group *h)
 {
-    enqueue_forces(h, true);                   // the H-bond kernel also draws full_forces' Gaussians
+    enqueue_forces(h, true);
     if (!h->pev) {
-        tis::launch_integrate(h->dev, h->stream);  // recentring shift; last block per replica: skin check
+        tis::launch_move(h->dev, h->stream);  // last block per replica: skin check
         tis::launch_rebuild(h->dev, h->stream);
         return;
     }
-    // the same four launches with events between them (their programmatic
-    // dependent launch then waits for the event nodes like a plain dependency)
-    void (*chain[4])(const tis::Dev &, cudaStream_t) = {tis::launch_shift, tis::launch_move, tis::launch_cells,
-                                                         tis::launch_search};
-    for (int k = 0; k < 4; ++k) {
-        mark(h, h->stream, 4 + k, true);
+    // the same launches with events between them (their programmatic dependent launch
+    // then waits for the event nodes like a plain dependency)
+    void (*chain[3])(const tis::Dev &, cudaStream_t) = {tis::launch_move, tis::launch_cells, tis::launch_search};
+    for (int k = 0; k < 3; ++k) {
+        mark(h, h->stream, 5 + k, true);
         chain[k](h->dev, h->stream);
-        mark(h, h->stream, 4 + k, false);
+        mark(h, h->stream, 5 + k, false);
     }
     ++h->pev_next;
 }
@@ -383,12 +360,6 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
     };
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess)
         return bail(fail(TIS_ERR_CUDA, "cudaStreamCreate failed"));
-    for (int k = 0; k < 3; ++k)
-        if (cudaStreamCreateWithFlags(&h->side[k], cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&h->join[k], cudaEventDisableTiming) != cudaSuccess)
-            return bail(fail(TIS_ERR_CUDA, "cudaStreamCreate/cudaEventCreate failed"));
-    if (cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming) != cudaSuccess)
-        return bail(fail(TIS_ERR_CUDA, "cudaEventCreate failed"));
 
     std::vector<tis::RepParams> rp(n_replicas);
     std::vector<int> code, blk_rep, rep_of, cell_rep;
@@ -723,8 +694,6 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
     d.C = h->C;
     d.fp64 = prm.precision == TIS_PREC_FP64;
     d.full_lists = prm.full_lists ? 1 : 0;
-    d.lanes_sr = prm.lanes_sr;
-    d.lanes_lr = prm.lanes_lr;
     d.noise = prm.noise;
     d.cap_sr = cap_sr;
     d.cap_lr = cap_lr;
@@ -770,7 +739,7 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
     for (int c = 0; c < 9; ++c)
         if ((rc = dupload(O, sd[c], st[c]))) return bail(rc);
     if ((rc = dalloc(O, &d.f, 3 * (size_t)h->P)) || (rc = dalloc(O, &d.flr, 3 * (size_t)h->P)) ||
-        (rc = dalloc(O, &d.gnoise, (size_t)h->R * tis::kNoise)) || (rc = dalloc(O, &d.cell_of, h->P)) ||
+        (rc = dalloc(O, &d.gnoise, (size_t)h->R * tis::kNoiseStride)) || (rc = dalloc(O, &d.force_blocks, 1)) || (rc = dalloc(O, &d.cell_of, h->P)) ||
         (rc = dalloc(O, &d.cell_count, h->C)) || (rc = dalloc(O, &d.cell_start, h->C)) ||
         (rc = dalloc(O, &d.cell_fill, h->C)) || (rc = dalloc(O, &d.cell_list, h->P)) || (rc = dalloc(O, &d.qs, h->P)) ||
         (rc = dalloc(O, &d.n_sr, h->P)) || (rc = dalloc(O, &d.n_lr, h->P)) ||
@@ -828,7 +797,7 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
         (rc = dalloc(O, &d.hb_active, nhb)) || (rc = dalloc(O, &d.ca_exc, ca_list.size())) ||
         (rc = dalloc(O, &d.hb_K, (size_t)kscr)) || (rc = dalloc(O, &d.hb_A, ca_list.size())) ||
         (rc = dalloc(O, &d.hb_energy, nhb)) || (rc = dalloc(O, &d.hb_code, nhb)) ||
-        (rc = dalloc(O, &d.hb_term, 6 * nhb)) || (rc = dalloc(O, &d.hb_br, 3 * nhb)))
+        (rc = dalloc(O, &d.hb_term, 6 * nhb)))
         return bail(rc);
     {  // the Monte Carlo's views of the candidates: per over-valence atom its candidates, per candidate its such atoms
         std::vector<int> ca_pos(nhba, -1), ca_coff{0}, ca_cidx, hb_coff{0}, hb_cpos;
@@ -866,7 +835,7 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
         d.k_nmax = k_nmax;
         d.cidx_max = cidx_max;
         d.cpos_max = cpos_max;
-        const size_t smem = tis::hb_layout(hb_nmax, ca_nmax, k_nmax, cidx_max, cpos_max).total;
+        const size_t smem = tis::hb_layout(hb_nmax, ca_nmax, k_nmax, cidx_max, cpos_max, d.fp64 != 0).total;
         d.hb_smem = smem <= 160 * 1024 ? (int)smem : 0;
     }
     if (tis::configure_kernels(d) != 0) return bail(fail(TIS_ERR_CUDA, "cudaFuncSetAttribute failed"));
@@ -1034,9 +1003,9 @@ static int grp_compute_forces(Group *h, int r, int mask, double *forces, double 
     const tis::Dev &d = h->dev;
     TIS_CUDA(cudaMemsetAsync(d.eterm, 0, sizeof(double) * h->R * tis::kNE, h->stream));
     TIS_CUDA(cudaMemsetAsync(d.f, 0, sizeof(unsigned long long) * 3 * h->P, h->stream));
-    if (mask & TIS_TERM_SR) tis::launch_pair_sr(d, h->stream, true, false);
-    if (mask & TIS_TERM_LR) tis::launch_pair_lr(d, h->stream, true, true);
-    else TIS_CUDA(cudaMemsetAsync(d.flr, 0, sizeof(unsigned long long) * 3 * h->P, h->stream));
+    const int m_sr = mask & TIS_TERM_SR ? 1 : 0, m_lr = mask & TIS_TERM_LR ? 2 : 0;
+    if (m_sr || m_lr) tis::launch_pair(d, h->stream, true, false, m_sr, m_lr);
+    if (!m_lr) TIS_CUDA(cudaMemsetAsync(d.flr, 0, sizeof(unsigned long long) * 3 * h->P, h->stream));
     const int tmask = (mask & TIS_TERM_BONDED ? 4 : 0) | (mask & TIS_TERM_STACK ? 8 : 0) | (mask & TIS_TERM_HB ? 16 : 0);
     if (tmask) tis::launch_topology(d, h->stream, tmask, true, false, false);
     tis::launch_rg(d, h->stream, r, h->d_scalar);
@@ -1257,13 +1226,12 @@ static int grp_traj_grad(Group *h, int64_t steps, int K, const double *const *se
             h->dev.hb_rec = aj.rhb;
             enqueue_forces(h, true);
             h->dev.hb_rec = nullptr;
-            TIS_CUDA(cudaMemcpyAsync(aj.rg, d.gnoise, sizeof(double) * R * tis::kNoise, cudaMemcpyDeviceToDevice, h->stream));
             TIS_CUDA(cudaMemcpyAsync(dj.n_sr, d.n_sr, 4 * P, cudaMemcpyDeviceToDevice, h->stream));
             TIS_CUDA(cudaMemcpyAsync(dj.n_lr, d.n_lr, 4 * P, cudaMemcpyDeviceToDevice, h->stream));
             TIS_CUDA(cudaMemcpyAsync(dj.nbr_sr, d.nbr_sr, 4 * (size_t)d.cap_sr * P, cudaMemcpyDeviceToDevice, h->stream));
             TIS_CUDA(cudaMemcpyAsync(dj.nbr_lr, d.nbr_lr, 4 * (size_t)d.cap_lr * P, cudaMemcpyDeviceToDevice, h->stream));
             tis::launch_adj_record(d, aj, h->stream);
-            tis::launch_integrate(d, h->stream);
+            tis::launch_move(d, h->stream);
             tis::launch_rebuild(d, h->stream);
         }
         for (int j = len - 1; j >= 0; --j) {
@@ -1402,9 +1370,9 @@ static int grp_profile_stages(Group *h, int64_t n, double *ms)
     const tis::Dev &d = h->dev;
     for (int64_t s = 0; s < n; ++s) {
         TIS_CUDA(cudaEventRecord(ev[0], h->stream));
-        tis::launch_pair_sr(d, h->stream, false, true);
+        tis::launch_pair(d, h->stream, false, true, 1, 0);
         TIS_CUDA(cudaEventRecord(ev[1], h->stream));
-        tis::launch_pair_lr(d, h->stream, false, false);
+        tis::launch_pair(d, h->stream, false, true, 0, 1);
         TIS_CUDA(cudaEventRecord(ev[2], h->stream));
         tis::launch_topology(d, h->stream, 4 | 8, false, false, true);
         TIS_CUDA(cudaEventRecord(ev[3], h->stream));
@@ -1623,8 +1591,8 @@ int tis_create(const tis_system *const *systems, int n_replicas, const tis_run_p
     if (prm.groups < 0) return fail(TIS_ERR_ARG, "tis_create: negative group count");
     if (prm.fused_ctas < 0 || prm.fused_ctas > 8)
         return fail(TIS_ERR_ARG, "tis_create: fused_ctas %d is not 0 .. 8", prm.fused_ctas);
-    if (prm.lanes_sr == 0) prm.lanes_sr = tis::kLanesSR;
-    if (prm.lanes_lr == 0) prm.lanes_lr = tis::kLanesLR;
+    if (prm.lanes_sr == 0) prm.lanes_sr = 1;
+    if (prm.lanes_lr == 0) prm.lanes_lr = 4;
     if (prm.lanes_sr != 1 && prm.lanes_sr != 2 && prm.lanes_sr != 4)
         return fail(TIS_ERR_ARG, "tis_create: lanes_sr %d is not 1, 2 or 4", prm.lanes_sr);
     if (prm.lanes_lr != 2 && prm.lanes_lr != 4 && prm.lanes_lr != 8)
@@ -2396,6 +2364,7 @@ int tis_profile_in_step(tis_handle *h, int32_t steps, double *ms)
             for (size_t gi = 0; gi < G && !rc; ++gi)
                 for (int st = 0; st < steps; ++st) {
                     float t = 0;
+                    if (k >= 1 && k <= 4) continue;  // inside the force launch (stage 0)
                     const size_t b = gi * n_ev + 2 * ((size_t)st * TIS_N_STAGES + k);
                     const cudaError_t e = cudaEventElapsedTime(&t, ev[b], ev[b + 1]);
                     if (e != cudaSuccess) {

@@ -1,12 +1,12 @@
 // CUDA kernels of the TIS-RNA Langevin step for sm_103a.
 //
 // One step of every replica (E: = src/16SCD_Mg_Cl_K_COPY_fast.cpp):
-//   k_pair_sr     SR_interactions_lists      E:1783-1847   per particle, full neighbour list
-//   k_pair_lr     LR_interactions_lists      E:1851-1907   every lr_interval steps or after a rebuild
-//   k_bonded_stack polymer_constraints      E:2354-2520   one thread per term, all replicas
-//                  stacking_interactions    E:1911-2141
-//   k_hbond       hydrogen_bonds_interactions E:2145-2350  one block per replica:
-//                 energies, valence-limited MC, forces; full_forces' Gaussians E:2590-2611
+//   k_forces      deterministic_forces_MPI   E:2524-2586   every force of a replica group:
+//                 pair tasks (SR_interactions_lists E:1783-1847; LR_interactions_lists
+//                 E:1851-1907 every lr_interval steps or after a rebuild), bonded terms
+//                 (polymer_constraints E:2354-2520), stacks by term (E:1911-2141), H-bonds of
+//                 a replica per block with the valence-limited Monte Carlo (E:2145-2350),
+//                 full_forces' Gaussians (E:2590-2611), adjust_box's shift (E:2632-2656)
 //   k_integrate   full_forces (application) + move_rigid_units + leap_frog_move_atom + adjust_box
 //                                             E:2612-2732, E:570-642; its last block per
 //                 replica runs check_shifts      E:1741-1776
@@ -129,17 +129,72 @@ __device__ Real<D> dihedral_of(const Pos<D> &P, int i1, int i2, int i3, int i4)
     return atan2_(dot(v1, n) * sqrt_(dot(v2, v2)), dot(m, n));
 }
 
+// The geometry of a term, from which its value and its force follow; a term's thread
+// keeps it in registers while the other terms of its restraint are summed.
+template <bool D>
+struct BondGeom {
+    V3<Real<D>> v;
+    Real<D> r;
+};
+template <bool D>
+struct AngleGeom {
+    V3<Real<D>> a, b, w;
+    Real<D> aa, bb, ab, ww, th;
+};
+template <bool D>
+struct DihedralGeom {
+    V3<Real<D>> m, n;
+    Real<D> mm, nn, l2, p, q, psi;
+};
+
+template <bool D>
+__device__ __forceinline__ BondGeom<D> bond_geom(const Pos<D> &P, int i1, int i2)
+{
+    const V3<Real<D>> v = P.vec(i1, i2);
+    return {v, sqrt_(dot(v, v))};
+}
+
+template <bool D>
+__device__ __forceinline__ AngleGeom<D> angle_geom(const Pos<D> &P, int i1, int i2, int i3)
+{
+    AngleGeom<D> g;
+    g.a = P.vec(i2, i1);
+    g.b = P.vec(i2, i3);
+    g.aa = dot(g.a, g.a);
+    g.bb = dot(g.b, g.b);
+    g.ab = dot(g.a, g.b);
+    g.w = cross(g.a, g.b);
+    g.ww = sqrt_(dot(g.w, g.w));
+    g.th = atan2_(g.ww, g.ab);
+    return g;
+}
+
+template <bool D>
+__device__ __forceinline__ DihedralGeom<D> dihedral_geom(const Pos<D> &P, int i1, int i2, int i3, int i4)
+{
+    DihedralGeom<D> g;
+    const V3<Real<D>> v1 = P.vec(i1, i2), v2 = P.vec(i2, i3), v3 = P.vec(i3, i4);
+    g.m = cross(v1, v2);
+    g.n = cross(v2, v3);
+    g.mm = dot(g.m, g.m);
+    g.nn = dot(g.n, g.n);
+    const Real<D> v22 = dot(v2, v2);
+    g.l2 = sqrt_(v22);
+    g.psi = atan2_(dot(v1, g.n) * g.l2, dot(g.m, g.n));
+    g.p = dot(v1, v2) / v22;
+    g.q = dot(v3, v2) / v22;
+    return g;
+}
+
 // harmonic bond k0 (r0 - r)^2 (bead_bond_force / stacking_bond_force, E:924-982)
 template <bool D>
-__device__ void bond_force(const Pos<D> &P, Acc<D> &A, int i1, int i2, Real<D> k0, Real<D> r0)
+__device__ __forceinline__ void bond_apply(const BondGeom<D> &g, Acc<D> &A, int i1, int i2, Real<D> k0, Real<D> r0)
 {
     using R = Real<D>;
-    V3<R> v = P.vec(i1, i2);
-    R r = sqrt_(dot(v, v));
-    R t = R(2) * k0 * (r0 - r) / r;
-    V3<R> g = t * v;
-    A.add(i1, R(-1) * g);
-    A.add(i2, g);
+    const R t = R(2) * k0 * (r0 - g.r) / g.r;
+    const V3<R> f = t * g.v;
+    A.add(i1, R(-1) * f);
+    A.add(i2, f);
 }
 
 // harmonic angle k0 (theta0 - theta)^2 at i2 (bead_valence_force E:1031-1134;
@@ -149,19 +204,15 @@ __device__ void bond_force(const Pos<D> &P, Acc<D> &A, int i1, int i2, Real<D> k
 // with d theta/dx1 = a x w / (|a|^2 |w|), d theta/dx3 = -b x w / (|b|^2 |w|),
 // w = a x b, which keeps FP32 accurate where sin theta is small.
 template <bool D>
-__device__ void angle_force(const Pos<D> &P, Acc<D> &A, int i1, int i2, int i3, Real<D> k0, Real<D> th0, bool clamp)
+__device__ __forceinline__ void angle_apply(const AngleGeom<D> &g, Acc<D> &A, int i1, int i2, int i3, Real<D> k0,
+                                            Real<D> th0, bool clamp)
 {
     using R = Real<D>;
-    V3<R> a = P.vec(i2, i1), b = P.vec(i2, i3);
-    const R aa = dot(a, a), bb = dot(b, b), ab = dot(a, b);
-    if (clamp && ab * rsqrt_(aa * bb) < R(-0.99995)) return;  // theta = pi, no force
-    const V3<R> w = cross(a, b);
-    const R ww = sqrt_(dot(w, w));
-    if (ww == R(0)) return;
-    const R th = atan2_(ww, ab);
-    const R s = R(2) * k0 * (th0 - th) / ww;
-    const V3<R> g1 = (s / aa) * cross(a, w);
-    const V3<R> g3 = (-s / bb) * cross(b, w);
+    if (clamp && g.ab * rsqrt_(g.aa * g.bb) < R(-0.99995)) return;  // theta = pi, no force
+    if (g.ww == R(0)) return;
+    const R s = R(2) * k0 * (th0 - g.th) / g.ww;
+    const V3<R> g1 = (s / g.aa) * cross(g.a, g.w);
+    const V3<R> g3 = (-s / g.bb) * cross(g.b, g.w);
     A.add(i1, g1);
     A.add(i2, R(-1) * (g1 + g3));
     A.add(i3, g3);
@@ -174,25 +225,37 @@ __device__ void angle_force(const Pos<D> &P, Acc<D> &A, int i1, int i2, int i3, 
 // d psi/dx2 = -(1 + v1.v2/|v2|^2) d psi/dx1 + (v3.v2/|v2|^2) d psi/dx4,
 // which has no 1/sin psi and so no FP32 cancellation at planar (psi ~ 0, pi) geometry.
 template <bool D>
-__device__ void dihedral_force(const Pos<D> &P, Acc<D> &A, int i1, int i2, int i3, int i4, Real<D> k0,
-                               Real<D> psi0)
+__device__ __forceinline__ void dihedral_apply(const DihedralGeom<D> &g, Acc<D> &A, int i1, int i2, int i3, int i4,
+                                               Real<D> k0, Real<D> psi0)
 {
     using R = Real<D>;
-    const V3<R> v1 = P.vec(i1, i2), v2 = P.vec(i2, i3), v3 = P.vec(i3, i4);
-    const V3<R> m = cross(v1, v2), n = cross(v2, v3);
-    const R mm = dot(m, m), nn = dot(n, n), v22 = dot(v2, v2);
-    if (mm == R(0) || nn == R(0)) return;
-    const R l2 = sqrt_(v22);
-    const R psi = atan2_(dot(v1, n) * l2, dot(m, n));
-    const R c = R(2) * k0 * (psi0 - psi);
-    const V3<R> g1 = (-c * l2 / mm) * m;
-    const V3<R> g4 = (c * l2 / nn) * n;
-    const R p = dot(v1, v2) / v22, q = dot(v3, v2) / v22;
-    const V3<R> g2 = (R(-1) - p) * g1 + q * g4;
+    if (g.mm == R(0) || g.nn == R(0)) return;
+    const R c = R(2) * k0 * (psi0 - g.psi);
+    const V3<R> g1 = (-c * g.l2 / g.mm) * g.m;
+    const V3<R> g4 = (c * g.l2 / g.nn) * g.n;
+    const V3<R> g2 = (R(-1) - g.p) * g1 + g.q * g4;
     A.add(i1, g1);
     A.add(i2, g2);
     A.add(i3, R(-1) * (g1 + g2 + g4));
     A.add(i4, g4);
+}
+
+template <bool D>
+__device__ void bond_force(const Pos<D> &P, Acc<D> &A, int i1, int i2, Real<D> k0, Real<D> r0)
+{
+    bond_apply<D>(bond_geom<D>(P, i1, i2), A, i1, i2, k0, r0);
+}
+
+template <bool D>
+__device__ void angle_force(const Pos<D> &P, Acc<D> &A, int i1, int i2, int i3, Real<D> k0, Real<D> th0, bool clamp)
+{
+    angle_apply<D>(angle_geom<D>(P, i1, i2, i3), A, i1, i2, i3, k0, th0, clamp);
+}
+
+template <bool D>
+__device__ void dihedral_force(const Pos<D> &P, Acc<D> &A, int i1, int i2, int i3, int i4, Real<D> k0, Real<D> psi0)
+{
+    dihedral_apply<D>(dihedral_geom<D>(P, i1, i2, i3, i4), A, i1, i2, i3, i4, k0, psi0);
 }
 
 // native dihedral imaged to within pi of the current one (E:1999-2019): branch -1/0/+1
@@ -268,19 +331,19 @@ __device__ inline Real<D> six_term(const Pos<D> &P, const int *k, const double *
     return R(0.15) * dd * dd;
 }
 
-// force of term s of the six-term restraint (six_force's six calls, one at a time)
+// force of term s of the six-term restraint (six_force's six calls, one at a time); br:
+// the imaging branch of a dihedral
 template <bool D>
-__device__ inline void six_force_term(const Pos<D> &P, Acc<D> &A, const int *k, const double *nat, int code,
-                                      Real<D> w, int s)
+__device__ inline void six_force_term(const Pos<D> &P, Acc<D> &A, const int *k, const double *nat, int br, Real<D> w,
+                                      int s)
 {
     using R = Real<D>;
     if (s == 0) bond_force<D>(P, A, k[1], k[4], R(5) * w, (R)nat[0]);
     else if (s == 1) angle_force<D>(P, A, k[0], k[1], k[4], R(1.5) * w, (R)nat[1], true);
     else if (s == 2) angle_force<D>(P, A, k[3], k[4], k[1], R(1.5) * w, (R)nat[2], true);
-    else if (s == 3) dihedral_force<D>(P, A, k[0], k[1], k[4], k[3], R(0.15) * w, psi_shift<R>((R)nat[3], code % 3 - 1));
-    else if (s == 4)
-        dihedral_force<D>(P, A, k[4], k[1], k[0], k[2], R(0.15) * w, psi_shift<R>((R)nat[4], (code / 3) % 3 - 1));
-    else dihedral_force<D>(P, A, k[1], k[4], k[3], k[5], R(0.15) * w, psi_shift<R>((R)nat[5], code / 9 - 1));
+    else if (s == 3) dihedral_force<D>(P, A, k[0], k[1], k[4], k[3], R(0.15) * w, psi_shift<R>((R)nat[3], br));
+    else if (s == 4) dihedral_force<D>(P, A, k[4], k[1], k[0], k[2], R(0.15) * w, psi_shift<R>((R)nat[4], br));
+    else dihedral_force<D>(P, A, k[1], k[4], k[3], k[5], R(0.15) * w, psi_shift<R>((R)nat[5], br));
 }
 
 template <bool D>
@@ -384,196 +447,164 @@ struct PairTables {
     const float *dlj2, *dm, *flj, *qclb;
 };
 
+// The force of one list entry (partner j, packed position qj, ljw: the weight of its LJ
+// term) on the particle p of type tp: mixed precision, added to (ax, ay, az) in fixed
+// point.  An LR entry (LR known, or lr set) is farther than any LJ range and charged.
+template <bool LR, bool EN>
+__device__ __forceinline__ void pair_entry(const Dev &d, const RepParams *R, int p, const int4 &qp, int tp, bool chp,
+                                           int j, const int4 &qj, float ljw, const PairTables &tb, float kap, float lo,
+                                           float hi, long long &ax, long long &ay, long long &az, int &err,
+                                           double &e_lj, double &e_c)
+{
+    const float dx = (float)(int)((unsigned)qp.x - (unsigned)qj.x) * R->qstep[0];
+    const float dy = (float)(int)((unsigned)qp.y - (unsigned)qj.y) * R->qstep[1];
+    const float dz = (float)(int)((unsigned)qp.z - (unsigned)qj.z) * R->qstep[2];
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    const int tj = qj.w & 0xff, kj = (qj.w >> 8) & 0xff;
+    const int J = jn12(tp, tj);
+    const bool lj = !LR && ljw != 0.0f && r2 <= tb.dlj2[J];
+    bool cou = (LR || (chp && is_charged(kj))) && r2 <= hi;
+    if (cou && !(r2 <= lo)) cou = exact_r2(d, R, p, j) <= R->rc2;
+    if (!lj && !cou) return;
+    const float rr = sqrtf(r2);
+    float F = 0.0f;
+    if (lj) {  // LJ_FORCE (E:801-821)
+        const float dr = rr - tb.dm[J];
+        const float s = 1.5852f / dr;
+        const float s2 = s * s, s4 = s2 * s2, s8 = s4 * s4, s14 = s8 * s4 * s2;
+        F = ljw * (tb.flj[J] * (s14 - s8) * dr / rr);
+        if (EN) {
+            double e;
+            if ((double)r2 < R->d2min_d[J]) e = R->elj_d[J] * 1001.0;
+            else {
+                const float s6 = s4 * s2, s12 = s6 * s6;
+                e = (double)(R->elj[J] * (s12 - 2.0f * s6 + 1.0f));
+            }
+            e_lj += 0.5 * (double)ljw * e;
+        }
+    }
+    if (cou) {  // COULOMB_TRUNCATED_FORCE (E:841-855)
+        if (kap == 0.0f) {
+            F += tb.qclb[J] / (r2 * rr);
+            if (EN) e_c += 0.5 * (double)(tb.qclb[J] / rr);
+        } else {  // screened: U = C exp(-kappa r) / r, F / r = U (1 + kappa r) / r^2
+            const float kr = kap * rr, u = tb.qclb[J] * expf(-kr) / rr;
+            F += u * (1.0f + kr) / r2;
+            if (EN) e_c += 0.5 * (double)u;
+        }
+    }
+    if (F != 0.0f) {
+        ax += to_fix(F * dx, err);
+        ay += to_fix(F * dy, err);
+        az += to_fix(F * dz, err);
+    }
+}
+
+// the same entry in FP64, from the FP64 positions with the reference's image rule
+template <bool LR, bool EN>
+__device__ __forceinline__ void pair_entry(const Dev &d, const RepParams *R, int p, int tp, bool chp, int j, int wj,
+                                           double ljw, double &ax, double &ay, double &az, double &e_lj, double &e_c)
+{
+    const int tj = wj & 0xff, kj = (wj >> 8) & 0xff;
+    const int J = jn12(tp, tj);
+    double v[3];
+    exact_vec(d, R, p, j, v);
+    const double r2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
+    const bool lj = !LR && ljw != 0.0 && r2 <= R->dlj2_d[J];
+    const bool cou = (LR || (chp && is_charged(kj))) && r2 <= R->rc2;
+    if (!lj && !cou) return;
+    const double rr = sqrt(r2);
+    double F = 0.0;
+    if (lj) {
+        const double dr = rr + kSig0 - R->dlj_d[J];
+        const double s = kSig0 / dr;
+        const double s2 = s * s, s4 = s2 * s2, s8 = s4 * s4, s14 = s8 * s4 * s2;
+        F = ljw * (R->flj_d[J] * (s14 - s8) * dr / rr);
+        if (EN) {
+            double e;
+            if (r2 < R->d2min_d[J]) e = R->elj_d[J] * 1001.0;
+            else {
+                const double s6 = s4 * s2, s12 = s6 * s6;
+                e = R->elj_d[J] * (s12 - 2.0 * s6 + 1.0);
+            }
+            e_lj += 0.5 * ljw * e;
+        }
+    }
+    if (cou) {
+        if (R->kappa == 0.0) {
+            F += R->qclb_d[J] / (rr * r2);
+            if (EN) e_c += 0.5 * R->qclb_d[J] / rr;
+        } else {
+            const double kr = R->kappa * rr, u = R->qclb_d[J] * exp(-kr) / rr;
+            F += u * (1.0 + kr) / r2;
+            if (EN) e_c += 0.5 * u;
+        }
+    }
+    ax += v[0] * F;
+    ay += v[1] * F;
+    az += v[2] * F;
+}
+
 // The pair forces of particle p over its full list, by L threads (lane4 = its lane
 // among them): slot k of the list goes to lane k % L; lane 0 adds the sum (LR: stores
-// the held LR force).  err, e_lj, e_c accumulate per thread.
-template <bool D, bool LR, bool EN, bool EX, int L, bool CO>
+// the held LR force).  The persistent fused step kernel's form; the separate kernel
+// takes a block's list entries as tasks (k_pair).
+template <bool D, bool LR, int L>
 __device__ __forceinline__ void pair_particle(const Dev &d, const RepParams *R, int p, int lane4, const PairTables &tb,
-                                              int &err, double &e_lj, double &e_c)
+                                              int &err)
 {
     const int P = d.P;
     const int4 qp = d.q[p];
-    const int tp = qp.w & 0xff, kp = (qp.w >> 8) & 0xff, act = (qp.w >> 16) & 1;
-    const bool chp = is_charged(kp);
+    const int tp = qp.w & 0xff, act = (qp.w >> 16) & 1;
+    const bool chp = is_charged((qp.w >> 8) & 0xff);
     const int cnt = act ? (LR ? d.n_lr[p] : d.n_sr[p]) : 0;
     const int *nbr = LR ? d.nbr_lr : d.nbr_sr;
-    if (!D) {
-        long long ax = 0, ay = 0, az = 0;
-        const float sx = R->qstep[0], sy = R->qstep[1], sz = R->qstep[2];
-        const float rc2 = R->rc2f, lo = rc2 * (1.0f - kBand), hi = rc2 * (1.0f + kBand);
-        const float kap = R->kappaf;
-        for (int k = lane4; k < cnt; k += L) {
-            const int raw = ld_in<CO>(nbr + nb_idx(k, p, P));
-            const int j = raw & kIdxMask;
-            const float ljw = EX ? (float)(1 - (raw >> kExclShift)) : 1.0f;
-            const int4 qj = ld_in<CO>(d.q + j);
-            const float dx = (float)(int)((unsigned)qp.x - (unsigned)qj.x) * sx;
-            const float dy = (float)(int)((unsigned)qp.y - (unsigned)qj.y) * sy;
-            const float dz = (float)(int)((unsigned)qp.z - (unsigned)qj.z) * sz;
-            const float r2 = dx * dx + dy * dy + dz * dz;
-            const int tj = qj.w & 0xff, kj = (qj.w >> 8) & 0xff;
-            const int J = jn12(tp, tj);
-            float F = 0.0f;
-            if (!LR && ljw != 0.0f && r2 <= tb.dlj2[J]) {  // LJ_FORCE (E:801-821)
-                const float rr = sqrtf(r2);
-                const float dr = rr - tb.dm[J];
-                const float s = 1.5852f / dr;
-                const float s2 = s * s, s4 = s2 * s2, s8 = s4 * s4, s14 = s8 * s4 * s2;
-                F = ljw * (tb.flj[J] * (s14 - s8) * dr / rr);
-                if (EN) {
-                    double e;
-                    if ((double)r2 < R->d2min_d[J]) e = R->elj_d[J] * 1001.0;
-                    else {
-                        const float s6 = s4 * s2, s12 = s6 * s6;
-                        e = (double)(R->elj[J] * (s12 - 2.0f * s6 + 1.0f));
-                    }
-                    e_lj += 0.5 * (double)ljw * e;
-                }
-            }
-            if ((LR || (chp && is_charged(kj))) && r2 <= hi) {  // COULOMB_TRUNCATED_FORCE (E:841-855)
-                bool in = r2 <= lo || exact_r2(d, R, p, j) <= R->rc2;
-                if (in) {
-                    const float rr = sqrtf(r2);
-                    if (kap == 0.0f) {
-                        F += tb.qclb[J] / (r2 * rr);
-                        if (EN) e_c += 0.5 * (double)(tb.qclb[J] / rr);
-                    } else {  // screened: U = C exp(-kappa r) / r, F / r = U (1 + kappa r) / r^2
-                        const float kr = kap * rr, u = tb.qclb[J] * expf(-kr) / rr;
-                        F += u * (1.0f + kr) / r2;
-                        if (EN) e_c += 0.5 * (double)u;
-                    }
-                }
-            }
-            if (F != 0.0f) {
-                ax += to_fix(F * dx, err);
-                ay += to_fix(F * dy, err);
-                az += to_fix(F * dz, err);
-            }
+    double e0 = 0, e1 = 0;
+    typename std::conditional<D, double, long long>::type ax = 0, ay = 0, az = 0;
+    const float lo = R->rc2f * (1.0f - kBand), hi = R->rc2f * (1.0f + kBand);
+    const float kap = R->kappaf;
+    for (int k = lane4; k < cnt; k += L) {
+        const int raw = ld_in<true>(nbr + nb_idx(k, p, P));
+        const int j = raw & kIdxMask;
+        if constexpr (!D) {
+            const float ljw = LR ? 1.0f : (float)(1 - (raw >> kExclShift));
+            pair_entry<LR, false>(d, R, p, qp, tp, chp, j, ld_in<true>(d.q + j), ljw, tb, kap, lo, hi, ax, ay, az, err,
+                                  e0, e1);
+        } else {
+            const double ljw = LR ? 1.0 : (double)(1 - (raw >> kExclShift));
+            pair_entry<LR, false>(d, R, p, tp, chp, j, d.q[j].w, ljw, ax, ay, az, e0, e1);
         }
-        for (int o = 1; o < L; o <<= 1) {
-            ax += __shfl_xor_sync(kFull, ax, o);
-            ay += __shfl_xor_sync(kFull, ay, o);
-            az += __shfl_xor_sync(kFull, az, o);
-        }
-        if (lane4 == 0) {
-            if (LR) {  // the LR force is kept for the MTS interval: overwrite
-                d.flr[p] = (unsigned long long)ax;
-                d.flr[P + p] = (unsigned long long)ay;
-                d.flr[2 * P + p] = (unsigned long long)az;
-            } else if (act) {  // other force kernels run concurrently: accumulate
-                atomic_add_fix(d.f + p, ax);
-                atomic_add_fix(d.f + P + p, ay);
-                atomic_add_fix(d.f + 2 * P + p, az);
-            }
+    }
+    for (int o = 1; o < L; o <<= 1) {
+        ax += __shfl_xor_sync(kFull, ax, o);
+        ay += __shfl_xor_sync(kFull, ay, o);
+        az += __shfl_xor_sync(kFull, az, o);
+    }
+    if (lane4 != 0) return;
+    if constexpr (!D) {
+        if (LR) {  // the LR force is kept for the MTS interval: overwrite
+            d.flr[p] = (unsigned long long)ax;
+            d.flr[P + p] = (unsigned long long)ay;
+            d.flr[2 * P + p] = (unsigned long long)az;
+        } else if (act) {  // other force kernels run concurrently: accumulate
+            atomic_add_fix(d.f + p, ax);
+            atomic_add_fix(d.f + P + p, ay);
+            atomic_add_fix(d.f + 2 * P + p, az);
         }
     } else {
-        double ax = 0, ay = 0, az = 0;
-        for (int k = lane4; k < cnt; k += L) {
-            const int raw = ld_in<CO>(nbr + nb_idx(k, p, P));
-            const int j = raw & kIdxMask;
-            const double ljw = EX ? (double)(1 - (raw >> kExclShift)) : 1.0;
-            const int tj = d.q[j].w & 0xff, kj = (d.q[j].w >> 8) & 0xff;
-            const int J = jn12(tp, tj);
-            double v[3];
-            exact_vec(d, R, p, j, v);
-            const double r2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
-            double F = 0.0;
-            if (!LR && ljw != 0.0 && r2 <= R->dlj2_d[J]) {
-                const double rr = sqrt(r2);
-                const double dr = rr + kSig0 - R->dlj_d[J];
-                const double s = kSig0 / dr;
-                const double s2 = s * s, s4 = s2 * s2, s8 = s4 * s4, s14 = s8 * s4 * s2;
-                F = ljw * (R->flj_d[J] * (s14 - s8) * dr / rr);
-                if (EN) {
-                    double e;
-                    if (r2 < R->d2min_d[J]) e = R->elj_d[J] * 1001.0;
-                    else {
-                        const double s6 = s4 * s2, s12 = s6 * s6;
-                        e = R->elj_d[J] * (s12 - 2.0 * s6 + 1.0);
-                    }
-                    e_lj += 0.5 * ljw * e;
-                }
-            }
-            if ((LR || (chp && is_charged(kj))) && r2 <= R->rc2) {
-                const double rr = sqrt(r2);
-                if (R->kappa == 0.0) {
-                    F += R->qclb_d[J] / (rr * r2);
-                    if (EN) e_c += 0.5 * R->qclb_d[J] / rr;
-                } else {
-                    const double kr = R->kappa * rr, u = R->qclb_d[J] * exp(-kr) / rr;
-                    F += u * (1.0 + kr) / r2;
-                    if (EN) e_c += 0.5 * u;
-                }
-            }
-            ax += v[0] * F;
-            ay += v[1] * F;
-            az += v[2] * F;
-        }
-        for (int o = 1; o < L; o <<= 1) {
-            ax += __shfl_xor_sync(kFull, ax, o);
-            ay += __shfl_xor_sync(kFull, ay, o);
-            az += __shfl_xor_sync(kFull, az, o);
-        }
-        if (lane4 == 0) {
-            if (LR) {
-                double *out = (double *)d.flr;
-                out[p] = ax;
-                out[P + p] = ay;
-                out[2 * P + p] = az;
-            } else if (act) {
-                double *out = (double *)d.f;
-                atomicAdd(out + p, ax);
-                atomicAdd(out + P + p, ay);
-                atomicAdd(out + 2 * P + p, az);
-            }
+        double *out = LR ? (double *)d.flr : (double *)d.f;
+        if (LR) {
+            out[p] = ax;
+            out[P + p] = ay;
+            out[2 * P + p] = az;
+        } else if (act) {
+            atomicAdd(out + p, ax);
+            atomicAdd(out + P + p, ay);
+            atomicAdd(out + 2 * P + p, az);
         }
     }
 }
 
-// Particle block b (kBlock particles) by T threads, L per particle: slot k of a
-// particle's list goes to its thread k % L; the block's particles in kBlock L / T passes.
-template <bool D, bool LR, bool EN, bool EX, int L, int T>
-__device__ void pair_block(const Dev &d, int b, int force_all)
-{
-    const int r = d.blk_rep[b];
-    const RepParams *R = d.rp + r;
-    if (LR && !force_all && !d.rs[r].lr_now) return;
-    __shared__ float s_dlj2[46], s_dm[46], s_flj[46], s_qclb[46];
-    if (!D) {
-        for (int t = threadIdx.x; t < 46; t += blockDim.x) {
-            s_dlj2[t] = R->dlj2[t];
-            s_dm[t] = R->dm[t];
-            s_flj[t] = R->flj[t];
-            s_qclb[t] = R->qclb[t];
-        }
-        __syncthreads();
-    }
-    const PairTables tb{s_dlj2, s_dm, s_flj, s_qclb};
-    const int lane4 = threadIdx.x & (L - 1);
-    int err = 0;
-    double e_lj = 0, e_c = 0;
-    constexpr int kPasses = kBlock * L / T;
-#pragma unroll
-    for (int pass = 0; pass < kPasses; ++pass) {
-        const int p = b * kBlock + pass * (T / L) + (int)threadIdx.x / L;
-        pair_particle<D, LR, EN, EX, L, false>(d, R, p, lane4, tb, err, e_lj, e_c);
-    }
-    if (EN) {
-        if (!LR) atomicAdd(d.eterm + r * kNE + 0, e_lj);
-        atomicAdd(d.eterm + r * kNE + (LR ? 2 : 1), e_c);
-    }
-    if (err) atomicOr(&d.rs[r].err, err);
-}
-
-template <bool D, bool LR, bool EN, bool EX, int L, int T>
-__global__ void __launch_bounds__(T) k_pair(Dev d, int force_all)
-{
-    pair_block<D, LR, EN, EX, L, T>(d, blockIdx.x, force_all);
-}
-
-// ---------------------------------------------------------------------------
-// block reductions
-// ---------------------------------------------------------------------------
 // barriers of the threads that run a block-level part: the whole CTA, or warps
 // 0 .. n/32-1 of it on a named barrier (the fused step kernel's H-bond warps)
 struct CtaBar {
@@ -584,6 +615,194 @@ struct NamedBar {
     __device__ void operator()() const { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 };
 
+
+constexpr int kPairTasks = 512;  // tasks of a sub-block held in shared memory at a time
+
+template <int PB>
+struct PairSmem {
+    float dlj2[46], dm[46], flj[46], qclb[46];
+    int4 q[PB];          // packed positions of the particles
+    int4 at[PB];         // places of a particle's tasks: first full chunk, remainders (SR | LR << 16); its SR and LR entries
+    int4 cnt[PB / 32];   // per 32 particles: tasks of a full chunk, of 3, 2, 1 entries
+    int task[kPairTasks];
+};
+
+// Pair forces of PB particles (sub-block pb) by the TS threads of one sub-block, over
+// their SR lists and, where the LR force is due (do_lr: 0 never, 1 when
+// RepState::lr_now is set, 2 always), their LR lists.
+//
+// The lists are short and uneven (2.9 SR entries on average, 0 to 40), so a thread per
+// particle ran a warp as long as its longest list, one dependent load after another.
+// Here the sub-block's list entries are cut into tasks of one list chunk (four entries,
+// 16 bytes) for one thread: full chunks first, then those with 3, 2 and 1 entries, so the
+// threads of a warp do equal work and a task's four partner positions are loaded
+// together.  FP64 tasks hold one entry: FP64 latency and the narrow FP64 pipe bound them.
+// Alone, SR lists of 5 replicas of a 346-nt chain: 22.3 -> 11.9 us; one 76-nt replica in
+// FP64: 52 -> 15 us.
+template <bool D, bool EN, bool EX, int PB, int TS, class Bar>
+__device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int do_lr, int tid, PairSmem<PB> &sm, Bar bar)
+{
+    constexpr int U = D ? 1 : 4, UL = D ? 0 : 2;  // entries per task, its logarithm
+    constexpr int kW = PB / 32;
+    static_assert(TS >= PB, "a thread per particle");
+    const int p0 = pb * PB, r = d.blk_rep[p0 / kBlock], P = d.P;
+    const RepParams *R = d.rp + r;
+    const bool lr = do_lr == 2 || (do_lr == 1 && d.rs[r].lr_now);
+    if (!do_sr && !lr) return;
+    if (!D)
+        for (int t = tid; t < 46; t += TS) {
+            sm.dlj2[t] = R->dlj2[t];
+            sm.dm[t] = R->dm[t];
+            sm.flj[t] = R->flj[t];
+            sm.qclb[t] = R->qclb[t];
+        }
+    const PairTables tb{sm.dlj2, sm.dm, sm.flj, sm.qclb};
+    const int lane = tid & 31;
+    if (tid < PB) {
+        const int p = p0 + tid;
+        const int4 qp = d.q[p];
+        sm.q[tid] = qp;
+        const bool act = (qp.w >> 16) & 1;
+        const int ns = act && do_sr ? d.n_sr[p] : 0, nl = act && lr ? d.n_lr[p] : 0;
+        if (lr)  // the LR force is kept for the MTS interval: started again here, its tasks add to it
+            for (int c = 0; c < 3; ++c) d.flr[c * P + p] = 0ull;  // FP64 mode: 0.0 has the same bits
+        const int full = (ns >> UL) + (nl >> UL);
+        int incl = full;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += t;
+        }
+        const unsigned lt = (1u << lane) - 1u;
+        int c[3] = {0, 0, 0}, as = 0, al = 0;
+        if (U > 1)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const unsigned ms = __ballot_sync(kFull, (ns & 3) == 3 - k), ml = __ballot_sync(kFull, (nl & 3) == 3 - k);
+                c[k] = __popc(ms) + __popc(ml);
+                if ((ns & 3) == 3 - k) as = __popc(ms & lt);
+                if ((nl & 3) == 3 - k) al = __popc(ms) + __popc(ml & lt);
+            }
+        sm.at[tid] = make_int4(incl - full, as | (al << 16), ns, nl);
+        if (lane == 31) sm.cnt[tid >> 5] = make_int4(incl, c[0], c[1], c[2]);
+    }
+    bar();
+    int total = 0;
+#pragma unroll
+    for (int v = 0; v < kW; ++v) total += sm.cnt[v].x + sm.cnt[v].y + sm.cnt[v].z + sm.cnt[v].w;
+    int err = 0;
+    double e_lj = 0, e_c = 0, e_cl = 0;
+    for (int win = 0; win < total; win += kPairTasks) {
+        if (win) bar();  // the previous window's tasks are done
+        if (tid < PB) {
+            int4 first = make_int4(-win, -win, -win, -win);  // first task of each class of this particle's 32
+#pragma unroll
+            for (int v = 0; v < kW; ++v) {
+                const int4 n = sm.cnt[v];
+                const bool lower = v < (tid >> 5);
+                first.x += lower ? n.x : 0;
+                first.y += n.x + (lower ? n.y : 0);
+                first.z += n.x + n.y + (lower ? n.z : 0);
+                first.w += n.x + n.y + n.z + (lower ? n.w : 0);
+            }
+            const int4 at = sm.at[tid];
+            const int ns = at.z, nl = at.w;
+            int to = first.x + at.x;
+            for (int k = 0; k < (ns >> UL); ++k, ++to)
+                if ((unsigned)to < (unsigned)kPairTasks) sm.task[to] = tid | ((U - 1) << 8) | (k << 10);
+            for (int k = 0; k < (nl >> UL); ++k, ++to)
+                if ((unsigned)to < (unsigned)kPairTasks) sm.task[to] = tid | (1 << 7) | ((U - 1) << 8) | (k << 10);
+            if (U > 1) {
+                const int rs = ns & 3, rl = nl & 3;
+                to = (rs == 3 ? first.y : rs == 2 ? first.z : first.w) + (at.y & 0xffff);
+                if (rs && (unsigned)to < (unsigned)kPairTasks) sm.task[to] = tid | ((rs - 1) << 8) | ((ns >> 2) << 10);
+                to = (rl == 3 ? first.y : rl == 2 ? first.z : first.w) + (at.y >> 16);
+                if (rl && (unsigned)to < (unsigned)kPairTasks)
+                    sm.task[to] = tid | (1 << 7) | ((rl - 1) << 8) | ((nl >> 2) << 10);
+            }
+        }
+        bar();
+        const int nt = min(total - win, kPairTasks);
+        const float lo = R->rc2f * (1.0f - kBand), hi = R->rc2f * (1.0f + kBand);
+        const float kap = R->kappaf;
+        for (int t = tid; t < nt; t += TS) {
+            const int task = sm.task[t];
+            const int pl = task & 127, p = p0 + pl, cnt = ((task >> 8) & 3) + 1;
+            const bool tlr = (task >> 7) & 1;
+            const int *nbr = tlr ? d.nbr_lr : d.nbr_sr;
+            double ec = 0;
+            if constexpr (!D) {
+                const int4 e4 = __ldg((const int4 *)nbr + (size_t)(task >> 10) * P + p);
+                const int raw[4] = {e4.x, e4.y, e4.z, e4.w};
+                const int4 qp = sm.q[pl];
+                const int tp = qp.w & 0xff;
+                const bool chp = is_charged((qp.w >> 8) & 0xff);
+                long long ax = 0, ay = 0, az = 0;
+                int4 qj[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k < cnt) qj[k] = __ldg(d.q + (raw[k] & kIdxMask));
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (k < cnt) {
+                        const float ljw = EX ? (float)(1 - (raw[k] >> kExclShift)) : 1.0f;
+                        pair_entry<false, EN>(d, R, p, qp, tp, chp, raw[k] & kIdxMask, qj[k], ljw, tb, kap, lo, hi, ax,
+                                              ay, az, err, e_lj, ec);
+                    }
+                if (ax | ay | az) {
+                    unsigned long long *out = tlr ? d.flr : d.f;
+                    atomic_add_fix(out + p, ax);
+                    atomic_add_fix(out + P + p, ay);
+                    atomic_add_fix(out + 2 * P + p, az);
+                }
+            } else {
+                const int raw = __ldg(nbr + nb_idx(task >> 10, p, P));
+                const int wp = sm.q[pl].w;
+                const double ljw = EX ? (double)(1 - (raw >> kExclShift)) : 1.0;
+                double ax = 0, ay = 0, az = 0;
+                pair_entry<false, EN>(d, R, p, wp & 0xff, is_charged((wp >> 8) & 0xff), raw & kIdxMask,
+                                      __ldg(&d.q[raw & kIdxMask].w), ljw, ax, ay, az, e_lj, ec);
+                if (ax != 0 || ay != 0 || az != 0) {
+                    double *out = (double *)(tlr ? d.flr : d.f);
+                    atomicAdd(out + p, ax);
+                    atomicAdd(out + P + p, ay);
+                    atomicAdd(out + 2 * P + p, az);
+                }
+            }
+            if (EN) {
+                if (tlr) e_cl += ec;
+                else e_c += ec;
+            }
+        }
+    }
+    if (EN) {
+        for (int o = 16; o > 0; o >>= 1) {
+            e_lj += __shfl_down_sync(kFull, e_lj, o);
+            e_c += __shfl_down_sync(kFull, e_c, o);
+            e_cl += __shfl_down_sync(kFull, e_cl, o);
+        }
+        if (lane == 0) {
+            if (do_sr) {
+                atomicAdd(d.eterm + r * kNE + 0, e_lj);
+                atomicAdd(d.eterm + r * kNE + 1, e_c);
+            }
+            if (lr) atomicAdd(d.eterm + r * kNE + 2, e_cl);
+        }
+    }
+    if (err) atomicOr(&d.rs[r].err, err);
+}
+
+// the pair forces alone (tis_compute_forces, stage timing)
+constexpr int kPairAlone = 128;
+template <bool D, bool EN, bool EX>
+__global__ void __launch_bounds__(kPairAlone) k_pair(Dev d, int do_sr, int do_lr)
+{
+    __shared__ PairSmem<32> sm;
+    pair_tasks<D, EN, EX, 32, kPairAlone>(d, blockIdx.x, do_sr, do_lr, (int)threadIdx.x, sm, CtaBar{});
+}
+
+// ---------------------------------------------------------------------------
+// block reductions
+// ---------------------------------------------------------------------------
 // sum of NV doubles over threads tid = 0 .. nthr-1 (a multiple of 32) into tid 0
 template <int NV, class Bar>
 __device__ void block_sum_t(double (&v)[NV], double *smem /* NV * 32 */, int tid, int nthr, Bar bar)
@@ -667,6 +886,13 @@ __device__ __forceinline__ float cut_to_float(double x)
     return hi < 0 ? -m : m;
 }
 
+// the step's 3000 Gaussians of replica r (RepState::pending)
+__device__ __forceinline__ const double *step_noise(const Dev &d, int r)
+{
+    const unsigned pending = __ldcg(&d.rs[r].pending), drawn = pending ? pending - 1u : 0u;  // written in this very kernel (k_forces)
+    return d.gnoise + (size_t)r * kNoiseStride + (drawn <= kNoiseSpare ? drawn : kNoise + kNoiseSpare);
+}
+
 // leap_frog_move_atom (E:570-642) with the noise of full_forces (E:2612-2622).
 // FP64 mode follows the reference's operation order.  Mixed mode evaluates the
 // same update v' = K1 v + K2 (f + g sigma) as K1 v + (K2 2^-32) f_fix + (K2 sigma) g
@@ -680,7 +906,7 @@ __device__ inline void leap_frog(const Dev &d, const RepParams *R, int r, int p,
     const double x0[3] = {d.x[p], d.y[p], d.z[p]};
     const double o0[3] = {d.xo[p], d.yo[p], d.zo[p]};
     const int k = (p - R->p0 + 1) % 1000;
-    const double *g = d.gnoise + r * kNoise;
+    const double *g = step_noise(d, r);
     if (D) {
         double f[3] = {total_force<D>(d, p, 0), total_force<D>(d, p, 1), total_force<D>(d, p, 2)};
         if (d.noise == 0) {
@@ -727,31 +953,33 @@ __device__ inline void leap_frog(const Dev &d, const RepParams *R, int r, int p,
     }
 }
 
-// full_forces' Gaussians (E:2594-2606) of one replica from draw c0 on, by the
-// threads of one block
+// the Gaussians of full_forces (E:2594-2606) made from draws c and c + 1
 template <bool D>
-__device__ void gen_noise(const Dev &d, int r, unsigned long long c0, int tid, int nthr)
+__device__ __forceinline__ void noise_pair(const RepParams *R, unsigned long long c, double *out)
 {
-    const RepParams *R = d.rp + r;
-    if (d.noise != 0) return;
-    for (int t = tid; t < kNoise / 2; t += nthr) {
-        const uint32_t v1 = rand_value(R->seed, c0 + 2 * t);
-        const uint32_t v2 = rand_value(R->seed, c0 + 2 * t + 1);
-        if (D) {  // Box-Muller as the reference forms it (E:2598-2606), in FP64
-            const double a = sqrt(-2.0 * log(u31_ratio(v1)));
-            const double b = 2.0 * 3.14159265358979323846 * u31_ratio(v2);
-            double sn, cs;
-            sincos(b, &sn, &cs);
-            d.gnoise[r * kNoise + 2 * t] = a * cs;
-            d.gnoise[r * kNoise + 2 * t + 1] = a * sn;
-        } else {  // FP32 Box-Muller, radius accurate over the whole uniform range
-            const float a = bm_radius(v1);
-            float sn, cs;
-            sincospif(2.0f * ((float)v2 * (1.0f / 2147483647.0f)), &sn, &cs);
-            d.gnoise[r * kNoise + 2 * t] = (double)(a * cs);
-            d.gnoise[r * kNoise + 2 * t + 1] = (double)(a * sn);
-        }
+    const uint32_t v1 = rand_value(R->seed, c), v2 = rand_value(R->seed, c + 1);
+    if (D) {  // Box-Muller as the reference forms it (E:2598-2606), in FP64
+        const double a = sqrt(-2.0 * log(u31_ratio(v1)));
+        const double b = 2.0 * 3.14159265358979323846 * u31_ratio(v2);
+        double sn, cs;
+        sincos(b, &sn, &cs);
+        out[0] = a * cs;
+        out[1] = a * sn;
+    } else {  // FP32 Box-Muller, radius accurate over the whole uniform range
+        const float a = bm_radius(v1);
+        float sn, cs;
+        sincospif(2.0f * ((float)v2 * (1.0f / 2147483647.0f)), &sn, &cs);
+        out[0] = (double)(a * cs);
+        out[1] = (double)(a * sn);
     }
+}
+
+// all Gaussians of one replica from draw c0 on, by the threads of one block
+template <bool D>
+__device__ void gen_noise(const Dev &d, int r, unsigned long long c0, double *out, int tid, int nthr)
+{
+    if (d.noise != 0) return;
+    for (int t = tid; t < kNoise / 2; t += nthr) noise_pair<D>(d.rp + r, c0 + 2 * t, out + 2 * t);
 }
 
 // the step's Gaussians alone (the drop-in full_forces call), one block per replica;
@@ -761,7 +989,7 @@ __global__ void k_noise(Dev d)
 {
     const int r = blockIdx.x;
     const unsigned long long c0 = d.rs[r].ctr;
-    gen_noise<D>(d, r, c0, (int)threadIdx.x, (int)blockDim.x);
+    gen_noise<D>(d, r, c0, d.gnoise + (size_t)r * kNoiseStride, (int)threadIdx.x, (int)blockDim.x);
     __syncthreads();
     if (threadIdx.x == 0) d.rs[r].ctr = c0 + kNoise;
 }
@@ -769,7 +997,6 @@ __global__ void k_noise(Dev d)
 // ---------------------------------------------------------------------------
 // bonded terms and stacks of every replica, one thread per term
 // ---------------------------------------------------------------------------
-constexpr int kTopoThreads = 256;
 
 // LJ force of an excluded (bonded) pair, as reduce_forces subtracts it (E:880-897)
 template <bool D, bool EN>
@@ -808,50 +1035,191 @@ __device__ void exclusion_lj(const Dev &d, const RepParams *R, const Pos<D> &P, 
     }
 }
 
-// polymer_constraints (E:2354-2520), then stacking_interactions (E:1911-2141):
-// items [0, nbt) are bonded terms, then tertiary stacks, then secondary stacks.
-// A secondary stack is off this step when a tertiary stack sharing one of its
-// sites (ST_EXCESS == 1) is within 10 A of its native distance (E:1960-1981);
-// each secondary stack checks the few tertiary stacks that can do that.
-// item t of the handle's bonded terms and stacks (above), by one thread
-template <bool D, bool EN>
-__device__ __forceinline__ void topo_item(const Dev &d, int t, int mask, int excl_in_list)
+template <bool D>
+__device__ __forceinline__ Acc<D> force_acc(const Dev &d)
 {
-    using Rl = Real<D>;
-    int r, kind;  // kind: 0 bonded, 1 tertiary, 2 secondary
-    int item;
-    if (t < d.nbt) { kind = 0; item = t; r = d.rep_of[d.bt_idx[t].x]; }
-    else if (t < d.nbt + d.nst3) { kind = 1; item = t - d.nbt; r = d.rep_of[d.st3_idx[6 * item]]; }
-    else if (t < d.nbt + d.nst3 + d.nst2) { kind = 2; item = t - d.nbt - d.nst3; r = d.rep_of[d.st2_idx[7 * item]]; }
-    else return;
-    if ((kind == 0 && !(mask & 4)) || (kind > 0 && !(mask & 8))) return;
-    const RepParams *R = d.rp + r;
-    const Pos<D> P = make_pos<D>(d, R);
     Acc<D> A;
     A.f = (decltype(A.f))d.f;
     A.P = d.P;
     A.err = 0;
+    return A;
+}
+
+// polymer_constraints (E:2354-2520): bonded term `item`, by one thread
+template <bool D, bool EN>
+__device__ __forceinline__ void bonded_item(const Dev &d, int item, int excl_in_list)
+{
+    using Rl = Real<D>;
+    const int4 id = d.bt_idx[item];
+    const double2 par = d.bt_par[item];
+    const int r = d.rep_of[id.x];
+    const RepParams *R = d.rp + r;
+    const Pos<D> P = make_pos<D>(d, R);
+    Acc<D> A = force_acc<D>(d);
     double e_excl = 0;
-    if (kind == 0) {
-        const int4 id = d.bt_idx[item];
-        const double2 par = d.bt_par[item];
-        const int ex = id.w == 0 ? id.y : id.z;  // excluded pair partner of id.x
-        if (id.w == 0) bond_force<D>(P, A, id.x, id.y, (Rl)par.x, (Rl)par.y);
-        else angle_force<D>(P, A, id.x, id.y, id.z, (Rl)par.x, (Rl)par.y, false);
-        if (!excl_in_list || EN) exclusion_lj<D, EN>(d, R, P, A, id.x, ex, e_excl);
-        if (EN) {
-            double *e = d.eterm + r * kNE;
-            if (id.w == 0) {
-                const Rl rr = distance<D>(P, id.x, id.y);
-                atomicAdd(e + 3, (double)((Rl)par.x * (rr - (Rl)par.y) * (rr - (Rl)par.y)));
-            } else {
-                const Rl th = angle_of<D>(P, id.x, id.y, id.z);
-                atomicAdd(e + 4, (double)((Rl)par.x * (th - (Rl)par.y) * (th - (Rl)par.y)));
-            }
-            if (e_excl != 0) atomicAdd(e + 5, e_excl);
+    const int ex = id.w == 0 ? id.y : id.z;  // excluded pair partner of id.x
+    if (id.w == 0) bond_force<D>(P, A, id.x, id.y, (Rl)par.x, (Rl)par.y);
+    else angle_force<D>(P, A, id.x, id.y, id.z, (Rl)par.x, (Rl)par.y, false);
+    if (!excl_in_list || EN) exclusion_lj<D, EN>(d, R, P, A, id.x, ex, e_excl);
+    if (EN) {
+        double *e = d.eterm + r * kNE;
+        if (id.w == 0) {
+            const Rl rr = distance<D>(P, id.x, id.y);
+            atomicAdd(e + 3, (double)((Rl)par.x * (rr - (Rl)par.y) * (rr - (Rl)par.y)));
+        } else {
+            const Rl th = angle_of<D>(P, id.x, id.y, id.z);
+            atomicAdd(e + 4, (double)((Rl)par.x * (th - (Rl)par.y) * (th - (Rl)par.y)));
         }
-    } else if (kind == 1) {
-        const int *id = d.st3_idx + 6 * item;
+        if (e_excl != 0) atomicAdd(e + 5, e_excl);
+    }
+    if (A.err) atomicOr(&d.rs[r].err, A.err);
+}
+
+// A secondary stack is off this step when a tertiary stack sharing one of its
+// sites (ST_EXCESS == 1) is within 10 A of its native distance (E:1960-1981);
+// each secondary stack checks the few tertiary stacks that can do that.
+template <bool D>
+__device__ __forceinline__ bool stack2_off(const Dev &d, const Pos<D> &P, int item)
+{
+    using Rl = Real<D>;
+    for (int u = d.st2_offby_off[item]; u < d.st2_offby_off[item + 1]; ++u) {
+        const int k = d.st2_offby_idx[u];
+        const int *tid = d.st3_idx + 6 * k;
+        if (distance<D>(P, tid[1], tid[4]) - (Rl)d.st3_nat[6 * k] < Rl(10)) return true;
+    }
+    return false;
+}
+
+// Stacks by term (stacking_interactions, E:1911-2141): a unit of 32 stacks is run by one
+// warp per term, lane = stack, so that the lanes of a warp evaluate the same kind of term
+// and the terms of a stack run side by side: value, exchange through q, force from the
+// geometry still in registers.  Measured against one thread per stack, which ran the terms
+// and then their forces one after another: 18.2 -> 9.8 us with the bonded terms (5 replicas
+// of a 346-nt chain, alone), 80 -> 19 us in FP64 (one 76-nt replica).
+// w: the warp's index in its unit (0 .. 7 tertiary: 0 distance, 1-2 angles, 3-5 dihedrals;
+// 0 .. 3 secondary: 0 distance, 1-2 dihedrals, 3 the switch); q: 8 (4) x 32 values.
+template <bool D, bool EN, class Bar>
+__device__ __forceinline__ void stack3_unit(const Dev &d, int unit, int w, int lane, Real<D> *q, Bar bar)
+{
+    using Rl = Real<D>;
+    const int item = unit * 32 + lane;
+    const bool on = item < d.nst3 && w < 6;
+    const int *id = d.st3_idx + 6 * item;
+    int r = 0;
+    BondGeom<D> gb;
+    AngleGeom<D> ga;
+    DihedralGeom<D> gd;
+    Rl nat = Rl(0), val = Rl(0);
+    Pos<D> P;
+    if (on) {
+        r = d.rep_of[id[0]];
+        P = make_pos<D>(d, d.rp + r);
+        nat = (Rl)d.st3_nat[6 * item + w];
+        if (w == 0) {
+            gb = bond_geom<D>(P, id[1], id[4]);
+            const Rl rdev = gb.r - nat;
+            val = Rl(5) * rdev * rdev;
+        } else if (w <= 2) {
+            ga = w == 1 ? angle_geom<D>(P, id[0], id[1], id[4]) : angle_geom<D>(P, id[3], id[4], id[1]);
+            val = Rl(1.5) * (ga.th - nat) * (ga.th - nat);
+        } else {
+            gd = w == 3 ? dihedral_geom<D>(P, id[0], id[1], id[4], id[3])
+                        : w == 4 ? dihedral_geom<D>(P, id[4], id[1], id[0], id[2])
+                                 : dihedral_geom<D>(P, id[1], id[4], id[3], id[5]);
+            nat = psi_shift<Rl>(nat, psi_branch<Rl>(gd.psi, nat));
+            val = Rl(0.15) * (gd.psi - nat) * (gd.psi - nat);
+        }
+        q[w * 32 + lane] = val;
+    }
+    bar();
+    if (on) {
+        Rl Dn = Rl(1);
+        for (int s = 0; s < 6; ++s) Dn += q[s * 32 + lane];
+        const Rl E = (Rl)d.st3_E[item] / Dn, wt = -E / Dn;
+        Acc<D> A = force_acc<D>(d);
+        if (w == 0) {
+            bond_apply<D>(gb, A, id[1], id[4], Rl(5) * wt, nat);
+            d.st_energy[item] = (double)E;
+            atomicAdd(EN ? d.eterm + r * kNE + 7 : &d.rs[r].e3st_acc, (double)E);
+        } else if (w == 1) {
+            angle_apply<D>(ga, A, id[0], id[1], id[4], Rl(1.5) * wt, nat, true);
+        } else if (w == 2) {
+            angle_apply<D>(ga, A, id[3], id[4], id[1], Rl(1.5) * wt, nat, true);
+        } else if (w == 3) {
+            dihedral_apply<D>(gd, A, id[0], id[1], id[4], id[3], Rl(0.15) * wt, nat);
+        } else if (w == 4) {
+            dihedral_apply<D>(gd, A, id[4], id[1], id[0], id[2], Rl(0.15) * wt, nat);
+        } else {
+            dihedral_apply<D>(gd, A, id[1], id[4], id[3], id[5], Rl(0.15) * wt, nat);
+        }
+        if (A.err) atomicOr(&d.rs[r].err, A.err);
+    }
+}
+
+template <bool D, bool EN, class Bar>
+__device__ __forceinline__ void stack2_unit(const Dev &d, int unit, int w, int lane, Real<D> *q, Bar bar)
+{
+    using Rl = Real<D>;
+    const int item = unit * 32 + lane;
+    const bool on = item < d.nst2;
+    const int *id = d.st2_idx + 7 * item;  // k_10 k00 k01 k10 k20 k21 k30
+    int r = 0;
+    BondGeom<D> gb;
+    DihedralGeom<D> gd;
+    Rl nat = Rl(0), val = Rl(0);
+    if (on) {
+        r = d.rep_of[id[0]];
+        const Pos<D> P = make_pos<D>(d, d.rp + r);
+        if (w == 0) {
+            gb = bond_geom<D>(P, id[2], id[5]);
+            nat = (Rl)d.st2_r0[item];
+            val = Rl(1.4) * (gb.r - nat) * (gb.r - nat);
+        } else if (w <= 2) {
+            gd = w == 1 ? dihedral_geom<D>(P, id[0], id[1], id[3], id[4]) : dihedral_geom<D>(P, id[6], id[4], id[3], id[1]);
+            nat = w == 1 ? Rl(-2.58684) : Rl(3.07135);
+            nat = psi_shift<Rl>(nat, psi_branch<Rl>(gd.psi, nat));
+            val = Rl(4) * (gd.psi - nat) * (gd.psi - nat);
+        } else {
+            val = stack2_off<D>(d, P, item) ? Rl(1) : Rl(0);
+        }
+        q[w * 32 + lane] = val;
+    }
+    bar();
+    if (on && w < 3 && q[3 * 32 + lane] == Rl(0)) {
+        Rl Dn = Rl(1) + q[lane];
+        Dn += q[32 + lane];
+        Dn += q[64 + lane];
+        const Rl E = (Rl)d.st2_E[item] / Dn, wt = -E / Dn;
+        Acc<D> A = force_acc<D>(d);
+        if (w == 0) {
+            bond_apply<D>(gb, A, id[2], id[5], Rl(1.4) * wt, nat);
+            atomicAdd(EN ? d.eterm + r * kNE + 6 : &d.rs[r].e2st_acc, (double)E);
+        } else if (w == 1) {
+            dihedral_apply<D>(gd, A, id[0], id[1], id[3], id[4], Rl(4) * wt, nat);
+        } else {
+            dihedral_apply<D>(gd, A, id[6], id[4], id[3], id[1], Rl(4) * wt, nat);
+        }
+        if (A.err) atomicOr(&d.rs[r].err, A.err);
+    }
+}
+
+// item t of the handle's bonded terms, tertiary and secondary stacks, by one thread (the
+// fused step kernel's form)
+template <bool D>
+__device__ __forceinline__ void topo_item(const Dev &d, int t)
+{
+    using Rl = Real<D>;
+    if (t < d.nbt) {
+        bonded_item<D, false>(d, t, 1);
+        return;
+    }
+    const bool tert = t < d.nbt + d.nst3;
+    const int item = tert ? t - d.nbt : t - d.nbt - d.nst3;
+    const int *id = tert ? d.st3_idx + 6 * item : d.st2_idx + 7 * item;
+    const int r = d.rep_of[id[0]];
+    const Pos<D> P = make_pos<D>(d, d.rp + r);
+    Acc<D> A = force_acc<D>(d);
+    if (tert) {
         const double *nat = d.st3_nat + 6 * item;
         const Rl rdev = distance<D>(P, id[1], id[4]) - (Rl)nat[0];
         int code;
@@ -859,14 +1227,9 @@ __device__ __forceinline__ void topo_item(const Dev &d, int t, int mask, int exc
         const Rl E = (Rl)d.st3_E[item] / Dn;
         six_force<D>(P, A, id, nat, code, -E / Dn);
         d.st_energy[item] = (double)E;
-        atomicAdd(EN ? d.eterm + r * kNE + 7 : &d.rs[r].e3st_acc, (double)E);
+        atomicAdd(&d.rs[r].e3st_acc, (double)E);
     } else {
-        for (int u = d.st2_offby_off[item]; u < d.st2_offby_off[item + 1]; ++u) {
-            const int k = d.st2_offby_idx[u];
-            const int *tid = d.st3_idx + 6 * k;
-            if (distance<D>(P, tid[1], tid[4]) - (Rl)d.st3_nat[6 * k] < Rl(10)) return;
-        }
-        const int *id = d.st2_idx + 7 * item;  // k_10 k00 k01 k10 k20 k21 k30
+        if (stack2_off<D>(d, P, item)) return;
         const Rl rr = distance<D>(P, id[2], id[5]);
         const Rl p1 = dihedral_of<D>(P, id[0], id[1], id[3], id[4]);
         const Rl p2 = dihedral_of<D>(P, id[6], id[4], id[3], id[1]);
@@ -881,15 +1244,50 @@ __device__ __forceinline__ void topo_item(const Dev &d, int t, int mask, int exc
         bond_force<D>(P, A, id[2], id[5], Rl(1.4) * w, r0);
         dihedral_force<D>(P, A, id[0], id[1], id[3], id[4], Rl(4) * w, p10);
         dihedral_force<D>(P, A, id[6], id[4], id[3], id[1], Rl(4) * w, p20);
-        atomicAdd(EN ? d.eterm + r * kNE + 6 : &d.rs[r].e2st_acc, (double)E);
+        atomicAdd(&d.rs[r].e2st_acc, (double)E);
     }
     if (A.err) atomicOr(&d.rs[r].err, A.err);
 }
 
+// Block b of the topology blocks (topo_plan): units of tertiary stacks (two per block of
+// kForceThreads), units of secondary stacks (four per block), bonded terms, then the
+// Gaussian pairs of every replica (noise: 1500 and kNoiseSpare / 2 more each, from the
+// replica's draw counter on; the H-bond Monte Carlo's draws of the step come first, so
+// the step's Gaussians start as many draws later in this table).
 template <bool D, bool EN>
-__global__ void __launch_bounds__(kTopoThreads) k_bonded_stack(Dev d, int mask, int excl_in_list)
+__device__ __forceinline__ void topo_block(const Dev &d, const TopoPlan &tp, int b, int mask, int excl_in_list,
+                                           Real<D> *q /* 16 x 32 */)
 {
-    topo_item<D, EN>(d, blockIdx.x * blockDim.x + threadIdx.x, mask, excl_in_list);
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    if (b < tp.n3) {
+        if (mask & 8) stack3_unit<D, EN>(d, 2 * b + (w >> 3), w & 7, lane, q + (w >> 3) * 8 * 32, NamedBar{1 + (w >> 3), 256});
+        return;
+    }
+    b -= tp.n3;
+    if (b < tp.n2) {
+        if (mask & 8) stack2_unit<D, EN>(d, 4 * b + (w >> 2), w & 3, lane, q + (w >> 2) * 4 * 32, NamedBar{1 + (w >> 2), 128});
+        return;
+    }
+    b -= tp.n2;
+    if (b < tp.nb) {
+        const int item = b * tp.per + tid;
+        if ((mask & 4) && tid < tp.per && item < d.nbt) bonded_item<D, EN>(d, item, excl_in_list);
+        return;
+    }
+    b -= tp.nb;
+    constexpr int kPairs = (kNoise + kNoiseSpare) / 2;
+    const int item = b * tp.per + tid;
+    if (tid < tp.per && item < d.R * kPairs) {
+        const int r = item / kPairs, k = item - r * kPairs;
+        noise_pair<D>(d.rp + r, d.rs[r].ctr + 2 * k, d.gnoise + (size_t)r * kNoiseStride + 2 * k);
+    }
+}
+
+template <bool D, bool EN>
+__global__ void __launch_bounds__(kForceThreads) k_topo(Dev d, TopoPlan tp, int mask, int excl_in_list)
+{
+    __shared__ Real<D> s_q[16 * 32];
+    topo_block<D, EN>(d, tp, blockIdx.x, mask, excl_in_list, s_q);
 }
 
 __device__ __forceinline__ unsigned long long global_ns_hb()
@@ -908,20 +1306,29 @@ __device__ __forceinline__ unsigned long long global_ns_hb()
 // else in global scratch.  status starts as the list build left it (0: live,
 // -1: out of range) and every live bond is back to 0 when the kernel ends, so
 // the shared copy is never written back.
+template <bool D>
 struct HbWork {
-    double *en;    // energy of each live bond this step
-    double *term;  // its six restraint terms (six per bond)
+    Real<D> *en;   // energy of each live bond this step
+    Real<D> *term; // its six restraint terms (six per bond)
     int *st;       // status: 0 formed, 1 broken this step, -1 out of range
-    int *code;     // imaging branch of its dihedrals
-    int *br;       // the branches of its three dihedrals (three per bond)
+    signed char *br;  // per bond: the imaging branches of its three dihedrals; 1 when its distance breaks it
     int *exc;      // excess valence of each over-valence atom
-    int *al;       // over-valence atoms with positive excess (the reference's A list)
+    int *al;       // a bit per over-valence atom: positive excess (the reference's A list)
     int *kl;       // candidate bonds of the chosen atom (the reference's K list)
     const int *ca_off, *ca_idx;  // candidates of each over-valence atom: ca_idx[ca_off[i] ..]
     const int *hb_off, *hb_pos;  // over-valence atoms of each bond: hb_pos[hb_off[k] ..]
 };
 
 constexpr int kHbThreads = 512;
+
+// n ints to shared memory by bd threads, landing by copy_async_wait
+__device__ __forceinline__ void copy_async(int *dst, const int *src, int n, int tid, int bd)
+{
+    const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
+    for (int i = tid; i < n; i += bd)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s + 4u * (unsigned)i), "l"(src + i) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // rand() draws vbase .. vbase + 63 of a replica into v[], by 17 lanes of one warp
 // (one Philox block of four draws each; the same words rand_value returns)
@@ -944,8 +1351,9 @@ __device__ inline void fill_draws(uint32_t *v, unsigned long long seed, unsigned
 
 // One block per replica.  The restraint energies and forces of the live bonds run
 // as (chunk of 32 bonds, term) warp tasks, so that the lanes of a warp evaluate
-// the same term; the Monte Carlo runs on one warp; then the step's Gaussians,
-// drawn by the block while its warps finish the force tasks.
+// the same term; the Monte Carlo runs on one warp.  make_noise: 1 the block then draws the
+// step's Gaussians itself; 2 they are being made beside it (topo_block), and the Monte
+// Carlo's draw count is left for control_step to book with them.
 template <bool D, bool EN, class Bar>
 __device__ __forceinline__ void hbond_block(const Dev &d, int r, int do_hb, int make_noise, int tid, int bd, Bar bar)
 {
@@ -953,15 +1361,11 @@ __device__ __forceinline__ void hbond_block(const Dev &d, int r, int do_hb, int 
     extern __shared__ __align__(16) unsigned char s_dyn[];
     __shared__ uint32_t s_v[64];  // draws vbase .. vbase + 63 of the replica's rand() stream
     __shared__ unsigned long long s_ctr;
-    __shared__ double s_red[2 * 32];
     const RepParams *R = d.rp + r;
     RepState *S = d.rs + r;
     const Pos<D> P = make_pos<D>(d, R);
-    Acc<D> A;
-    A.f = (decltype(A.f))d.f;
-    A.P = d.P;
-    A.err = 0;
-    if (tid == 0) s_ctr = S->ctr;
+    Acc<D> A = force_acc<D>(d);
+    const unsigned long long c0 = S->ctr;
     double e2hb = 0, e3hb = 0;
     const int hb0 = R->hb0, nhb = R->hb1 - R->hb0, ca0 = R->ca0, nca = R->ca1 - R->ca0;
     const int warp = tid >> 5, nwarp = bd >> 5, lane = tid & 31;
@@ -975,38 +1379,39 @@ __device__ __forceinline__ void hbond_block(const Dev &d, int r, int do_hb, int 
             tlap = t;
         }
     };
-    HbWork w;
+    HbWork<D> w;
     const int nact = do_hb ? S->n_active : 0;
-    bar();
 
     // ---- hydrogen_bonds_interactions (E:2145-2350) ----
     if (do_hb) {
         const int c_base = d.ca_coff[ca0], n_cidx = d.ca_coff[R->ca1] - c_base;
         const int h_base = d.hb_coff[hb0], n_cpos = d.hb_coff[R->hb1] - h_base;
+        int off_c = 0, off_h = 0;  // what the offsets below start from
         if (d.hb_smem) {
-            const HbLayout L = hb_layout(d.hb_nmax, d.ca_nmax, d.k_nmax, d.cidx_max, d.cpos_max);
-            w.en = (double *)(s_dyn + L.en);
-            w.term = (double *)(s_dyn + L.term);
+            const HbLayout L = hb_layout(d.hb_nmax, d.ca_nmax, d.k_nmax, d.cidx_max, d.cpos_max, D);
+            w.en = (Rl *)(s_dyn + L.en);
+            w.term = (Rl *)(s_dyn + L.term);
             w.st = (int *)(s_dyn + L.st);
-            w.code = (int *)(s_dyn + L.code);
-            w.br = (int *)(s_dyn + L.br);
+            w.br = (signed char *)(s_dyn + L.br);
             w.exc = (int *)(s_dyn + L.exc);
             w.al = (int *)(s_dyn + L.al);
             w.kl = (int *)(s_dyn + L.kl);
             int *cao = (int *)(s_dyn + L.ca_off), *cai = (int *)(s_dyn + L.ca_idx);
             int *hbo = (int *)(s_dyn + L.hb_off), *hbp = (int *)(s_dyn + L.hb_pos);
-            for (int i = tid; i < nhb; i += bd) w.st[i] = d.hb_status[hb0 + i];
-            for (int i = tid; i <= nca; i += bd) cao[i] = d.ca_coff[ca0 + i] - c_base;
-            for (int i = tid; i < n_cidx; i += bd) cai[i] = d.ca_cidx[c_base + i];
-            for (int i = tid; i <= nhb; i += bd) hbo[i] = d.hb_coff[hb0 + i] - h_base;
-            for (int i = tid; i < n_cpos; i += bd) hbp[i] = d.hb_cpos[h_base + i];
+            // the replica's tables travel to shared memory while the terms are evaluated
+            copy_async(w.st, d.hb_status + hb0, nhb, tid, bd);
+            copy_async(cao, d.ca_coff + ca0, nca + 1, tid, bd);
+            copy_async(cai, d.ca_cidx + c_base, n_cidx, tid, bd);
+            copy_async(hbo, d.hb_coff + hb0, nhb + 1, tid, bd);
+            copy_async(hbp, d.hb_cpos + h_base, n_cpos, tid, bd);
+            off_c = c_base;
+            off_h = h_base;
             w.ca_off = cao; w.ca_idx = cai; w.hb_off = hbo; w.hb_pos = hbp;
         } else {
-            w.en = d.hb_energy + hb0;
-            w.term = d.hb_term + 6 * (size_t)hb0;
+            w.en = (Rl *)(d.hb_energy + hb0);
+            w.term = (Rl *)(d.hb_term + 6 * (size_t)hb0);
             w.st = d.hb_status + hb0;
-            w.code = d.hb_code + hb0;
-            w.br = d.hb_br + 3 * (size_t)hb0;
+            w.br = (signed char *)(d.hb_code + hb0);
             w.exc = d.ca_exc + ca0;
             w.al = d.hb_A + ca0;
             w.kl = d.hb_K + R->kscr0;
@@ -1014,74 +1419,89 @@ __device__ __forceinline__ void hbond_block(const Dev &d, int r, int do_hb, int 
             w.hb_off = d.hb_coff + hb0; w.hb_pos = d.hb_cpos;
         }
         for (int i = tid; i < nca; i += bd) w.exc[i] = d.hb_excess[d.ca_list[ca0 + i]];
-        bar();
-        // a live bond whose central distance strays more than 2 A from native breaks (E:2165-2175)
-        for (int t = tid; t < nact; t += bd) {
-            const int k = d.hb_active[hb0 + t], kl = k - hb0;
-            const Rl rdev = distance<D>(P, d.hb_idx[6 * k + 1], d.hb_idx[6 * k + 4]) - (Rl)d.hb_nat[6 * k];
-            if (fabs((double)rdev) > 2.0) {
-                w.st[kl] = 1;
-                for (int u = w.hb_off[kl]; u < w.hb_off[kl + 1]; ++u) atomicSub(w.exc + w.hb_pos[u], 1);
-                w.en[kl] = 0.0;
-            }
-            int br;
-            w.term[6 * kl] = (double)six_term<D>(P, d.hb_idx + 6 * k, d.hb_nat + 6 * k, 0, rdev, br);
-        }
-        // the angle and dihedral terms: warp task (chunk of 32 live bonds, term 1..5)
+        // the restraint terms: warp task (chunk of 32 live bonds, term 0..5)
         const int nchunk = (nact + 31) >> 5;
-        for (int task = warp; task < 5 * nchunk; task += nwarp) {
-            const int s = 1 + task % 5, t = (task / 5) * 32 + lane;
+        for (int task = warp; task < 6 * nchunk; task += nwarp) {
+            const int s = task % 6, t = (task / 6) * 32 + lane;
             if (t < nact) {
                 const int k = d.hb_active[hb0 + t], kl = k - hb0;
                 int br;
-                const Rl v = six_term<D>(P, d.hb_idx + 6 * k, d.hb_nat + 6 * k, s, Rl(0), br);
-                w.term[6 * kl + s] = (double)v;
-                if (s >= 3) w.br[3 * kl + s - 3] = br;
+                Rl rdev = Rl(0);
+                if (s == 0) {
+                    rdev = distance<D>(P, d.hb_idx[6 * k + 1], d.hb_idx[6 * k + 4]) - (Rl)d.hb_nat[6 * k];
+                    w.br[4 * kl + 3] = fabs(rdev) > Rl(2);
+                }
+                w.term[6 * kl + s] = six_term<D>(P, d.hb_idx + 6 * k, d.hb_nat + 6 * k, s, rdev, br);
+                if (s >= 3) w.br[4 * kl + s - 3] = (signed char)br;
             }
         }
+        copy_async_wait();
         bar();
         for (int t = tid; t < nact; t += bd) {
             const int k = d.hb_active[hb0 + t], kl = k - hb0;
-            if (w.st[kl] == 1) continue;
+            if (w.br[4 * kl + 3]) {  // a live bond whose central distance strays more than 2 A from native breaks (E:2165-2175)
+                w.st[kl] = 1;
+                for (int u = w.hb_off[kl] - off_h; u < w.hb_off[kl + 1] - off_h; ++u) atomicSub(w.exc + w.hb_pos[u], 1);
+                w.en[kl] = Rl(0);
+                continue;
+            }
             Rl q = Rl(0);
-            for (int s = 0; s < 6; ++s) q += (Rl)w.term[6 * kl + s];
-            w.en[kl] = (double)((Rl)d.hb_E[k] * exp_(-q));
-            w.code[kl] = (w.br[3 * kl] + 1) + 3 * (w.br[3 * kl + 1] + 1) + 9 * (w.br[3 * kl + 2] + 1);
+            for (int s = 0; s < 6; ++s) q += w.term[6 * kl + s];
+            w.en[kl] = (Rl)d.hb_E[k] * exp_(-q);
         }
         bar();
         lap(8);
         if (tid < 32) {  // valence-limited Monte Carlo (E:2239-2315), one warp
             const unsigned lt = (1u << lane) - 1u;
-            unsigned long long ctr = s_ctr, vbase = ctr;
-            fill_draws(s_v, R->seed, vbase, lane);
+            unsigned long long ctr = c0, vbase = ctr;
+            bool filled = false;
             const double T = R->T;
             const float inv_t = 1.0f / R->Tf;
+            // A: atoms with positive excess, in atom order: a bit each, kept up as they lose it
+            const int nword = (nca + 31) >> 5;
+            int nA = 0;
+            for (int v = 0; v < nword; ++v) {
+                const int i = 32 * v + lane;
+                const unsigned m = __ballot_sync(kFull, i < nca && w.exc[i] > 0);
+                if (lane == 0) w.al[v] = (int)m;
+                nA += __popc(m);
+            }
+            __syncwarp();
             int guard = nact + 2;
-            while (guard-- > 0) {
-                // A: atoms with positive excess, in atom order
-                int nA = 0;
-                for (int base = 0; base < nca; base += 32) {
-                    const int i = base + lane;
-                    const bool pos = i < nca && w.exc[i] > 0;
-                    const unsigned m = __ballot_sync(kFull, pos);
-                    if (pos) w.al[nA + __popc(m & lt)] = i;
-                    nA += __popc(m);
-                }
-                if (nA == 0) break;
+            while (nA > 0 && guard-- > 0) {
                 // draws ctr, ctr+1, ...: the atom, the K shuffle, the acceptances; u[i] is draw ctr + i
-                if (ctr - vbase > 32) {
+                if (!filled || ctr - vbase > 32) {
                     vbase = ctr;
                     fill_draws(s_v, R->seed, vbase, lane);
+                    filled = true;
                 }
                 const uint32_t *u = s_v + (ctr - vbase);
                 const int nu = 64 - (int)(ctr - vbase);  // draws held from u[0] on (at least 32)
-                const int atom = w.al[pick_index(u[0], nA) - 1];
+                int nth = pick_index(u[0], nA), atom = 0;
+                for (int v0 = 0; v0 < nword; v0 += 32) {  // the nth set bit
+                    const unsigned m = v0 + lane < nword ? (unsigned)w.al[v0 + lane] : 0u;
+                    const int c = __popc(m);
+                    int incl = c;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int t = __shfl_up_sync(kFull, incl, o);
+                        if (lane >= o) incl += t;
+                    }
+                    const unsigned at = __ballot_sync(kFull, incl >= nth);
+                    if (at) {
+                        const int src = __ffs((int)at) - 1;
+                        unsigned mm = __shfl_sync(kFull, m, src);
+                        for (int i = nth - __shfl_sync(kFull, incl - c, src); i > 1; --i) mm &= mm - 1u;
+                        atom = 32 * (v0 + src) + __ffs((int)mm) - 1;
+                        break;
+                    }
+                    nth -= __shfl_sync(kFull, incl, 31);
+                }
                 // K: the atom's candidates still formed, in candidate order
-                const int c0 = w.ca_off[atom], nc = w.ca_off[atom + 1] - c0;
+                const int k0 = w.ca_off[atom] - off_c, nc = w.ca_off[atom + 1] - off_c - k0;
                 int nK = 0;
                 for (int base = 0; base < nc; base += 32) {
                     const int t = base + lane;
-                    const int k = t < nc ? w.ca_idx[c0 + t] : 0;
+                    const int k = t < nc ? w.ca_idx[k0 + t] : 0;
                     const bool ok = t < nc && w.st[k] == 0;
                     const unsigned m = __ballot_sync(kFull, ok);
                     if (ok) w.kl[nK + __popc(m & lt)] = k;
@@ -1093,35 +1513,54 @@ __device__ __forceinline__ void hbond_block(const Dev &d, int r, int do_hb, int 
                     A.err |= kErrRange;
                     break;
                 }
-                if (lane == 0)
-                    for (int i = 1; i <= nK; ++i) {
-                        const int jj = pick_index(i < nu ? u[i] : rand_value(R->seed, ctr + i), nK);
-                        const int tmp = w.kl[i - 1];
-                        w.kl[i - 1] = w.kl[jj - 1];
-                        w.kl[jj - 1] = tmp;
-                    }
-                __syncwarp();
-                // Metropolis walk over the shuffled K (draws nK+1 .. 2nK-1): lane a*nK+b
-                // decides whether candidate a replaces candidate b
-                int kc = 0;
+                int chosen;
                 if (nK * nK <= 32) {
+                    // lane l holds entry l of the list; the swaps in draw order
+                    int kl = w.kl[min(lane, nK - 1)];
+                    const int jj = pick_index(u[min(lane + 1, nK)], nK) - 1;
+                    for (int i = 0; i < nK; ++i) {
+                        const int J = __shfl_sync(kFull, jj, i), ka = __shfl_sync(kFull, kl, i), kb = __shfl_sync(kFull, kl, J);
+                        kl = lane == i ? kb : lane == J ? ka : kl;
+                    }
+                    // Metropolis walk over the shuffled K (draws nK+1 .. 2nK-1): lane a*nK+b
+                    // decides whether candidate a replaces candidate b
+                    const Rl en = w.en[kl];
                     const int a = lane / nK, b = lane - a * nK;
-                    const bool acc = lane < nK * nK && a >= 1 &&
-                                     accept_move(u[nK + a], w.en[w.kl[a]], w.en[w.kl[b]], T, inv_t);
+                    const Rl ea = __shfl_sync(kFull, en, a), eb = __shfl_sync(kFull, en, b);
+                    const bool acc = lane < nK * nK && a >= 1 && accept_move(u[nK + a], ea, eb, T, inv_t);
                     const unsigned dm = __ballot_sync(kFull, acc);
+                    int kc = 0;
                     for (int a2 = 1; a2 < nK; ++a2)
                         if ((dm >> (a2 * nK + kc)) & 1u) kc = a2;
-                } else if (lane == 0) {
-                    for (int i = 2; i <= nK; ++i) {
-                        const int di = nK + i - 1;
-                        const uint32_t v = di < nu ? u[di] : rand_value(R->seed, ctr + di);
-                        if (accept_move(v, w.en[w.kl[i - 1]], w.en[w.kl[kc]], T, inv_t)) kc = i - 1;
+                    chosen = __shfl_sync(kFull, kl, kc);
+                } else {
+                    int kc = 0;
+                    if (lane == 0) {
+                        for (int i = 1; i <= nK; ++i) {
+                            const int jj = pick_index(i < nu ? u[i] : rand_value(R->seed, ctr + i), nK);
+                            const int tmp = w.kl[i - 1];
+                            w.kl[i - 1] = w.kl[jj - 1];
+                            w.kl[jj - 1] = tmp;
+                        }
+                        for (int i = 2; i <= nK; ++i) {
+                            const int di = nK + i - 1;
+                            const uint32_t v = di < nu ? u[di] : rand_value(R->seed, ctr + di);
+                            if (accept_move(v, w.en[w.kl[i - 1]], w.en[w.kl[kc]], T, inv_t)) kc = i - 1;
+                        }
+                        kc = w.kl[kc];
                     }
+                    chosen = __shfl_sync(kFull, kc, 0);
                 }
-                if (lane == 0) {
-                    const int k = w.kl[kc];
-                    w.st[k] = 1;
-                    for (int u = w.hb_off[k]; u < w.hb_off[k + 1]; ++u) w.exc[w.hb_pos[u]] -= 1;
+                if (lane == 0) w.st[chosen] = 1;
+                const int h0 = w.hb_off[chosen] - off_h, nh = w.hb_off[chosen + 1] - off_h - h0;
+                for (int t0 = 0; t0 < nh; t0 += 32) {
+                    bool gone = false;
+                    if (t0 + lane < nh) {
+                        const int i = w.hb_pos[h0 + t0 + lane];
+                        gone = atomicSub(w.exc + i, 1) == 1;
+                        if (gone) atomicAnd(w.al + (i >> 5), ~(1 << (i & 31)));
+                    }
+                    nA -= __popc(__ballot_sync(kFull, gone));
                 }
                 ctr += 2 * nK;
                 __syncwarp();
@@ -1130,6 +1569,27 @@ __device__ __forceinline__ void hbond_block(const Dev &d, int r, int do_hb, int 
         }
         bar();
         lap(9);
+        if (warp == nwarp - 1) {  // the energies
+            for (int t = lane; t < nact; t += 32) {
+                const int k = d.hb_active[hb0 + t], kl = k - hb0;
+                if (w.st[kl] != 1) {
+                    if (d.hb_dode[k]) e3hb += (double)w.en[kl];
+                    else e2hb += (double)w.en[kl];
+                }
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                e2hb += __shfl_down_sync(kFull, e2hb, o);
+                e3hb += __shfl_down_sync(kFull, e3hb, o);
+            }
+            if (lane == 0) {
+                S->e2hb = e2hb;
+                S->e3hb = e3hb;
+                if (EN) {
+                    double *e = d.eterm + r * kNE;
+                    e[8] += e2hb; e[9] += e3hb;
+                }
+            }
+        }
         // forces of the bonds still formed: warp task (chunk of 32 live bonds, term 0..5)
         for (int task = warp; task < 6 * nchunk; task += nwarp) {
             const int s = task % 6, t = (task / 6) * 32 + lane;
@@ -1137,11 +1597,7 @@ __device__ __forceinline__ void hbond_block(const Dev &d, int r, int do_hb, int 
                 const int k = d.hb_active[hb0 + t], kl = k - hb0;
                 if (w.st[kl] != 1) {
                     const Rl wk = -(Rl)w.en[kl];
-                    if (s == 0) {
-                        if (d.hb_dode[k]) e3hb -= (double)wk;
-                        else e2hb -= (double)wk;
-                    }
-                    six_force_term<D>(P, A, d.hb_idx + 6 * k, d.hb_nat + 6 * k, w.code[kl], wk, s);
+                    six_force_term<D>(P, A, d.hb_idx + 6 * k, d.hb_nat + 6 * k, s >= 3 ? w.br[4 * kl + s - 3] : 0, wk, s);
                 }
             }
         }
@@ -1150,27 +1606,26 @@ __device__ __forceinline__ void hbond_block(const Dev &d, int r, int do_hb, int 
         for (int i = tid; i < nhb; i += bd) d.hb_rec[hb0 + i] = w.st[i] == 0 ? 1 : 0;
     lap(10);
     // ---- full_forces: the step's Gaussians follow the Monte Carlo draws ----
-    const unsigned long long c1 = s_ctr;
-    if (make_noise) gen_noise<D>(d, r, c1, tid, bd);
+    const unsigned long long c1 = do_hb ? s_ctr : c0;
+    double *noise = d.gnoise + (size_t)r * kNoiseStride;
+    if (make_noise == 1) gen_noise<D>(d, r, c1, noise, tid, bd);
+    if (make_noise == 2 && c1 - c0 > (unsigned long long)kNoiseSpare)  // past the table's end: all of them here
+        gen_noise<D>(d, r, c1, noise + kNoise + kNoiseSpare, tid, bd);
     if (d.fprof) {  // the Gaussians of every thread are done (timer runs only)
         bar();
         lap(11);
     }
 
-    double v[2] = {e2hb, e3hb};
-    block_sum_t<2>(v, s_red, tid, bd, bar);
-    if (do_hb)
+    if (do_hb && !d.hb_smem) {
+        bar();  // every warp has read the statuses
         for (int t = tid; t < nact; t += bd) {  // every live bond is formed again for the next step
             const int kl = d.hb_active[hb0 + t] - hb0;
             if (w.st[kl] == 1) w.st[kl] = 0;
         }
+    }
     if (tid == 0) {
-        S->ctr = make_noise ? c1 + kNoise : c1;
-        if (do_hb) { S->e2hb = v[0]; S->e3hb = v[1]; }
-        if (EN) {
-            double *e = d.eterm + r * kNE;
-            e[8] += v[0]; e[9] += v[1];
-        }
+        if (make_noise == 2) S->pending = 1u + (unsigned)(c1 - c0);
+        else S->ctr = make_noise ? c1 + kNoise : c1;
     }
     if (A.err) atomicOr(&S->err, A.err);
 }
@@ -1179,6 +1634,59 @@ template <bool D, bool EN>
 __global__ void __launch_bounds__(kHbThreads) k_hbond(Dev d, int do_hb, int make_noise)
 {
     hbond_block<D, EN>(d, blockIdx.x, do_hb, make_noise, (int)threadIdx.x, (int)blockDim.x, CtaBar{});
+}
+
+// The recentring shift of adjust_box (E:2632-2656), the centre bead's new position moved
+// to the box centre, of replica r
+template <bool D>
+__device__ __forceinline__ void form_shift(const Dev &d, int r)
+{
+    const RepParams *R = d.rp + r;
+    double xn[3], vn[3];
+    leap_frog<D>(d, R, r, R->center, xn, vn);
+    for (int c = 0; c < 3; ++c) d.shift[3 * r + c] = R->hbox[c] - xn[c];
+}
+
+// deterministic_forces_MPI (E:2524-2586) with the step's Gaussians, of every replica of the
+// group in one launch: blocks [0, R) the H-bonds of a replica each (the longest chain, so
+// first), then the topology blocks, then the pairs, kForceThreads / TS sub-blocks of PB
+// particles per block.  With finish, the group's last block to end forms the recentring
+// shifts, for which every force of the centre beads must be in.
+// One launch instead of four on forked streams and one for the shift: a step is a chain of
+// kernels of a few microseconds, so each launch, fork and join in it counts (step of one
+// 346-nt replica 32.1 -> 24.7 us, of one 76-nt replica in FP64 96 -> 35 us), and an LR launch
+// with nothing due waited for room beside the other groups' work (64 replicas: 114 -> 107 us).
+// Two blocks of 512 threads per SM; FP64 needs the registers of one.
+template <bool D, int PB, int TS>
+__global__ void __launch_bounds__(kForceThreads, D ? 1 : 2) k_forces(Dev d, TopoPlan tp, int noise, int finish)
+{
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    const int tid = threadIdx.x;
+    int b = blockIdx.x;
+    if (b < d.R) {
+        hbond_block<D, false>(d, b, 1, noise ? 2 : 0, tid, kForceThreads, CtaBar{});
+    } else if ((b -= d.R) < tp.blocks()) {
+        topo_block<D, false>(d, tp, b, 4 | 8, 1, (Real<D> *)s_dyn);
+    } else {
+        constexpr int kSub = kForceThreads / TS;
+        const int sub = tid / TS, pb = (b - tp.blocks()) * kSub + sub;
+        if (pb * PB < d.P)
+            pair_tasks<D, false, true, PB, TS>(d, pb, 1, 1, tid - sub * TS, ((PairSmem<PB> *)s_dyn)[sub],
+                                               NamedBar{1 + sub, TS});
+    }
+    if (!finish) return;
+    __shared__ int s_last;
+    __syncthreads();  // every force of this block is issued
+    if (tid == 0) {
+        __threadfence();
+        s_last = atomicAdd(d.force_blocks, 1u) == gridDim.x - 1;
+        if (s_last) *d.force_blocks = 0u;
+    }
+    __syncthreads();
+    if (s_last) {
+        __threadfence();
+        for (int r = tid; r < d.R; r += kForceThreads) form_shift<D>(d, r);
+    }
 }
 
 __device__ void control_step(const Dev &d, int r);
@@ -1198,19 +1706,12 @@ __device__ inline bool bounded(double x)
     return ((unsigned)(__double_as_longlong(x) >> 52) & 0x7ffu) < 1023u + 20u;
 }
 
-// the recentring shift of adjust_box (E:2632-2656): the centre bead's new position
-// moved to the box centre; one warp per replica, after every force is final
+// the recentring shift alone (the drop-in move_rigid_units, stage timing)
 template <bool D>
 __global__ void k_shift(Dev d)
 {
     wait_prior_grid();
-    const int r = blockIdx.x;
-    const RepParams *R = d.rp + r;
-    if (threadIdx.x == 0) {
-        double xn[3], vn[3];
-        leap_frog<D>(d, R, r, R->center, xn, vn);
-        for (int c = 0; c < 3; ++c) d.shift[3 * r + c] = R->hbox[c] - xn[c];
-    }
+    if (threadIdx.x == 0) form_shift<D>(d, blockIdx.x);
 }
 
 // The five Energies-file values of replica r (E:6308-6312: E2_HB, E3_HB, E2_STACK,
@@ -1392,8 +1893,10 @@ __device__ void control_step(const Dev &d, int r)
     RepState *S = d.rs + r;
     if (threadIdx.x == 0) {
         const double d2 = __longlong_as_double((long long)__ldcg(&S->maxd2));  // every block of the step has added its own
+        const unsigned pending = __ldcg(&S->pending);
         const long long kl = __ldcg(&S->klok) + 1;
         const double e2 = __ldcg(&S->e2st_acc), e3 = __ldcg(&S->e3st_acc);
+        const unsigned long long ctr = __ldcg(&S->ctr);
         double progress = __ldcg(&S->progress);
         const double sh = sqrt(d2);
         progress += (sh + sh);
@@ -1404,6 +1907,10 @@ __device__ void control_step(const Dev &d, int r)
         S->klok = kl;
         S->rebuild = reb;
         S->lr_now = (R->lr_interval <= 1) || ((kl + 1) % R->lr_interval == 1) || (progress == 0.0);
+        if (pending) {  // the step's Monte Carlo draws and Gaussians (hbond_block)
+            S->ctr = ctr + (pending - 1u) + (unsigned long long)kNoise;
+            S->pending = 0u;
+        }
         S->e2st = e2;  // stacking energies of the step just finished (E2_STACK, E3_STACK)
         S->e3st = e3;
         S->e2st_acc = 0.0;
@@ -1882,15 +2389,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_step_fused(Dev d, int step
             hbond_block<D, false>(d, r, 1, 1, tid, kFusedHbThreads, NamedBar{1, kFusedHbThreads});
             if (timer) ph[1] += global_ns() - t0;
         } else {
-            double e0 = 0, e1 = 0;
-            for (int i = wk; i < npad; i += nwk) pair_particle<D, false, false, true, 1, true>(d, R, p0 + i, 0, tb, err, e0, e1);
+            for (int i = wk; i < npad; i += nwk) pair_particle<D, false, 1>(d, R, p0 + i, 0, tb, err);
             if (lr_now)  // groups of four workers per particle (every group of a warp runs the same passes)
                 for (int i = wk >> 2; i < npad; i += nwk >> 2)
-                    pair_particle<D, true, false, false, 4, true>(d, R, p0 + i, wk & 3, tb, err, e0, e1);
+                    pair_particle<D, true, 4>(d, R, p0 + i, wk & 3, tb, err);
             for (int i = wk; i < nb + n3 + n2; i += nwk) {
                 const int t = i < nb ? R->bt0 + i
                                      : (i < nb + n3 ? d.nbt + R->s30 + (i - nb) : d.nbt + d.nst3 + R->s20 + (i - nb - n3));
-                topo_item<D, false>(d, t, 4 | 8, 1);
+                topo_item<D>(d, t);
             }
         }
         cluster_barrier();
@@ -2053,65 +2559,74 @@ void launch_ion_counts(const Dev &d, cudaStream_t s, int r, int nrna, int kind, 
     k_ion_counts<<<(nrna + 127) / 128, 128, 0, s>>>(d, r, kind, r2cut, count, hit);
 }
 
-void launch_pair_sr(const Dev &d, cudaStream_t s, bool en, bool ex)
+void launch_pair(const Dev &d, cudaStream_t s, bool en, bool ex, int sr, int lr)
 {
-    constexpr int L = kLanesSR, T = kBlock * kLanesSR;
-    if (!en && ex && d.lanes_sr == 2) {  // the step's SR launch in the other shapes (tis_run_params.lanes_sr)
-        if (d.fp64) k_pair<true, false, false, true, 2, 2 * kBlock><<<d.nblk, 2 * kBlock, 0, s>>>(d, 1);
-        else k_pair<false, false, false, true, 2, 2 * kBlock><<<d.nblk, 2 * kBlock, 0, s>>>(d, 1);
-        return;
-    }
-    if (!en && ex && d.lanes_sr == 4) {
-        if (d.fp64) k_pair<true, false, false, true, 4, 4 * kBlock><<<d.nblk, 4 * kBlock, 0, s>>>(d, 1);
-        else k_pair<false, false, false, true, 4, 4 * kBlock><<<d.nblk, 4 * kBlock, 0, s>>>(d, 1);
-        return;
-    }
+    const int nb = d.P / 32;
     if (d.fp64) {
-        if (en) k_pair<true, false, true, false, L, T><<<d.nblk, T, 0, s>>>(d, 1);
-        else if (ex) k_pair<true, false, false, true, L, T><<<d.nblk, T, 0, s>>>(d, 1);
-        else k_pair<true, false, false, false, L, T><<<d.nblk, T, 0, s>>>(d, 1);
+        if (en) k_pair<true, true, false><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
+        else if (ex) k_pair<true, false, true><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
+        else k_pair<true, false, false><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
     } else {
-        if (en) k_pair<false, false, true, false, L, T><<<d.nblk, T, 0, s>>>(d, 1);
-        else if (ex) k_pair<false, false, false, true, L, T><<<d.nblk, T, 0, s>>>(d, 1);
-        else k_pair<false, false, false, false, L, T><<<d.nblk, T, 0, s>>>(d, 1);
+        if (en) k_pair<false, true, false><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
+        else if (ex) k_pair<false, false, true><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
+        else k_pair<false, false, false><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
     }
 }
 
-void launch_pair_lr(const Dev &d, cudaStream_t s, bool en, bool force_all)
+namespace {
+
+TopoPlan topo_plan(const Dev &d, bool noise)
 {
-    constexpr int L = kLanesLR, T = kThreadsLR;
-    const int fa = force_all ? 1 : 0;
-    if (!en && d.lanes_lr == 2) {  // the step's LR launch in the other shapes (tis_run_params.lanes_lr)
-        if (d.fp64) k_pair<true, true, false, false, 2, 2 * kBlock><<<d.nblk, 2 * kBlock, 0, s>>>(d, fa);
-        else k_pair<false, true, false, false, 2, 2 * kBlock><<<d.nblk, 2 * kBlock, 0, s>>>(d, fa);
-        return;
-    }
-    if (!en && d.lanes_lr == 8) {
-        if (d.fp64) k_pair<true, true, false, false, 8, 8 * kBlock><<<d.nblk, 8 * kBlock, 0, s>>>(d, fa);
-        else k_pair<false, true, false, false, 8, 8 * kBlock><<<d.nblk, 8 * kBlock, 0, s>>>(d, fa);
-        return;
-    }
+    TopoPlan tp;
+    tp.per = d.wide ? 64 : kForceThreads;
+    tp.n3 = (d.nst3 + 63) / 64;
+    tp.n2 = (d.nst2 + 127) / 128;
+    tp.nb = (d.nbt + tp.per - 1) / tp.per;
+    tp.nn = noise && d.noise == 0 ? (d.R * ((kNoise + kNoiseSpare) / 2) + tp.per - 1) / tp.per : 0;
+    return tp;
+}
+
+template <bool D, int PB, int TS>
+size_t forces_smem(const Dev &d)
+{
+    const size_t pair = sizeof(PairSmem<PB>) * (kForceThreads / TS), topo = sizeof(Real<D>) * 16 * 32;
+    size_t m = pair > topo ? pair : topo;
+    return m > (size_t)d.hb_smem ? m : (size_t)d.hb_smem;
+}
+
+template <bool D, int PB, int TS>
+void launch_forces_t(const Dev &d, cudaStream_t s, bool noise, bool finish)
+{
+    const TopoPlan tp = topo_plan(d, noise);
+    constexpr int per = PB * (kForceThreads / TS);  // particles per pair block
+    k_forces<D, PB, TS><<<d.R + tp.blocks() + (d.P + per - 1) / per, kForceThreads, forces_smem<D, PB, TS>(d), s>>>(
+        d, tp, noise ? 1 : 0, finish ? 1 : 0);
+}
+
+}  // namespace
+
+void launch_forces(const Dev &d, cudaStream_t s, bool noise, bool finish)
+{
     if (d.fp64) {
-        if (en) k_pair<true, true, true, false, L, T><<<d.nblk, T, 0, s>>>(d, fa);
-        else k_pair<true, true, false, false, L, T><<<d.nblk, T, 0, s>>>(d, fa);
+        if (d.wide) launch_forces_t<true, 32, 512>(d, s, noise, finish);
+        else launch_forces_t<true, 32, 128>(d, s, noise, finish);
     } else {
-        if (en) k_pair<false, true, true, false, L, T><<<d.nblk, T, 0, s>>>(d, fa);
-        else k_pair<false, true, false, false, L, T><<<d.nblk, T, 0, s>>>(d, fa);
+        if (d.wide) launch_forces_t<false, 32, 128>(d, s, noise, finish);
+        else launch_forces_t<false, 128, 128>(d, s, noise, finish);
     }
 }
 
 void launch_topology(const Dev &d, cudaStream_t s, int mask, bool en, bool make_noise, bool ex)
 {
     const int xl = ex ? 1 : 0;
-    const int items = d.nbt + d.nst3 + d.nst2;
-    const int blocks = (items + kTopoThreads - 1) / kTopoThreads;
-    if ((mask & (4 | 8)) && blocks > 0) {
+    const TopoPlan tp = topo_plan(d, false);
+    if ((mask & (4 | 8)) && tp.blocks() > 0) {
         if (d.fp64) {
-            if (en) k_bonded_stack<true, true><<<blocks, kTopoThreads, 0, s>>>(d, mask, xl);
-            else k_bonded_stack<true, false><<<blocks, kTopoThreads, 0, s>>>(d, mask, xl);
+            if (en) k_topo<true, true><<<tp.blocks(), kForceThreads, 0, s>>>(d, tp, mask, xl);
+            else k_topo<true, false><<<tp.blocks(), kForceThreads, 0, s>>>(d, tp, mask, xl);
         } else {
-            if (en) k_bonded_stack<false, true><<<blocks, kTopoThreads, 0, s>>>(d, mask, xl);
-            else k_bonded_stack<false, false><<<blocks, kTopoThreads, 0, s>>>(d, mask, xl);
+            if (en) k_topo<false, true><<<tp.blocks(), kForceThreads, 0, s>>>(d, tp, mask, xl);
+            else k_topo<false, false><<<tp.blocks(), kForceThreads, 0, s>>>(d, tp, mask, xl);
         }
     }
     const int hb = (mask & 16) ? 1 : 0, mn = make_noise ? 1 : 0;
@@ -2127,33 +2642,30 @@ void launch_topology(const Dev &d, cudaStream_t s, int mask, bool en, bool make_
     }
 }
 
-int configure_kernels(const Dev &d)
+// Every kernel with dynamic shared memory may take as much as a block can have: the
+// limit belongs to the function, not to a handle, so no handle's size is set.
+int configure_kernels(const Dev &)
 {
-    cudaError_t e = cudaSuccess;
-    if (fused_smem(d) > 48 * 1024) {
-        const int b = (int)fused_smem(d);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_step_fused<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_step_fused<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    }
-    if (d.cell_smem > 48 * 1024) {
-        const int b = d.cell_smem;
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cells<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_cells<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    }
-    if (d.hb_smem > 48 * 1024) {
-        const int b = d.hb_smem;
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hbond<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hbond<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hbond<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hbond<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    int dev = 0, most = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    for (const void *k : {(const void *)k_step_fused<true>, (const void *)k_step_fused<false>, (const void *)k_cells<true>,
+                          (const void *)k_cells<false>, (const void *)k_hbond<true, true>, (const void *)k_hbond<true, false>,
+                          (const void *)k_hbond<false, true>, (const void *)k_hbond<false, false>,
+                          (const void *)k_forces<true, 32, 512>, (const void *)k_forces<true, 32, 128>,
+                          (const void *)k_forces<false, 32, 128>, (const void *)k_forces<false, 128, 128>}) {
+        cudaFuncAttributes a;
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
     }
     return (int)e;
 }
 
 void launch_noise(const Dev &d, cudaStream_t s)
 {
-    if (d.fp64) k_noise<true><<<d.R, kTopoThreads, 0, s>>>(d);
-    else k_noise<false><<<d.R, kTopoThreads, 0, s>>>(d);
+    if (d.fp64) k_noise<true><<<d.R, kForceThreads, 0, s>>>(d);
+    else k_noise<false><<<d.R, kForceThreads, 0, s>>>(d);
 }
 
 // a launch that may begin before the previous kernel on the stream has finished
@@ -2219,8 +2731,8 @@ void launch_force_all_rebuild(const Dev &d, cudaStream_t s) { k_force_rebuild<<<
 
 void launch_rg(const Dev &d, cudaStream_t s, int replica, double *out) { k_rg<<<1, 256, 0, s>>>(d, replica, out); }
 
-// pair SR, pair LR, bonded+stacking, H-bonds (+Gaussians), shift, integrate (+skin check), cells, pair search
-int kernel_launches_per_step() { return 8; }
+// forces (+ Gaussians, recentring shift), integrate (+ skin check), cells, pair search
+int kernel_launches_per_step() { return 4; }
 
 size_t fused_smem(const Dev &d) { return (size_t)max(d.hb_smem, d.cell_smem); }
 

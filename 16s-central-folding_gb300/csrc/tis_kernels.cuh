@@ -31,7 +31,7 @@ struct Dev {
     double *x, *y, *z, *xo, *yo, *zo, *vx, *vy, *vz;
     int4 *q;                    // fixed-point position + (type | kind << 8 | active << 16)
     unsigned long long *f, *flr;  // 3P each: int64 fixed point (mixed) or double (FP64)
-    double *gnoise;             // R x kNoise
+    double *gnoise;             // R x kNoiseStride
     // cells
     int *cell_of, *cell_count, *cell_start, *cell_fill, *cell_list;
     int4 *qs;                   // packed positions in cell order (qs[slot] = q[cell_list[slot]])
@@ -62,23 +62,29 @@ struct Dev {
     const int *hb_coff, *hb_cpos;   // such atoms of each candidate (CSR; replica-local numbers in ca_list)
     int *hb_status, *hb_excess, *hb_active, *hb_K, *hb_A, *ca_exc;
     double *hb_energy;
-    int *hb_code;               // imaging branch of the three native dihedrals
+    int *hb_code;               // four bytes per candidate: dihedral imaging branches, broken (global scratch)
     double *hb_term;            // six restraint terms per candidate (global scratch)
-    int *hb_br;                 // three dihedral branches per candidate (global scratch)
     int hb_nmax, ca_nmax, k_nmax;   // largest per-replica candidate, over-valence atom and K counts
     int cidx_max, cpos_max;         // largest per-replica ca_cidx and hb_cpos lengths
     int hb_smem;                // dynamic shared bytes of the H-bond kernel (0: its arrays stay in global scratch)
     double *eterm;              // R x kNE (per-term energies, compute_forces only)
-    int wide;                   // 1: few particles for the GPU: blocks of fewer particles each
+    unsigned *force_blocks;     // force blocks of the running step that have ended
+    int wide;                   // 1: few particles for the GPU: force blocks of fewer particles each
     double *shift;              // R x 3, recentring shift of the current step (adjust_box)
     const int *cell_rep;        // replica of every cell
     int *hb_rec;                // when not null: 1 per H-bond candidate formed after the step's Monte Carlo, else 0
-    int lanes_sr, lanes_lr;     // threads per particle of the step's SR (1, 2, 4) and LR (2, 4, 8) pair launches
     unsigned long long *fprof;  // when not null: the fused step kernel's phase times, kFusedPhases per replica (ns)
     FrameRing fr;               // frame output from inside the step (fr.every = 0: off)
 };
 constexpr int kFusedPhases = 12;  // forces, H-bond chain, shift, move, control, rebuild, steps with LR, rebuild steps,
                                   // and the H-bond chain's restraint terms, Monte Carlo, forces, Gaussians
+
+// Block counts of the topology blocks (topo_block): tertiary and secondary stack units,
+// bonded terms and Gaussian pairs, the latter two `per` per block
+struct TopoPlan {
+    int n3, n2, nb, nn, per;
+    __host__ __device__ int blocks() const { return n3 + n2 + nb + nn; }
+};
 
 // Adjoint work of one handle (tis_adjoint.cu).  Arrays of 3P or 9P values are
 // component-major (c * P + p) like the state arrays.
@@ -100,17 +106,17 @@ struct AdjDev {
 // Byte offsets of the H-bond kernel's shared-memory arrays (one replica's working
 // set; the kernel and the engine's size check both use this layout).
 struct HbLayout {
-    size_t en, term, st, code, br, exc, al, kl, ca_off, ca_idx, hb_off, hb_pos, total;
+    size_t en, term, st, br, exc, al, kl, ca_off, ca_idx, hb_off, hb_pos, total;
 };
-__host__ __device__ inline HbLayout hb_layout(int hb_nmax, int ca_nmax, int k_nmax, int cidx_max, int cpos_max)
+__host__ __device__ inline HbLayout hb_layout(int hb_nmax, int ca_nmax, int k_nmax, int cidx_max, int cpos_max, bool fp64)
 {
     HbLayout L;
     size_t o = 0;
-    L.en = o; o += 8 * (size_t)hb_nmax;              // double per candidate
-    L.term = o; o += 48 * (size_t)hb_nmax;           // six doubles per candidate
+    const size_t rb = fp64 ? 8 : 4;                  // Real<D>
+    L.en = o; o += rb * (size_t)hb_nmax;             // energy per candidate
+    L.term = o; o += 6 * rb * (size_t)hb_nmax;       // six restraint terms per candidate
     L.st = o; o += 4 * (size_t)hb_nmax;
-    L.code = o; o += 4 * (size_t)hb_nmax;
-    L.br = o; o += 12 * (size_t)hb_nmax;             // three ints per candidate
+    L.br = o; o += 4 * (size_t)hb_nmax;              // four bytes per candidate
     L.exc = o; o += 4 * (size_t)ca_nmax;
     L.al = o; o += 4 * (size_t)ca_nmax;
     L.kl = o; o += 4 * (size_t)k_nmax;
@@ -137,13 +143,15 @@ void launch_ion_counts(const Dev &d, cudaStream_t s, int r, int nrna, int kind, 
 // does not subtract it in the bonded kernel (the reference's net force, without
 // the cancellation of two large equal terms); false gives the reference's
 // per-term split (tis_compute_forces).
-void launch_pair_sr(const Dev &d, cudaStream_t s, bool energies, bool excl_in_list);
-void launch_pair_lr(const Dev &d, cudaStream_t s, bool energies, bool force_all);
+// sr: 1 with the SR lists; lr: the LR lists never (0), of the replicas whose refresh is
+// due (1), of all replicas (2)
+void launch_pair(const Dev &d, cudaStream_t s, bool energies, bool excl_in_list, int sr, int lr);
+// the step's forces in one launch; noise: its Gaussians too; finish: the recentring shifts too
+void launch_forces(const Dev &d, cudaStream_t s, bool noise, bool finish);
 void launch_topology(const Dev &d, cudaStream_t s, int mask, bool energies, bool make_noise, bool excl_in_list);
 void launch_noise(const Dev &d, cudaStream_t s);  // the step's Gaussians only
-int configure_kernels(const Dev &d);
-              // kernel attributes (shared-memory limits); cudaError_t
-void launch_integrate(const Dev &d, cudaStream_t s);  // recentring shift, then the particles
+int configure_kernels(const Dev &d);                  // kernel attributes (shared-memory limits); cudaError_t
+void launch_integrate(const Dev &d, cudaStream_t s);  // recentring shift, then the particles (the drop-in call)
 void launch_rebuild(const Dev &d, cudaStream_t s);  // gated on RepState::rebuild: cells, then pair search
 // the parts of launch_integrate and launch_rebuild, for stage timing
 void launch_shift(const Dev &d, cudaStream_t s);

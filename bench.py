@@ -538,13 +538,17 @@ def gpu_arm(args):
         items = (len(sd["bt_kind"]) + len(sd["st3_E"]) + len(sd["st2_E"])) * N_REPLICAS
         nhb = len(sd["hb_E"]) * N_REPLICAS
         alg = stage_bytes(n_part, sr, lr, 0.1 + reb_rep / N_REPLICAS, nreb, nrna, items, nhb, N_REPLICAS)
+        inside = [k for k in in_step if not in_step[k] > 0]  # stages that run in the force launch ("pair_sr")
+        alg["pair_sr"] += sum(alg[k] for k in inside)
+        for k in inside:
+            alg[k] = 0.0
         per_stage = {}
         for k in in_step:
             b = alg[k] / groups  # one launch = one replica group's kernel in one step
             per_stage[k] = {"in_step_us": 1000 * in_step[k], "alone_us_per_group": 1000 * stages[k] / groups,
                             "alg_bytes_per_launch": b,
                             "achieved_gbs": b / (in_step[k] * 1e-3) / 1e9 if in_step[k] > 0 else None}
-        dom = max(stages, key=stages.get)  # the most execution time of its own (stages timed alone)
+        dom = max((k for k in stages if in_step[k] > 0), key=stages.get)  # the most time of its own (timed alone)
         ach = per_stage[dom]["achieved_gbs"]
         traffic = NCU_DRAM_BYTES_PER_REPLICA.get(dom)
         roofline = {"bound": "latency", "axis": "hbm", "kernel": dom, "achieved": ach, "peak": peak, "unit": "GB/s",

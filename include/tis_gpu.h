@@ -121,9 +121,10 @@ typedef struct tis_run_params {
                               the next rebuild */
     int32_t groups;        /* replica groups whose step graphs run concurrently on the GPU
                               (0: (3 n + 15) / 16 for n replicas, 12 for 64); results do not depend on it */
-    int32_t lanes_sr;      /* threads per particle of the step's SR pair launch: 1, 2, 4 (0: 1) */
-    int32_t lanes_lr;      /* threads per particle of the step's LR pair launch: 2, 4, 8 (0: 4); in mixed
-                              precision results do not depend on either (fixed-point sums) */
+    int32_t lanes_sr;      /* 1, 2, 4 (0: 1) and */
+    int32_t lanes_lr;      /* 2, 4, 8 (0: 4): threads per particle of the pair launches of earlier versions;
+                              accepted and checked, without effect since the force launch deals list
+                              entries out as equal tasks */
     int32_t fused_ctas;    /* 0: a step is the chain of separate kernels (pair, bonded, H-bond, integrator,
                               rebuild); 1..8: tis_step runs the persistent fused step kernel, in which one
                               thread-block cluster of fused_ctas CTAs per replica runs whole steps back to
@@ -340,12 +341,14 @@ int tis_replica_size(tis_handle *h, int replica, int *n_particles);
 #define TIS_N_STAGES 8
 int tis_profile_stages(tis_handle *h, int64_t n, double *ms);
 
-/* The same eight kernels timed inside the step as it runs (no counterpart in the
+/* The step's kernels timed inside the step as it runs (no counterpart in the
  * reference): `steps` (1..1000) fused steps of every group captured with CUDA
  * events around each kernel, all groups' graphs replayed concurrently;
  * ms[TIS_N_STAGES] receives each kernel's mean duration per launch (one group,
  * one step), averaged over the steps and groups, with the other groups' work
- * running beside it.  Advances every replica by `steps` steps. */
+ * running beside it.  The step runs its forces, Gaussians and recentring shift in
+ * one launch: its duration is entry 0, and entries 1 to 4 are 0.  Advances every
+ * replica by `steps` steps. */
 int tis_profile_in_step(tis_handle *h, int32_t steps, double *ms);
 
 /* The persistent fused step kernel (tis_run_params.fused_ctas) run for `steps`
@@ -369,9 +372,8 @@ int tis_get_launch_count(tis_handle *h, int64_t *n);
 int tis_rand_stream(uint64_t seed, uint64_t first, int64_t n, int32_t *out);
 
 /* Measured choice of the launch configuration (no counterpart in the reference):
- * replica groups, steps per captured graph, the threads per particle of the SR
- * and LR pair launches and the step path (fused_ctas: the separate kernels, or
- * the persistent fused kernel with 1, 2 or 4 CTAs per replica), tuned one after
+ * replica groups, steps per captured graph and the step path (fused_ctas: the separate
+ * kernels, or the persistent fused kernel with 1, 2 or 4 CTAs per replica), tuned one after
  * another (coordinate descent), for calls of `steps` steps (0: 300): each trial
  * times, with CUDA events on the handle's stream, as many tis_step(steps) calls of
  * the given replicas as make up at least 1000 steps, after a warm-up that captures
