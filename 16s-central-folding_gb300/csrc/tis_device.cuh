@@ -63,6 +63,9 @@ struct RepParams {
     double k2fix[10], k2sig[10];  // K2 * 2^-32 (fixed-point force to velocity), K2 * sigma (noise)
     // pair tables, 1..45 (E:2908-2938); dm = D_LJ - 1.5852
     float dlj2[46], dm[46], flj[46], elj[46], d2min[46], qclb[46];
+    // pair search: cell sides, and how far (squared, with a margin) a charged bead looks, one
+    // without charge in the reference's full lists, and one in pruned lists, by type
+    float lcellf[3], reach_lr, reach_sr, reach_lj[10];
     float ljkeep2[46];           // (D_LJ + skin)^2 with a 1e-5 margin: pruned-list radius of uncharged pairs
     double dlj2_d[46], dlj_d[46], flj_d[46], elj_d[46], d2min_d[46], qclb_d[46];
     unsigned long long seed;

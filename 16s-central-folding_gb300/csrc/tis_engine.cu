@@ -496,6 +496,20 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
                 R.qclb[J] = (float)(Q * lB);
                 R.ljkeep2[J] = (float)((Dl + prm.skin) * (Dl + prm.skin) * (1.0 + 1e-5));
             }
+        {
+            auto reach = [](double r2) { return (float)((sqrt(r2) + 0.05) * (sqrt(r2) + 0.05)); };
+            R.reach_lr = reach(R.r2lr);
+            R.reach_sr = reach(R.r2sr);
+            for (int a = 1; a <= 9; ++a) {
+                double most = 0;
+                for (int b = 1; b <= 9; ++b) {
+                    const int lo = std::min(a, b), hi = std::max(a, b);
+                    most = std::max(most, (double)R.ljkeep2[(lo - 1) * 9 - (lo - 1) * lo / 2 + hi]);
+                }
+                R.reach_lj[a] = reach(std::min(most, R.r2sr));
+            }
+            for (int k = 0; k < 3; ++k) R.lcellf[k] = (float)R.lcell[k];
+        }
         R.seed = (unsigned long long)scalar_i64(s, "seed", base + r + 1);
 
         // particles
@@ -700,7 +714,12 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
     {
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, prm.device);
-        d.search_warps = std::max(4, sms * 4);  // one block of 4 warps per SM: rebuilds are rare
+        // one replica or so rebuilds in a step: enough warps that each takes a few of its
+        // particles, few enough that the blocks of the steps without a rebuild cost little.
+        // 4 / 8 / 16 per SM: 7 replicas of 3,000 particles 1.25 / 1.22 / 1.20 ms (33 steps), 64
+        // of 5,400 in 12 groups 9.72 / 9.53 / 9.54 ms (100), 16 of 48,900 in 3 groups 9.6 / 8.6 /
+        // 8.2 ms (40); 64 replicas' list builds and 20 steps 2.64 / 2.66 / 2.69 ms
+        d.search_warps = std::max(4, sms * (h->P >= 100000 ? 16 : 8));
         d.sm_count = std::max(1, sms);
         d.wide = total_blocks <= 4 * d.sm_count;
         int nc_max = 1;

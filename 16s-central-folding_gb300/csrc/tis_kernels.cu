@@ -1956,42 +1956,14 @@ __device__ inline int cell_axis_q(double v, unsigned q, double side, double l, i
     return cell_axis(v, side, l);
 }
 
-// Work items of the replicas that rebuild this step, laid end to end (`per`: 0 =
-// padded particles, 1 = cells).  Warp-collective: maps item i to its replica r and
-// the offset within it; returns false past the end.
-__device__ inline bool rebuild_item(const Dev &d, int per, int i, int &r, int &off)
-{
-    const int lane = threadIdx.x & 31;
-    int acc = 0;
-    for (int base = 0; base < d.R; base += 32) {
-        const int rr = base + lane;
-        const int n = (rr < d.R && d.rs[rr].rebuild) ? (per ? d.rp[rr].nc : d.rp[rr].npad) : 0;
-        int incl = n;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const int tot = __shfl_sync(kFull, incl, 31);
-        if (i < acc + tot) {
-            const unsigned m = __ballot_sync(kFull, i < acc + incl);
-            const int src = __ffs(m) - 1;
-            r = base + src;
-            off = i - acc - __shfl_sync(kFull, incl - n, src);
-            return true;
-        }
-        acc += tot;
-    }
-    return false;
-}
-
 // populate_lists' cell binning (separate_in_cells, E:1461-1542) and hydrogen-bond
 // candidate status (E:1698-1736) of one rebuilding replica per block.  Counting
 // and filling run on shared-memory cell counters when the replica's cells fit
 // (Dev::cell_smem), else on the global ones.  In FP64 mode each cell's particles
 // are put in index order, as the reference appends them (E:1536-1540), so that
 // list order and FP64 summation order are reproducible; mixed-precision sums are
-// exact in fixed point and need no order.  Then the packed positions are copied
-// in cell order, so the pair search reads each cell's candidates contiguously.
+// exact in fixed point and need no order.  The packed positions are copied in cell
+// order, so the pair search reads each cell's candidates contiguously.
 constexpr int kCellThreads = 1024;
 
 template <bool D>
@@ -2014,22 +1986,40 @@ __device__ __forceinline__ void cells_block(const Dev &d, int r)
     }
     if (tid == 0) s_carry = 0;
     __syncthreads();
-    for (int i = tid; i < R->npad; i += bd) {
-        const int p = R->p0 + i;
-        int c = -1;
-        const int4 qp = d.q[p];
-        if ((qp.w >> 16) & 1) {
-            const int i1 = cell_axis_q(d.x[p], (unsigned)qp.x, R->box[0], R->lcell[0], R->mc[0]);
-            const int i2 = cell_axis_q(d.y[p], (unsigned)qp.y, R->box[1], R->lcell[1], R->mc[1]);
-            const int i3 = cell_axis_q(d.z[p], (unsigned)qp.z, R->box[2], R->lcell[2], R->mc[2]);
-            if (i1 < 1 || i1 > R->mc[0] || i2 < 1 || i2 > R->mc[1] || i3 < 1 || i3 > R->mc[2]) {
-                atomicOr(&S->err, kErrRange);
-            } else {
-                c = (i1 - 1) * R->mc[1] * R->mc[2] + (i2 - 1) * R->mc[2] + (i3 - 1);
-                atomicAdd(cnt + c, 1);
+    constexpr int kF = 4;  // particles of a thread whose loads are in flight together
+    for (int i0 = tid; i0 < R->npad; i0 += kF * bd) {
+        int4 qv[kF];
+        double xv[kF][3];
+#pragma unroll
+        for (int u = 0; u < kF; ++u) {
+            const int i = i0 + u * bd, p = R->p0 + i;
+            qv[u] = make_int4(0, 0, 0, 0);
+            if (i < R->npad) {
+                qv[u] = d.q[p];
+                xv[u][0] = d.x[p];
+                xv[u][1] = d.y[p];
+                xv[u][2] = d.z[p];
             }
         }
-        d.cell_of[p] = c;
+#pragma unroll
+        for (int u = 0; u < kF; ++u) {
+            const int i = i0 + u * bd;
+            if (i >= R->npad) break;
+            int c = -1;
+            const int4 qp = qv[u];
+            if ((qp.w >> 16) & 1) {
+                const int i1 = cell_axis_q(xv[u][0], (unsigned)qp.x, R->box[0], R->lcell[0], R->mc[0]);
+                const int i2 = cell_axis_q(xv[u][1], (unsigned)qp.y, R->box[1], R->lcell[1], R->mc[1]);
+                const int i3 = cell_axis_q(xv[u][2], (unsigned)qp.z, R->box[2], R->lcell[2], R->mc[2]);
+                if (i1 < 1 || i1 > R->mc[0] || i2 < 1 || i2 > R->mc[1] || i3 < 1 || i3 > R->mc[2]) {
+                    atomicOr(&S->err, kErrRange);
+                } else {
+                    c = (i1 - 1) * R->mc[1] * R->mc[2] + (i2 - 1) * R->mc[2] + (i3 - 1);
+                    atomicAdd(cnt + c, 1);
+                }
+            }
+            d.cell_of[R->p0 + i] = c;
+        }
     }
     __syncthreads();
     // exclusive scan of the counts: first slot of every cell
@@ -2063,10 +2053,25 @@ __device__ __forceinline__ void cells_block(const Dev &d, int r)
         __syncthreads();
     }
     const int nslots = s_carry;
-    for (int i = tid; i < R->npad; i += bd) {
-        const int p = R->p0 + i;
-        const int c = d.cell_of[p];
-        if (c >= 0) d.cell_list[R->p0 + first[c] + atomicAdd(fill + c, 1)] = p;
+    for (int i0 = tid; i0 < R->npad; i0 += kF * bd) {
+        int cv[kF];
+        int4 qv[kF];
+#pragma unroll
+        for (int u = 0; u < kF; ++u) {
+            const int i = i0 + u * bd;
+            cv[u] = -1;
+            if (i < R->npad) {
+                cv[u] = d.cell_of[R->p0 + i];
+                if (!D) qv[u] = d.q[R->p0 + i];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kF; ++u)
+            if (cv[u] >= 0) {
+                const int slot = R->p0 + first[cv[u]] + atomicAdd(fill + cv[u], 1);
+                d.cell_list[slot] = R->p0 + i0 + u * bd;
+                if (!D) d.qs[slot] = qv[u];
+            }
     }
     __syncthreads();
     if (D)  // one warp per cell: rank sort (at most 8 particles per lane), or insertion sort by one lane
@@ -2099,8 +2104,10 @@ __device__ __forceinline__ void cells_block(const Dev &d, int r)
                 __syncwarp();
             }
         }
-    __syncthreads();
-    for (int i = tid; i < nslots; i += bd) d.qs[R->p0 + i] = d.q[d.cell_list[R->p0 + i]];
+    if (D) {
+        __syncthreads();
+        for (int i = tid; i < nslots; i += bd) d.qs[R->p0 + i] = d.q[d.cell_list[R->p0 + i]];
+    }
 
     // hydrogen-bond candidates: live (0) when the central pair is within the SR radius
     for (int a = R->hba0 + tid; a < R->hba1; a += bd) d.hb_excess[a] = d.hba_n[a] - d.hba_val[a];
@@ -2146,19 +2153,17 @@ __global__ void __launch_bounds__(kCellThreads) k_cells(Dev d)
     cells_block<D>(d, blockIdx.x);
 }
 
-// distinct periodic neighbours of cell index i (1..m) along one axis
-__device__ inline int axis_neighbours(int i, int m, int out[3])
+// how far, in cells, the cell d (-1, 0, 1) from cell i of m along an axis is from
+// fixed-point coordinate q, which lies in cell i up to rounding at its faces
+__device__ __forceinline__ float cell_gap(unsigned q, int m, int i, int d)
 {
-    int n = 0;
-    for (int dd = -1; dd <= 1; ++dd) {
-        int v = i + dd;
-        if (v < 1) v += m;
-        if (v > m) v -= m;
-        bool dup = false;
-        for (int t = 0; t < n; ++t) dup |= (out[t] == v);
-        if (!dup) out[n++] = v;
-    }
-    return n;
+    const unsigned long long u = (unsigned long long)q * (unsigned)m;
+    float f = (float)((int)(u >> 32) - i) + (float)(unsigned)u * 2.3283064365386963e-10f;  // from the lower face
+    // a bead on the box's face may be binned on its other side
+    f = f > 0.5f * (float)m + 0.5f ? f - (float)m : f < 0.5f - 0.5f * (float)m ? f + (float)m : f;
+    const float below = fmaxf(0.0f, f), above = fmaxf(0.0f, 1.0f - f);
+    if (d == 0 || m == 1) return 0.0f;
+    return m == 2 ? fminf(below, above) : d < 0 ? below : above;  // of two cells, the other one is on both sides
 }
 
 // SR and LR neighbour lists (E:1576-1694).  A pair is SR when r^2 <= (sr+skin)^2,
@@ -2166,138 +2171,154 @@ __device__ inline int axis_neighbours(int i, int m, int out[3])
 // distance from the exact integer differences decides outside a narrow band
 // around each threshold; inside it the FP64 distance with the reference's
 // rounding and image rule decides, so the lists are the reference's sets.
-// One warp per particle: the lanes scan a neighbour cell's candidates together
-// (contiguous in cell order) and append hits in candidate order by ballot.  The
-// warps stride over the particles of the replicas that rebuild this step.
-// populate_lists' pair search for particle `off` of replica r by one warp; pre, beg:
-// the warp's 32 + 32 ints of shared memory
+// One warp per particle.  Its up to 27 neighbour cells (a lane each) are those the sphere
+// it looks in reaches: the LR list radius, or, for a bead without charge and pruned lists,
+// its widest LJ range plus the skin (of 35 A cells, 18 and 3 on average, where all 27 were
+// scanned before).  The cells' candidates, contiguous in cell order, are scanned end to end,
+// 32 kU at a time, and hits appended in candidate order by ballot: the reference's order.
+// Bound by instructions and the latency of the candidates' loads.  Alone, per step and 64
+// replicas in one launch: 88 -> 49 us; 16 large ones: 200 -> 113 us.
+// populate_lists' pair search for particle `off` of replica r by one warp; seg: the warp's
+// 32 ints of shared memory
 template <bool D>
-__device__ __forceinline__ void search_particle(const Dev &d, int r, int off, int lane, int *pre, int *beg)
+__device__ __forceinline__ void search_particle(const Dev &d, int r, int off, int lane, int *seg)
 {
     const unsigned lt = (1u << lane) - 1u;
     const int P = d.P;
     const RepParams *R = d.rp + r;
+    const int p = R->p0 + off;
+    const int c = d.cell_of[p];
+    if (c < 0) {
+        if (lane == 0) { d.n_sr[p] = 0; d.n_lr[p] = 0; }
+        return;
+    }
     const float sx = R->qstep[0], sy = R->qstep[1], sz = R->qstep[2];
     const float sr_lo = R->r2srf * (1.0f - kBand), sr_hi = R->r2srf * (1.0f + kBand);
     const float lr_lo = R->r2lrf * (1.0f - kBand), lr_hi = R->r2lrf * (1.0f + kBand);
-    {
-        const int p = R->p0 + off;
-        const int c = d.cell_of[p];
-        if (c < 0) {
-            if (lane == 0) { d.n_sr[p] = 0; d.n_lr[p] = 0; }
-            return;
+    const int4 qp = d.q[p];
+    const int nex = d.n_excl[p];
+    const bool chp = is_charged((qp.w >> 8) & 0xff);
+    // the lane's cell of the 3 x 3 x 3 block, in the reference's cell order
+    int cnt = 0, start = 0;
+    if (lane < 27) {
+        const int m1 = R->mc[0], m2 = R->mc[1], m3 = R->mc[2];
+        const int i1 = c / (m2 * m3), i2 = (c / m3) % m2, i3 = c % m3;
+        const int d1 = lane / 9 - 1, d2 = (lane / 3) % 3 - 1, d3 = lane % 3 - 1;
+        // an axis of one or two cells repeats them: each cell once, where the reference meets it first
+        const bool rep = d1 > min(m1, 3) - 2 || d2 > min(m2, 3) - 2 || d3 > min(m3, 3) - 2;
+        const float reach = chp ? R->reach_lr : d.full_lists ? R->reach_sr : R->reach_lj[qp.w & 0xff];
+        const float g1 = cell_gap((unsigned)qp.x, m1, i1, d1) * R->lcellf[0], g2 = cell_gap((unsigned)qp.y, m2, i2, d2) * R->lcellf[1],
+                    g3 = cell_gap((unsigned)qp.z, m3, i3, d3) * R->lcellf[2];
+        if (!rep && g1 * g1 + g2 * g2 + g3 * g3 <= reach) {
+            int a = i1 + d1, b = i2 + d2, e = i3 + d3;
+            a += a < 0 ? m1 : a >= m1 ? -m1 : 0;
+            b += b < 0 ? m2 : b >= m2 ? -m2 : 0;
+            e += e < 0 ? m3 : e >= m3 ? -m3 : 0;
+            const int cc = R->c0 + (a * m2 + b) * m3 + e;
+            start = R->p0 + d.cell_start[cc];
+            cnt = d.cell_count[cc];
         }
-        const int4 qp = d.q[p];
-        const bool chp = is_charged((qp.w >> 8) & 0xff);
-        const int i1 = c / (R->mc[1] * R->mc[2]) + 1, i2 = (c / R->mc[2]) % R->mc[1] + 1, i3 = c % R->mc[2] + 1;
-        int n1[3], n2[3], n3[3];
-        const int m1 = axis_neighbours(i1, R->mc[0], n1);
-        const int m2 = axis_neighbours(i2, R->mc[1], n2);
-        const int m3 = axis_neighbours(i3, R->mc[2], n3);
-        int exl[kExcl];
-        const int nex = d.n_excl[p];
-        for (int t2 = 0; t2 < kExcl; ++t2) exl[t2] = t2 < nex ? d.excl[(size_t)t2 * P + p] : -1;
-        // the neighbour cells' candidate ranges laid end to end, in the reference's
-        // cell order (lane s < 27 holds cell s of the 3 x 3 x 3 block)
-        const int nseg = m1 * m2 * m3;
-        __syncwarp();  // the previous particle's reads of pre/beg are done
-        int cnt_l = 0, start_l = 0;
-        if (lane < nseg) {
-            const int a = lane / (m2 * m3), b = (lane / m3) % m2, e = lane % m3;
-            const int cc = (n1[a] - 1) * R->mc[1] * R->mc[2] + (n2[b] - 1) * R->mc[2] + (n3[e] - 1);
-            start_l = R->p0 + d.cell_start[R->c0 + cc];
-            cnt_l = d.cell_count[R->c0 + cc];
-        }
-        int incl = cnt_l;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const int total = __shfl_sync(kFull, incl, 31);
-        if (lane < nseg) {
-            pre[lane] = incl - cnt_l;
-            beg[lane] = start_l;
-        }
-        if (lane == 0) pre[nseg] = total;
-        __syncwarp();
-        int nsr = 0, nlr = 0, seg = 0;
-        constexpr int kU = 4;  // candidate chunks of 32 whose loads are issued together
-        for (int t0 = 0; t0 < total; t0 += 32 * kU) {
-            int jv[kU];
-            int4 qv[kU];
+    }
+    int incl = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += t;
+    }
+    const int total = __shfl_sync(kFull, incl, 31), first = incl - cnt;
+    const unsigned has = __ballot_sync(kFull, cnt > 0);
+    __syncwarp();  // the previous particle's reads of seg are done
+    if (cnt > 0) seg[__popc(has & lt)] = start - first;  // slot of candidate t of the n-th such cell: seg[n] + t
+    __syncwarp();
+    int exl[kExcl];
 #pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int t = t0 + 32 * u + lane;
-                jv[u] = -1;
-                qv[u] = make_int4(0, 0, 0, 0);
-                if (t < total) {
-                    while (t >= pre[seg + 1]) ++seg;
-                    const int slot = beg[seg] + (t - pre[seg]);
-                    jv[u] = d.cell_list[slot];
-                    qv[u] = d.qs[slot];
-                }
+    for (int k = 0; k < kExcl; ++k) exl[k] = k < nex ? d.excl[(size_t)k * P + p] : -1;
+    int nsr = 0, nlr = 0, before = 0;
+    constexpr int kU = 4;  // candidate chunks of 32 whose loads are issued together
+    for (int t0 = 0; t0 < total; t0 += 32 * kU) {
+        int jv[kU];
+        int4 qv[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+            const int t = t0 + 32 * u + lane;
+            // bit i: a cell's candidates begin at the chunk's i-th
+            const unsigned rel = (unsigned)(first - (t0 + 32 * u));
+            const unsigned begins = __reduce_or_sync(kFull, cnt > 0 && rel < 32u ? 1u << rel : 0u);
+            jv[u] = -1;
+            qv[u] = make_int4(0, 0, 0, 0);
+            if (t < total) {
+                const int slot = seg[before + __popc(begins & (lt | (1u << lane))) - 1] + t;
+                jv[u] = d.cell_list[slot];
+                qv[u] = d.qs[slot];
             }
+            before += __popc(begins);
+        }
 #pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                if (t0 + 32 * u >= total) break;
-                const int j = jv[u];
-                const int4 qj = qv[u];
-                int cls = 0;  // 0 none, 1 SR, 2 LR
-                if (j >= 0 && j != p) {
-                    const bool ch = chp && is_charged((qj.w >> 8) & 0xff);
-                    const float dx = (float)(int)((unsigned)qp.x - (unsigned)qj.x) * sx;
-                    const float dy = (float)(int)((unsigned)qp.y - (unsigned)qj.y) * sy;
-                    const float dz = (float)(int)((unsigned)qp.z - (unsigned)qj.z) * sz;
-                    const float r2f = dx * dx + dy * dy + dz * dz;
-                    if (D) {
-                        const double r2 = exact_r2(d, R, p, j);
-                        cls = r2 <= R->r2sr ? 1 : ((ch && r2 <= R->r2lr) ? 2 : 0);
-                    } else {
-                        if (r2f < sr_lo) cls = 1;
-                        else if (r2f > sr_hi && (!ch || r2f > lr_hi)) cls = 0;
-                        else if (r2f > sr_hi && r2f < lr_lo) cls = 2;
-                        else {
-                            const double e2 = exact_r2(d, R, p, j);
-                            cls = e2 <= R->r2sr ? 1 : ((ch && e2 <= R->r2lr) ? 2 : 0);
-                        }
+        for (int u = 0; u < kU; ++u) {
+            if (t0 + 32 * u >= total) break;
+            const int j = jv[u];
+            const int4 qj = qv[u];
+            int cls = 0;  // 0 none, 1 SR, 2 LR
+            if (j >= 0 && j != p) {
+                const bool ch = chp && is_charged((qj.w >> 8) & 0xff);
+                const float dx = (float)(int)((unsigned)qp.x - (unsigned)qj.x) * sx;
+                const float dy = (float)(int)((unsigned)qp.y - (unsigned)qj.y) * sy;
+                const float dz = (float)(int)((unsigned)qp.z - (unsigned)qj.z) * sz;
+                const float r2f = dx * dx + dy * dy + dz * dz;
+                if (D) {
+                    const double r2 = exact_r2(d, R, p, j);
+                    cls = r2 <= R->r2sr ? 1 : ((ch && r2 <= R->r2lr) ? 2 : 0);
+                } else {
+                    if (r2f < sr_lo) cls = 1;
+                    else if (r2f > sr_hi && (!ch || r2f > lr_hi)) cls = 0;
+                    else if (r2f > sr_hi && r2f < lr_lo) cls = 2;
+                    else {
+                        const double e2 = exact_r2(d, R, p, j);
+                        cls = e2 <= R->r2sr ? 1 : ((ch && e2 <= R->r2lr) ? 2 : 0);
                     }
-                    // pruned list: a pair with an uncharged bead can only exert LJ, which
-                    // vanishes beyond D_LJ; the skin keeps it exact until the next rebuild
-                    if (cls == 1 && !d.full_lists && !ch && r2f > R->ljkeep2[jn12(qp.w & 0xff, qj.w & 0xff)])
-                        cls = 0;
                 }
-                const unsigned bs = __ballot_sync(kFull, cls == 1), bl = __ballot_sync(kFull, cls == 2);
-                if (cls == 1) {
-                    int m = 0;  // how often the reference subtracts this pair's LJ again
-                    for (int t2 = 0; t2 < nex; ++t2) m += (exl[t2] == j);
-                    const int pos = nsr + __popc(bs & lt);
-                    if (pos < d.cap_sr) d.nbr_sr[nb_idx(pos, p, P)] = j | (m << kExclShift);
-                } else if (cls == 2) {
-                    const int pos = nlr + __popc(bl & lt);
-                    if (pos < d.cap_lr) d.nbr_lr[nb_idx(pos, p, P)] = j;
-                }
-                nsr += __popc(bs);
-                nlr += __popc(bl);
+                // pruned list: a pair with an uncharged bead can only exert LJ, which
+                // vanishes beyond D_LJ; the skin keeps it exact until the next rebuild
+                if (cls == 1 && !d.full_lists && !ch && r2f > R->ljkeep2[jn12(qp.w & 0xff, qj.w & 0xff)]) cls = 0;
             }
+            const unsigned bs = __ballot_sync(kFull, cls == 1), bl = __ballot_sync(kFull, cls == 2);
+            if (cls == 1) {
+                int m = 0;  // how often the reference subtracts this pair's LJ again
+                if (nex)
+#pragma unroll
+                    for (int k = 0; k < kExcl; ++k) m += exl[k] == j;
+                const int pos = nsr + __popc(bs & lt);
+                if (pos < d.cap_sr) d.nbr_sr[nb_idx(pos, p, P)] = j | (m << kExclShift);
+            } else if (cls == 2) {
+                const int pos = nlr + __popc(bl & lt);
+                if (pos < d.cap_lr) d.nbr_lr[nb_idx(pos, p, P)] = j;
+            }
+            nsr += __popc(bs);
+            nlr += __popc(bl);
         }
-        if (lane == 0) {
-            if (nsr > d.cap_sr || nlr > d.cap_lr) atomicOr(&d.rs[r].err, kErrCapacity);
-            d.n_sr[p] = min(nsr, d.cap_sr);
-            d.n_lr[p] = min(nlr, d.cap_lr);
-        }
+    }
+    if (lane == 0) {
+        if (nsr > d.cap_sr || nlr > d.cap_lr) atomicOr(&d.rs[r].err, kErrCapacity);
+        d.n_sr[p] = min(nsr, d.cap_sr);
+        d.n_lr[p] = min(nlr, d.cap_lr);
     }
 }
 
+// the warps stride over the particles of the replicas that rebuild this step, laid end to end
 template <bool D>
 __global__ void __launch_bounds__(128) k_pair_search(Dev d)
 {
     wait_prior_grid();
-    __shared__ int s_pre[4][32], s_beg[4][32];  // per warp: candidate offsets and first slots of its cells
-    const int lane = threadIdx.x & 31;
-    const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int r, off;
-    for (int item = wid; rebuild_item(d, 0, item, r, off); item += d.search_warps)
-        search_particle<D>(d, r, off, lane, s_pre[threadIdx.x >> 5], s_beg[threadIdx.x >> 5]);
+    __shared__ int s_seg[4][32];
+    const int lane = threadIdx.x & 31, warps = d.search_warps;
+    int next = (blockIdx.x * 4 + (threadIdx.x >> 5));  // this warp's next particle, counted from the replica's first
+    for (int base = 0; base < d.R; base += 32) {
+        unsigned m = __ballot_sync(kFull, base + lane < d.R && d.rs[min(base + lane, d.R - 1)].rebuild);
+        for (; m; m &= m - 1u) {
+            const int r = base + __ffs((int)m) - 1, npad = d.rp[r].npad;
+            for (; next < npad; next += warps) search_particle<D>(d, r, next, lane, s_seg[threadIdx.x >> 5]);
+            next -= npad;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2355,7 +2376,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_step_fused(Dev d, int step
     RepState *S = d.rs + r;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     __shared__ float s_dlj2[46], s_dm[46], s_flj[46], s_qclb[46];
-    __shared__ int s_pre[kFusedWarps][32], s_beg[kFusedWarps][32];
+    __shared__ int s_seg[kFusedWarps][32];
     __shared__ double s_shift[3];
     __shared__ unsigned long long s_max;
     for (int t = tid; t < 46; t += kFusedThreads) {
@@ -2441,7 +2462,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_step_fused(Dev d, int step
             if (rank == 0) cells_block<D>(d, r);
             cluster_barrier();
             for (int off = rank * kFusedWarps + warp; off < npad; off += cs * kFusedWarps)
-                search_particle<D>(d, r, off, lane, s_pre[warp], s_beg[warp]);
+                search_particle<D>(d, r, off, lane, s_seg[warp]);
             cluster_barrier();
             lap(5);
             ph[7] += 1;

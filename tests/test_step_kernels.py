@@ -96,3 +96,37 @@ def test_small_and_full_blocks_agree(precision, steps):
             else:
                 assert np.abs(a[k] - b[k]).max() < 1e-9, k
         assert many.counters(r + 94) == few.counters(r)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [PREC_MIXED, PREC_FP64])
+@pytest.mark.parametrize("box,full", [(60.0, 1), (60.0, 0), (67.0, 1), (99.5, 1), (101.0, 0), (133.5, 1), (200.0, 0)])
+def test_search_cells_of_any_grid(box, full, precision):
+    """The pair sets (and cells) of grids of one and of 2 x 2 x 2 cells (each neighbour met from both
+    sides), 3 and more cells per axis, against the oracle's; pruned lists, which the search
+    looks for in fewer cells, against the oracle's pairs within their range."""
+    s = load(golden_inputs(), "small", box=box, n_mg=4, n_cl=40, n_k=45)
+    sd = s.to_dict()
+    o = Oracle(sd, seed=3)
+    o.populate_lists()
+    e = Engine([s], precision=precision, full_lists=full)
+    e.populate_lists()
+    c, dims = e.cells(0)
+    oc, od = o.cells()
+    assert np.array_equal(dims, od) and np.array_equal(c, oc)
+    sets = [{tuple(sorted(p)) for p in np.asarray(o.pairs(w)).reshape(-1, 2).tolist()} for w in (0, 1)]
+    got = [{tuple(p) for p in e.pairs(0, w).tolist()} for w in (0, 1)]
+    assert got[1] == sets[1]
+    if full:
+        assert got[0] == sets[0]
+        return
+    # a pair with a sugar or base bead is kept within its contact distance plus the skin
+    x, kind, typ, rlj = np.stack([sd[k] for k in "xyz"], 1), sd["kind"], sd["type"], sd["rlj"]
+    assert got[0] <= sets[0]
+    for i, j in sets[0]:
+        dv = x[i] - x[j]
+        r = np.sqrt(((dv - box * np.round(dv / box)) ** 2).sum())
+        charged = kind[i] not in (1, 2) and kind[j] not in (1, 2)
+        reach = 3.0 + (3.2 if max(typ[i], typ[j]) <= 6 else rlj[typ[i] - 1] + rlj[typ[j] - 1])
+        if charged or abs(r - reach) > 1e-3:
+            assert ((i, j) in got[0]) == (charged or r < reach), (i, j, r)
