@@ -130,3 +130,54 @@ def test_search_cells_of_any_grid(box, full, precision):
         reach = 3.0 + (3.2 if max(typ[i], typ[j]) <= 6 else rlj[typ[i] - 1] + rlj[typ[j] - 1])
         if charged or abs(r - reach) > 1e-3:
             assert ((i, j) in got[0]) == (charged or r < reach), (i, j, r)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,box,sr,lr,offset", [(1, (40.0,) * 3, 5.0, 20.0, 0), (33, (40.0, 61.0, 95.0), 7.0, 20.0, 1),
+                                                (700, (70.0, 75.0, 200.0), 15.0, 33.0, 1), (2049, (150.0,) * 3, 15.0, 15.0, 0),
+                                                (4000, (120.0, 99.0, 101.5), 10.0, 33.0, 1)])
+def test_noalloc_pairs_of_any_grid(n, box, sr, lr, offset):
+    """tis_pair_lists_noalloc over grids of one to ten cells per axis, particles on the faces,
+    outside the box (wrapped once, or left out and counted), equal radii, capacities that cut
+    the output and an output array aligned to four bytes, against all pairs in FP64 numpy."""
+    import torch
+    from tis_gb300 import api
+    rng = np.random.default_rng(n)
+    L = np.asarray(box)
+    x = rng.uniform(-0.2, 1.2, (n, 3)) * L  # differences within 1.5 box sides: the image rule gives the nearest
+    x[rng.random((n, 3)) < 0.02] = 0.0
+    if n > 500:
+        x[: n // 3] = L / 3 + rng.normal(size=(n // 3, 3)) * 8.0  # a dense cluster
+        x[:3] = 3.0 * L  # beyond the single wrap
+    kind = rng.integers(0, 6, n).astype(np.int32)
+    # separate_in_cells (E:1461-1542): one wrap, then ceil(x / l), which puts x = 0 in no cell
+    m = (L / lr).astype(int)
+    w = np.where(x < 0, x + L, np.where(x > L, x - L, x))
+    cell = np.ceil(w / (L / m))
+    inside = ((cell >= 1) & (cell <= m)).all(1)
+    i, j = np.triu_indices(n, 1)
+    ok = inside[i] & inside[j]
+    i, j = i[ok], j[ok]
+    d = x[i] - x[j]
+    d = np.where(d > 0.5 * L, d - L, d)
+    d = np.where(d < -0.5 * L, d + L, d)
+    r2 = d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1] + d[:, 2] * d[:, 2]
+    charged = (kind != 1) & (kind != 2)
+    is_sr = r2 <= sr * sr
+    want = [np.stack([i[m], j[m]], 1) for m in (is_sr, ~is_sr & (r2 <= lr * lr) & charged[i] & charged[j])]
+    xyz = [torch.from_numpy(np.ascontiguousarray(x[:, c])).cuda() for c in range(3)]
+    k = torch.from_numpy(kind).cuda()
+    for cut in (1.0, 0.5):
+        caps = [max(1, int(cut * len(w)) + (64 if cut == 1.0 else 0)) for w in want]
+        out = [torch.full((2 * c + 3,), -7, dtype=torch.int32, device="cuda") for c in caps]
+        counts = torch.full((3,), -1, dtype=torch.int64, device="cuda")
+        api.pair_lists_noalloc(*[v.data_ptr() for v in xyz], k.data_ptr(), n, L, sr, lr, out[0].data_ptr() + 4 * offset, caps[0],
+                               out[1].data_ptr() + 4 * offset, caps[1], counts.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        c = counts.cpu().numpy()
+        assert c.tolist() == [len(want[0]), len(want[1]), int((~inside).sum())]
+        for w, o, cap in zip(want, out, caps):
+            o = o.cpu().numpy()
+            m = min(cap, len(w))
+            got = {tuple(p) for p in o[offset: offset + 2 * m].reshape(-1, 2).tolist()}
+            assert len(got) == m and got <= {tuple(p) for p in w.tolist()}
+            assert (o[:offset] == -7).all() and (o[offset + 2 * m:] == -7).all()
