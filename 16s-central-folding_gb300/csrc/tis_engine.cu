@@ -1123,8 +1123,7 @@ static int grp_param_grad(Group *h, double *out)
     a.px = h->dev.x;
     a.py = h->dev.y;
     a.pz = h->dev.z;
-    tis::launch_adj_pair(h->dev, a, h->stream, false, nullptr, 0);
-    tis::launch_adj_pair(h->dev, a, h->stream, true, nullptr, 0);
+    tis::launch_adj_pair(h->dev, a, h->stream, nullptr, nullptr);
     tis::launch_adj_topo(h->dev, a, h->stream, nullptr, 0);
     TIS_CUDA(cudaGetLastError());
     TIS_CUDA(cudaMemcpyAsync(out, a.dth, sizeof(double) * h->R * tis::kNParams, cudaMemcpyDeviceToHost, h->stream));

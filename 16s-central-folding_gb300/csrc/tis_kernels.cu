@@ -14,6 +14,7 @@
 #include <cstdio>
 
 #include "tis_kernels.cuh"
+#include "tis_tasks.cuh"
 
 namespace tis {
 
@@ -616,34 +617,26 @@ struct NamedBar {
 };
 
 
-constexpr int kPairTasks = 512;  // tasks of a sub-block held in shared memory at a time
-
 template <int PB>
 struct PairSmem {
     float dlj2[46], dm[46], flj[46], qclb[46];
     int4 q[PB];          // packed positions of the particles
-    int4 at[PB];         // places of a particle's tasks: first full chunk, remainders (SR | LR << 16); its SR and LR entries
-    int4 cnt[PB / 32];   // per 32 particles: tasks of a full chunk, of 3, 2, 1 entries
-    int task[kPairTasks];
+    TaskSmem<PB> tasks;
 };
 
 // Pair forces of PB particles (sub-block pb) by the TS threads of one sub-block, over
 // their SR lists and, where the LR force is due (do_lr: 0 never, 1 when
 // RepState::lr_now is set, 2 always), their LR lists.
 //
-// The lists are short and uneven (2.9 SR entries on average, 0 to 40), so a thread per
-// particle ran a warp as long as its longest list, one dependent load after another.
-// Here the sub-block's list entries are cut into tasks of one list chunk (four entries,
-// 16 bytes) for one thread: full chunks first, then those with 3, 2 and 1 entries, so the
-// threads of a warp do equal work and a task's four partner positions are loaded
-// together.  FP64 tasks hold one entry: FP64 latency and the narrow FP64 pipe bound them.
+// Their list entries are dealt out as tasks (tis_tasks.cuh): a thread per particle took one
+// dependent load after another for as long as its warp's longest list.  FP64 tasks hold
+// one entry: FP64 latency and the narrow FP64 pipe bound them.
 // Alone, SR lists of 5 replicas of a 346-nt chain: 22.3 -> 11.9 us; one 76-nt replica in
 // FP64: 52 -> 15 us.
 template <bool D, bool EN, bool EX, int PB, int TS, class Bar>
 __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int do_lr, int tid, PairSmem<PB> &sm, Bar bar)
 {
-    constexpr int U = D ? 1 : 4, UL = D ? 0 : 2;  // entries per task, its logarithm
-    constexpr int kW = PB / 32;
+    constexpr int U = D ? 1 : 4;  // entries per task
     static_assert(TS >= PB, "a thread per particle");
     const int p0 = pb * PB, r = d.blk_rep[p0 / kBlock], P = d.P;
     const RepParams *R = d.rp + r;
@@ -666,72 +659,27 @@ __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int 
         const int ns = act && do_sr ? d.n_sr[p] : 0, nl = act && lr ? d.n_lr[p] : 0;
         if (lr)  // the LR force is kept for the MTS interval: started again here, its tasks add to it
             for (int c = 0; c < 3; ++c) d.flr[c * P + p] = 0ull;  // FP64 mode: 0.0 has the same bits
-        const int full = (ns >> UL) + (nl >> UL);
-        int incl = full;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const unsigned lt = (1u << lane) - 1u;
-        int c[3] = {0, 0, 0}, as = 0, al = 0;
-        if (U > 1)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const unsigned ms = __ballot_sync(kFull, (ns & 3) == 3 - k), ml = __ballot_sync(kFull, (nl & 3) == 3 - k);
-                c[k] = __popc(ms) + __popc(ml);
-                if ((ns & 3) == 3 - k) as = __popc(ms & lt);
-                if ((nl & 3) == 3 - k) al = __popc(ms) + __popc(ml & lt);
-            }
-        sm.at[tid] = make_int4(incl - full, as | (al << 16), ns, nl);
-        if (lane == 31) sm.cnt[tid >> 5] = make_int4(incl, c[0], c[1], c[2]);
+        tasks_count<PB, U>(sm.tasks, tid, ns, nl);
     }
     bar();
-    int total = 0;
-#pragma unroll
-    for (int v = 0; v < kW; ++v) total += sm.cnt[v].x + sm.cnt[v].y + sm.cnt[v].z + sm.cnt[v].w;
+    const int total = tasks_total(sm.tasks);
     int err = 0;
     double e_lj = 0, e_c = 0, e_cl = 0;
     for (int win = 0; win < total; win += kPairTasks) {
         if (win) bar();  // the previous window's tasks are done
-        if (tid < PB) {
-            int4 first = make_int4(-win, -win, -win, -win);  // first task of each class of this particle's 32
-#pragma unroll
-            for (int v = 0; v < kW; ++v) {
-                const int4 n = sm.cnt[v];
-                const bool lower = v < (tid >> 5);
-                first.x += lower ? n.x : 0;
-                first.y += n.x + (lower ? n.y : 0);
-                first.z += n.x + n.y + (lower ? n.z : 0);
-                first.w += n.x + n.y + n.z + (lower ? n.w : 0);
-            }
-            const int4 at = sm.at[tid];
-            const int ns = at.z, nl = at.w;
-            int to = first.x + at.x;
-            for (int k = 0; k < (ns >> UL); ++k, ++to)
-                if ((unsigned)to < (unsigned)kPairTasks) sm.task[to] = tid | ((U - 1) << 8) | (k << 10);
-            for (int k = 0; k < (nl >> UL); ++k, ++to)
-                if ((unsigned)to < (unsigned)kPairTasks) sm.task[to] = tid | (1 << 7) | ((U - 1) << 8) | (k << 10);
-            if (U > 1) {
-                const int rs = ns & 3, rl = nl & 3;
-                to = (rs == 3 ? first.y : rs == 2 ? first.z : first.w) + (at.y & 0xffff);
-                if (rs && (unsigned)to < (unsigned)kPairTasks) sm.task[to] = tid | ((rs - 1) << 8) | ((ns >> 2) << 10);
-                to = (rl == 3 ? first.y : rl == 2 ? first.z : first.w) + (at.y >> 16);
-                if (rl && (unsigned)to < (unsigned)kPairTasks)
-                    sm.task[to] = tid | (1 << 7) | ((rl - 1) << 8) | ((nl >> 2) << 10);
-            }
-        }
+        if (tid < PB) tasks_window<PB, U>(sm.tasks, tid, win);
         bar();
         const int nt = min(total - win, kPairTasks);
         const float lo = R->rc2f * (1.0f - kBand), hi = R->rc2f * (1.0f + kBand);
         const float kap = R->kappaf;
         for (int t = tid; t < nt; t += TS) {
-            const int task = sm.task[t];
-            const int pl = task & 127, p = p0 + pl, cnt = ((task >> 8) & 3) + 1;
-            const bool tlr = (task >> 7) & 1;
+            const int task = sm.tasks.task[t];
+            const int pl = task_particle(task), p = p0 + pl, cnt = task_entries(task);
+            const bool tlr = task_lr(task);
             const int *nbr = tlr ? d.nbr_lr : d.nbr_sr;
             double ec = 0;
             if constexpr (!D) {
-                const int4 e4 = __ldg((const int4 *)nbr + (size_t)(task >> 10) * P + p);
+                const int4 e4 = __ldg((const int4 *)nbr + (size_t)task_chunk(task) * P + p);
                 const int raw[4] = {e4.x, e4.y, e4.z, e4.w};
                 const int4 qp = sm.q[pl];
                 const int tp = qp.w & 0xff;
@@ -755,7 +703,7 @@ __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int 
                     atomic_add_fix(out + 2 * P + p, az);
                 }
             } else {
-                const int raw = __ldg(nbr + nb_idx(task >> 10, p, P));
+                const int raw = __ldg(nbr + nb_idx(task_chunk(task), p, P));
                 const int wp = sm.q[pl].w;
                 const double ljw = EX ? (double)(1 - (raw >> kExclShift)) : 1.0;
                 double ax = 0, ay = 0, az = 0;

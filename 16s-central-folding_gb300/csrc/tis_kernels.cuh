@@ -174,9 +174,10 @@ void launch_fit(const Dev &d, cudaStream_t s, int r, int n_fit, const int *idx, 
 void launch_density(const Dev &d, cudaStream_t s, int r, int n, int kind, const double *fit, const double lo[3],
                     double delta, const int dims[3], unsigned long long *grid);
 
-// adjoint (tis_adjoint.cu).  mode 0: dU/dtheta into a.dth at positions a.px..;
-// mode 1: a.jv += J tan and the parameter terms of lambda = tan.
-void launch_adj_pair(const Dev &d, const AdjDev &a, cudaStream_t s, bool lr, const double *tan, int mode);
+// adjoint (tis_adjoint.cu).  Without tangents (mode 0): dU/dtheta into a.dth at positions
+// a.px..; with them (mode 1): a.jv += J tan and the parameter terms of lambda = tan, the
+// pairs' tangents ts for the SR and tl for the refreshed LR force.
+void launch_adj_pair(const Dev &d, const AdjDev &a, cudaStream_t s, const double *ts, const double *tl);
 void launch_adj_topo(const Dev &d, const AdjDev &a, cudaStream_t s, const double *tan, int mode);
 // the reverse pass of one recorded step: a.lam (after the step) -> a.lam (before it)
 void launch_adj_step(const Dev &d, const AdjDev &a, cudaStream_t s);

@@ -181,3 +181,24 @@ def test_noalloc_pairs_of_any_grid(n, box, sr, lr, offset):
             got = {tuple(p) for p in o[offset: offset + 2 * m].reshape(-1, 2).tolist()}
             assert len(got) == m and got <= {tuple(p) for p in w.tolist()}
             assert (o[:offset] == -7).all() and (o[offset + 2 * m:] == -7).all()
+
+
+@pytest.mark.gpu
+def test_gradients_of_small_and_full_blocks_agree():
+    """dU/dtheta and a trajectory gradient of replicas on full blocks (a handle of 96) against
+    the same replicas alone, on blocks of few particles: FP64 sums in another order."""
+    systems = [load(golden_inputs(), "small", seed=s) for s in (3, 4)]
+    many, few = (Engine(s, precision=PREC_MIXED, groups=1) for s in (systems * 48, systems))
+    for e in (many, few):
+        e.populate_lists()
+        e.step(200)
+        e.sync()
+    a, b = many.param_grad(), few.param_grad()
+    assert np.abs(a[:2] - b).max() <= 1e-10 * np.abs(b).max() and np.array_equal(a[94:] != 0, b != 0)
+    n = sum(few.n)
+    w = np.random.default_rng(5).normal(size=n)
+    ga, da = many.traj_grad(6, 4, {"x": np.tile(w, 48)}, want_state=True)
+    gb, db = few.traj_grad(6, 4, {"x": w}, want_state=True)
+    assert np.abs(ga[:2] - gb).max() <= 1e-9 * np.abs(gb).max()
+    for k in STATE_NAMES:
+        assert np.abs(da[k][:n] - db[k]).max() <= 1e-9 * max(1.0, np.abs(db[k]).max()), k
