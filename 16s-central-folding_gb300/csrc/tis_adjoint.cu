@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(128) k_adj_pair(Dev d, AdjDev a, const double 
     const int r = d.blk_rep[p0 / kBlock];
     const RepParams *R = d.rp + r;
     if (tid < PB) {
-        const int p = p0 + tid, w = d.q[p].w;
+        const int p = p0 + tid, w = d.code[p];
         const bool act = (w >> 16) & 1;
         sm.w[tid] = w;
         sm.x[0][tid] = a.px[p];
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(128) k_adj_pair(Dev d, AdjDev a, const double 
                 if (k >= cnt) break;
                 const int j = raw[k] & kIdxMask;
                 const double ljw = lr ? 0.0 : (double)(1 - (raw[k] >> kExclShift));
-                const int wj = d.q[j].w, tj = wj & 0xff, kj = (wj >> 8) & 0xff;
+                const int wj = __ldg(d.code + j), tj = wj & 0xff, kj = (wj >> 8) & 0xff;
                 const int J = jn12(tp, tj);
                 double v[3] = {sm.x[0][pl] - a.px[j], sm.x[1][pl] - a.py[j], sm.x[2][pl] - a.pz[j]};
 #pragma unroll
@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(kBlock) k_adj_center(Dev d, AdjDev a)
     const int r = d.blk_rep[blockIdx.x];
     const int P = d.P;
     double v[3] = {0, 0, 0};
-    if ((d.q[p].w >> 16) & 1)
+    if ((d.code[p] >> 16) & 1)
         for (int c = 0; c < 3; ++c) v[c] = a.lam[c * P + p] + a.lam[(3 + c) * P + p];
     block_reduce<3>(v, s_red);
     if (threadIdx.x == 0)
@@ -649,10 +649,10 @@ __global__ void __launch_bounds__(kBlock) k_adj_move(Dev d, AdjDev a)
     const int r = d.blk_rep[blockIdx.x];
     const RepParams *R = d.rp + r;
     const int P = d.P;
-    const int4 qp = d.q[p];
+    const int code = d.code[p];
     double g[2] = {0, 0};
-    if ((qp.w >> 16) & 1) {
-        const int t = qp.w & 0xff;
+    if ((code >> 16) & 1) {
+        const int t = code & 0xff;
         const double k1 = R->k1[t], k2 = R->k2[t], h = R->h;
         const double sg = d.noise == 0 ? R->sigma[t] : 0.0;
         const int kn = (p - R->p0 + 1) % 1000;
@@ -703,7 +703,8 @@ __global__ void __launch_bounds__(kBlock) k_adj_move(Dev d, AdjDev a)
     }
 }
 
-// lambda_x += J^T lamf (+ J_LR^T mu where the LR force was refreshed; mu then restarts)
+// lambda_x += J^T lamf (+ J_LR^T mu where the LR force was refreshed; mu then restarts); the
+// sum of the recentring shift's adjoint starts again for the next step
 __global__ void __launch_bounds__(kBlock) k_adj_finish(Dev d, AdjDev a)
 {
     const int p = blockIdx.x * kBlock + threadIdx.x;
@@ -713,16 +714,29 @@ __global__ void __launch_bounds__(kBlock) k_adj_finish(Dev d, AdjDev a)
         a.lam[c * P + p] += a.jv[c * P + p];
         if (a.rlr[r]) a.mu[c * P + p] = 0.0;
     }
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < 3 * d.R; i += kBlock) a.cen[i] = 0.0;
 }
 
 // the step's inputs, after its forces and before its integrator: x .. v, the force
-// (f + the held LR force, without the noise) in FP64, the LR refresh flag
-__global__ void __launch_bounds__(kBlock) k_adj_record(Dev d, AdjDev a)
+// (f + the held LR force, without the noise) in FP64, the LR refresh flag, and the entries
+// the lists hold (of slots ten times as many) into to's arrays
+__device__ __forceinline__ void copy_list(const int *src, int *dst, int n, int p, int P)
+{
+    for (int c = 0; c < (n + 3) >> 2; ++c) ((int4 *)dst)[(size_t)c * P + p] = ((const int4 *)src)[(size_t)c * P + p];
+}
+
+__global__ void __launch_bounds__(kBlock) k_adj_record(Dev d, AdjDev a, Dev to)
 {
     const int p = blockIdx.x * kBlock + threadIdx.x;
     const int P = d.P;
     const double *src[9] = {d.x, d.y, d.z, d.xo, d.yo, d.zo, d.vx, d.vy, d.vz};
     for (int c = 0; c < 9; ++c) a.rx[c * P + p] = src[c][p];
+    const int ns = d.n_sr[p], nl = d.n_lr[p];
+    to.n_sr[p] = ns;
+    to.n_lr[p] = nl;
+    copy_list(d.nbr_sr, to.nbr_sr, ns, p, P);
+    copy_list(d.nbr_lr, to.nbr_lr, nl, p, P);
     for (int c = 0; c < 3; ++c) {
         double v;
         if (d.fp64) v = ((const double *)d.f)[c * P + p] + ((const double *)d.flr)[c * P + p];
@@ -790,17 +804,24 @@ void launch_adj_topo(const Dev &d, const AdjDev &a, cudaStream_t s, const double
     else k_adj_topo<double><<<nb, kAdjTopoThreads, 0, s>>>(d, a, tan, mode);
 }
 
-void launch_adj_step(const Dev &d, const AdjDev &a, cudaStream_t s)
+void launch_adj_step(const Dev &d, const AdjDev &a, cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join)
 {
-    cudaMemsetAsync(a.cen, 0, sizeof(double) * 3 * d.R, s);
     k_adj_center<<<d.nblk, kBlock, 0, s>>>(d, a);
     k_adj_move<<<d.nblk, kBlock, 0, s>>>(d, a);
+    // the restraint terms, long chains of few threads, beside the pairs
+    cudaEventRecord(fork, s);
+    cudaStreamWaitEvent(side, fork, 0);
+    launch_adj_topo(d, a, side, a.lamf, 1);
+    cudaEventRecord(join, side);
     launch_adj_pair(d, a, s, a.lamf, a.mu);
-    launch_adj_topo(d, a, s, a.lamf, 1);
+    cudaStreamWaitEvent(s, join, 0);
     k_adj_finish<<<d.nblk, kBlock, 0, s>>>(d, a);
 }
 
-void launch_adj_record(const Dev &d, const AdjDev &a, cudaStream_t s) { k_adj_record<<<d.nblk, kBlock, 0, s>>>(d, a); }
+void launch_adj_record(const Dev &d, const AdjDev &a, const Dev &to, cudaStream_t s)
+{
+    k_adj_record<<<d.nblk, kBlock, 0, s>>>(d, a, to);
+}
 
 void launch_adj_unpack(const Dev &d, cudaStream_t s, double *dst, const double *stage, int n, unsigned mask)
 {

@@ -133,12 +133,23 @@ struct Group {
     double *a_st2_dss = nullptr, *a_hb_dhs = nullptr;
     int *a_st2_cls = nullptr;
     int nhb_all = 0, nhba_all = 0;  // H-bond candidates and H-bond atoms of all replicas
+    // tis_traj_grad: its streams (the reverse pass, its restraint terms) and events, made by the
+    // first call, and its memory, kept for the next call when not larger than kAdjKeep
+    cudaStream_t adj_stream[2] = {nullptr, nullptr};
+    cudaEvent_t adj_event[6] = {};
+    char *adj_mem = nullptr;
+    size_t adj_bytes = 0;
 
     ~Group()
     {
         if (graph) cudaGraphExecDestroy(graph);
         if (tail) cudaGraphExecDestroy(tail);
         for (void *p : owned) cudaFree(p);
+        if (adj_mem) cudaFree(adj_mem);
+        for (cudaStream_t s : adj_stream)
+            if (s) cudaStreamDestroy(s);
+        for (cudaEvent_t e : adj_event)
+            if (e) cudaEventDestroy(e);
         if (h_rs) cudaFreeHost(h_rs);
         if (h_peaks) cudaFreeHost(h_peaks);
         if (stream) cudaStreamDestroy(stream);
@@ -738,10 +749,11 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
     tis::RepState *d_rs = nullptr;
     int *d_blk = nullptr, *d_rep = nullptr, *d_cellrep = nullptr;
     int4 *d_q = nullptr;
-    if ((rc = dupload(O, &d_rp, rp)) || (rc = dupload(O, &d_rs, rs)) || (rc = dupload(O, &d_blk, blk_rep)) ||
+    int *d_code = nullptr;
+    if ((rc = dupload(O, &d_code, code)) || (rc = dupload(O, &d_rp, rp)) || (rc = dupload(O, &d_rs, rs)) || (rc = dupload(O, &d_blk, blk_rep)) ||
         (rc = dupload(O, &d_rep, rep_of)) || (rc = dupload(O, &d_cellrep, cell_rep)) || (rc = dupload(O, &d_q, q)))
         return bail(rc);
-    d.rp = d_rp; d.rs = d_rs; d.blk_rep = d_blk; d.rep_of = d_rep; d.cell_rep = d_cellrep; d.q = d_q;
+    d.rp = d_rp; d.rs = d_rs; d.blk_rep = d_blk; d.rep_of = d_rep; d.cell_rep = d_cellrep; d.q = d_q; d.code = d_code;
     {
         excl_of.resize(h->P);
         std::vector<int> ex((size_t)tis::kExcl * h->P, -1), nex(h->P, 0);
@@ -1154,6 +1166,9 @@ std::vector<std::pair<void *, size_t>> step_state(const Group *h)
 
 inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
+constexpr size_t kAdjKeep = (size_t)4 << 30;    // memory a group keeps between tis_traj_grad calls, at most
+constexpr size_t kAdjSecond = (size_t)8 << 30;  // recorded steps of one segment up to which a second set is taken
+
 // seed: the group's part of nine packed arrays from offset `off` (NULL entries zero);
 // dtheta: R x kNParams of the group; dstate0: packed like seed (NULL entries skipped)
 static int grp_traj_grad(Group *h, int64_t steps, int K, const double *const *seed, int64_t off, double *dtheta,
@@ -1168,20 +1183,73 @@ static int grp_traj_grad(Group *h, int64_t steps, int K, const double *const *se
     size_t sbytes = 0;
     for (const auto &e : st) sbytes += align256(e.second);
     const int64_t nseg = (steps + K - 1) / K;
-    AdjMem M;
-    char *arena = nullptr;
+    for (cudaStream_t &s : h->adj_stream)
+        if (!s) TIS_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    for (cudaEvent_t &e : h->adj_event)
+        if (!e) TIS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    const cudaStream_t back = h->adj_stream[0], side = h->adj_stream[1];
+    const cudaEvent_t fork = h->adj_event[0], join = h->adj_event[1];
+    const cudaEvent_t *recorded = &h->adj_event[2], *used = &h->adj_event[4];
+
+    // one block of device memory: the adjoint's arrays, the checkpoints, and one or (where
+    // there is room) two sets of K recorded steps, so that a segment is recomputed while the
+    // one after it is taken in reverse
     tis::AdjDev a = adj_base(h);
-    double *rx, *rf, *rg;
-    int *rhb, *rlr, *rnsr, *rnlr, *rbsr, *rblr;
-    const size_t Kz = (size_t)K, nhb = (size_t)h->nhb_all;
-    if ((rc = M.alloc(h, &arena, (size_t)(nseg + 1) * sbytes)) || (rc = M.alloc(h, &a.lam, 9 * P)) ||
-        (rc = M.alloc(h, &a.lamf, 3 * P)) || (rc = M.alloc(h, &a.mu, 3 * P)) || (rc = M.alloc(h, &a.jv, 3 * P)) ||
-        (rc = M.alloc(h, &a.cen, 3 * R)) || (rc = M.alloc(h, &a.dth, R * tis::kNParams)) ||
-        (rc = M.alloc(h, &rx, Kz * 9 * P)) || (rc = M.alloc(h, &rf, Kz * 3 * P)) ||
-        (rc = M.alloc(h, &rg, Kz * R * tis::kNoise)) || (rc = M.alloc(h, &rhb, Kz * std::max<size_t>(nhb, 1))) ||
-        (rc = M.alloc(h, &rlr, Kz * R)) || (rc = M.alloc(h, &rnsr, Kz * P)) || (rc = M.alloc(h, &rnlr, Kz * P)) ||
-        (rc = M.alloc(h, &rbsr, Kz * d.cap_sr * P)) || (rc = M.alloc(h, &rblr, Kz * d.cap_lr * P)))
-        return rc;
+    const size_t nhb = std::max<size_t>((size_t)h->nhb_all, 1), Kz = (size_t)std::min<int64_t>(K, steps);
+    struct Slot {
+        size_t rx, rf, rg, rhb, rlr, nsr, nlr, bsr, blr, bytes;
+    } sl{};
+    {
+        size_t o = 0;
+        auto put = [&](size_t &at, size_t bytes) {
+            at = o;
+            o += align256(bytes);
+        };
+        put(sl.rx, 72 * P); put(sl.rf, 24 * P); put(sl.rg, 8 * R * tis::kNoise); put(sl.rhb, 4 * nhb); put(sl.rlr, 4 * R);
+        put(sl.nsr, 4 * P); put(sl.nlr, 4 * P); put(sl.bsr, 4 * (size_t)d.cap_sr * P); put(sl.blr, 4 * (size_t)d.cap_lr * P);
+        sl.bytes = o;
+    }
+    const size_t work = align256(8 * (18 * P + 3 * R + R * tis::kNParams));
+    const size_t base = work + (size_t)(nseg + 1) * sbytes;
+    struct Free {  // memory above kAdjKeep goes back when the call ends
+        Group *h;
+        ~Free()
+        {
+            if (h->adj_bytes > kAdjKeep) {
+                cudaStreamSynchronize(h->stream);
+                for (cudaStream_t s : h->adj_stream) cudaStreamSynchronize(s);
+                cudaFree(h->adj_mem);
+                h->adj_mem = nullptr;
+                h->adj_bytes = 0;
+            }
+        }
+    } guard{h};
+    int sets = nseg > 1 && Kz * sl.bytes <= kAdjSecond ? 2 : 1;
+    for (;; sets = 1) {
+        const size_t need = base + (size_t)sets * Kz * sl.bytes;
+        if (h->adj_bytes >= need) break;
+        if (h->adj_mem) cudaFree(h->adj_mem);
+        h->adj_mem = nullptr;
+        h->adj_bytes = 0;
+        const cudaError_t e = cudaMalloc((void **)&h->adj_mem, need);
+        if (e == cudaSuccess) {
+            h->adj_bytes = need;
+            break;
+        }
+        cudaGetLastError();
+        if (sets == 1) return fail(TIS_ERR_NOMEM, "cudaMalloc(%zu bytes) for the adjoint: %s", need, cudaGetErrorString(e));
+    }
+    {
+        double *w = (double *)h->adj_mem;
+        a.lam = w;
+        a.lamf = w + 9 * P;
+        a.mu = w + 12 * P;
+        a.jv = w + 15 * P;
+        a.cen = w + 18 * P;
+        a.dth = a.cen + 3 * R;
+        TIS_CUDA(cudaMemsetAsync(w, 0, work, h->stream));
+    }
+    char *const arena = h->adj_mem + work, *const slots = h->adj_mem + base;
     auto save = [&](int64_t slot) {
         char *p = arena + slot * sbytes;
         for (const auto &e : st) {
@@ -1196,22 +1264,23 @@ static int grp_traj_grad(Group *h, int64_t steps, int K, const double *const *se
             p += align256(e.second);
         }
     };
-    // the recorded step j of a segment: its inputs and the lists its forces read
-    auto slot = [&](int j, tis::Dev &dj) {
+    // the recorded step j of a segment in set b: its inputs and the lists its forces read
+    auto slot = [&](int b, int j, tis::Dev &dj) {
+        char *const s = slots + ((size_t)b * Kz + (size_t)j) * sl.bytes;
         tis::AdjDev aj = a;
-        aj.rx = rx + (size_t)j * 9 * P;
-        aj.rf = rf + (size_t)j * 3 * P;
-        aj.rg = rg + (size_t)j * R * tis::kNoise;
-        aj.rhb = rhb + (size_t)j * std::max<size_t>(nhb, 1);
-        aj.rlr = rlr + (size_t)j * R;
+        aj.rx = (double *)(s + sl.rx);
+        aj.rf = (double *)(s + sl.rf);
+        aj.rg = (double *)(s + sl.rg);
+        aj.rhb = (int *)(s + sl.rhb);
+        aj.rlr = (int *)(s + sl.rlr);
         aj.px = aj.rx;
         aj.py = aj.rx + P;
         aj.pz = aj.rx + 2 * P;
         dj = d;
-        dj.n_sr = rnsr + (size_t)j * P;
-        dj.n_lr = rnlr + (size_t)j * P;
-        dj.nbr_sr = rbsr + (size_t)j * d.cap_sr * P;
-        dj.nbr_lr = rblr + (size_t)j * d.cap_lr * P;
+        dj.n_sr = (int *)(s + sl.nsr);
+        dj.n_lr = (int *)(s + sl.nlr);
+        dj.nbr_sr = (int *)(s + sl.bsr);
+        dj.nbr_lr = (int *)(s + sl.blr);
         return aj;
     };
 
@@ -1234,30 +1303,34 @@ static int grp_traj_grad(Group *h, int64_t steps, int K, const double *const *se
         }
     tis::launch_adj_unpack(d, h->stream, a.lam, h->stage, h->npk, mask);
 
-    // backward: each segment recomputed from its checkpoint, then its steps in reverse
-    for (int64_t g = nseg - 1; g >= 0; --g) {
+    // backward: each segment recomputed from its checkpoint on the group's stream, its steps
+    // taken in reverse on another; a set of recorded steps is written again only after its
+    // reverse pass has read it
+    for (int64_t g = nseg - 1, turn = 0; g >= 0; --g, ++turn) {
+        const int b = sets == 2 ? (int)(turn & 1) : 0;
+        if (turn >= sets) TIS_CUDA(cudaStreamWaitEvent(h->stream, used[b], 0));
         restore(g);
         const int len = (int)std::min<int64_t>(K, steps - g * K);
         for (int j = 0; j < len; ++j) {
             tis::Dev dj;
-            const tis::AdjDev aj = slot(j, dj);
+            const tis::AdjDev aj = slot(b, j, dj);
             h->dev.hb_rec = aj.rhb;
             enqueue_forces(h, true);
             h->dev.hb_rec = nullptr;
-            TIS_CUDA(cudaMemcpyAsync(dj.n_sr, d.n_sr, 4 * P, cudaMemcpyDeviceToDevice, h->stream));
-            TIS_CUDA(cudaMemcpyAsync(dj.n_lr, d.n_lr, 4 * P, cudaMemcpyDeviceToDevice, h->stream));
-            TIS_CUDA(cudaMemcpyAsync(dj.nbr_sr, d.nbr_sr, 4 * (size_t)d.cap_sr * P, cudaMemcpyDeviceToDevice, h->stream));
-            TIS_CUDA(cudaMemcpyAsync(dj.nbr_lr, d.nbr_lr, 4 * (size_t)d.cap_lr * P, cudaMemcpyDeviceToDevice, h->stream));
-            tis::launch_adj_record(d, aj, h->stream);
+            tis::launch_adj_record(d, aj, dj, h->stream);
             tis::launch_move(d, h->stream);
             tis::launch_rebuild(d, h->stream);
         }
+        TIS_CUDA(cudaEventRecord(recorded[b], h->stream));
+        TIS_CUDA(cudaStreamWaitEvent(back, recorded[b], 0));
         for (int j = len - 1; j >= 0; --j) {
             tis::Dev dj;
-            const tis::AdjDev aj = slot(j, dj);
-            tis::launch_adj_step(dj, aj, h->stream);
+            const tis::AdjDev aj = slot(b, j, dj);
+            tis::launch_adj_step(dj, aj, back, side, fork, join);
         }
+        TIS_CUDA(cudaEventRecord(used[b], back));
         TIS_CUDA(cudaGetLastError());
+        if (g == 0) TIS_CUDA(cudaStreamWaitEvent(h->stream, used[b], 0));
     }
     if ((rc = check_flags(h))) return rc;
     restore(nseg);

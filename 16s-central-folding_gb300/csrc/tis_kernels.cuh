@@ -30,6 +30,7 @@ struct Dev {
     const int *rep_of;          // replica of every particle (padded slots included)
     double *x, *y, *z, *xo, *yo, *zo, *vx, *vy, *vz;
     int4 *q;                    // fixed-point position + (type | kind << 8 | active << 16)
+    const int *code;            // type | kind << 8 | active << 16 alone: no step writes it
     unsigned long long *f, *flr;  // 3P each: int64 fixed point (mixed) or double (FP64)
     double *gnoise;             // R x kNoiseStride
     // cells
@@ -179,10 +180,12 @@ void launch_density(const Dev &d, cudaStream_t s, int r, int n, int kind, const 
 // pairs' tangents ts for the SR and tl for the refreshed LR force.
 void launch_adj_pair(const Dev &d, const AdjDev &a, cudaStream_t s, const double *ts, const double *tl);
 void launch_adj_topo(const Dev &d, const AdjDev &a, cudaStream_t s, const double *tan, int mode);
-// the reverse pass of one recorded step: a.lam (after the step) -> a.lam (before it)
-void launch_adj_step(const Dev &d, const AdjDev &a, cudaStream_t s);
-// records the step's inputs into a.rx, a.rf, a.rlr (after the forces, before the integrator)
-void launch_adj_record(const Dev &d, const AdjDev &a, cudaStream_t s);
+// the reverse pass of one recorded step: a.lam (after the step) -> a.lam (before it), the
+// restraint terms on `side` between the events fork and join
+void launch_adj_step(const Dev &d, const AdjDev &a, cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join);
+// records the step's inputs into a.rx, a.rf, a.rg, a.rlr and its lists into to's (after the
+// forces, before the integrator)
+void launch_adj_record(const Dev &d, const AdjDev &a, const Dev &to, cudaStream_t s);
 // packed host-order state arrays (tis_set_states layout) <-> 9P device arrays
 void launch_adj_unpack(const Dev &d, cudaStream_t s, double *dst, const double *stage, int n, unsigned mask);
 void launch_adj_pack(const Dev &d, cudaStream_t s, const double *src, double *stage, int n);
