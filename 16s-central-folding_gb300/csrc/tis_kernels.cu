@@ -2448,26 +2448,28 @@ __global__ void k_rg(Dev d, int r, double *out)
 
 // Ions of one kind within sqrt(r2cut) of each phosphate of replica r, from the SR
 // lists (complete within the SR radius between rebuilds): count[i] for RNA bead i
-// (-1 for sugars and bases), hit[j] = 1 for every ion j within range of some P.
+// (-1 for sugars and bases), hit[j] = 1 for every ion j within range of some P.  A warp
+// per bead, its lanes over the list.
 __global__ void k_ion_counts(Dev d, int r, int kind, double r2cut, int *count, int *hit)
 {
     const RepParams *R = d.rp + r;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (i >= R->nrna) return;
     const int p = R->p0 + i;
-    if (((d.q[p].w >> 8) & 0xff) != 0) {
-        count[i] = -1;
-        return;
-    }
-    int c = 0;
-    for (int k = 0; k < d.n_sr[p]; ++k) {
-        const int j = d.nbr_sr[nb_idx(k, p, d.P)] & kIdxMask;
-        if (((d.q[j].w >> 8) & 0xff) == kind && exact_r2(d, R, p, j) <= r2cut) {
-            ++c;
-            hit[j - R->p0] = 1;
+    int c = -1;
+    if (((d.q[p].w >> 8) & 0xff) == 0) {
+        const int n = d.n_sr[p];
+        c = 0;
+        for (int k = lane; k < n; k += 32) {
+            const int j = d.nbr_sr[nb_idx(k, p, d.P)] & kIdxMask;
+            if (((d.q[j].w >> 8) & 0xff) == kind && exact_r2(d, R, p, j) <= r2cut) {
+                ++c;
+                hit[j - R->p0] = 1;
+            }
         }
+        c = __reduce_add_sync(kFull, c);
     }
-    count[i] = c;
+    if (lane == 0) count[i] = c;
 }
 
 // clears every replica's device-side error flags
@@ -2525,7 +2527,7 @@ void launch_list_peaks(const Dev &d, cudaStream_t s, int *out) { k_list_peaks<<<
 
 void launch_ion_counts(const Dev &d, cudaStream_t s, int r, int nrna, int kind, double r2cut, int *count, int *hit)
 {
-    k_ion_counts<<<(nrna + 127) / 128, 128, 0, s>>>(d, r, kind, r2cut, count, hit);
+    k_ion_counts<<<(nrna + 3) / 4, 128, 0, s>>>(d, r, kind, r2cut, count, hit);
 }
 
 void launch_pair(const Dev &d, cudaStream_t s, bool en, bool ex, int sr, int lr)

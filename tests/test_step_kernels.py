@@ -202,3 +202,44 @@ def test_gradients_of_small_and_full_blocks_agree():
     assert np.abs(ga[:2] - gb).max() <= 1e-9 * np.abs(gb).max()
     for k in STATE_NAMES:
         assert np.abs(da[k][:n] - db[k]).max() <= 1e-9 * max(1.0, np.abs(db[k]).max()), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["same", "turned", "half_turn", "noisy", "unrelated", "mirrored", "three", "line"])
+def test_fit_of_any_frame(kind):
+    """The least-squares fit's rmsd against a singular value decomposition's, for frames that
+    fit exactly, turned by any angle and by pi (a vanishing quaternion component), with noise,
+    unrelated, mirrored, of three beads, and on a line (a double eigenvalue)."""
+    rng = np.random.default_rng(len(kind))
+    s = load(golden_inputs(), "small")
+    e = Engine([s], precision=PREC_MIXED)
+    st = e.get_state(0)
+    beads = np.arange(0, 3 if kind == "three" else 60, 1).astype(np.int32)
+    if kind == "line":
+        t = np.linspace(-30, 30, len(beads))
+        for k, u in zip("xyz", (0.6, 0.0, 0.8)):
+            st[k][beads] = 100.0 + u * t
+            st["o" + k][beads] = st[k][beads]
+        e.set_state(0, st)
+    x = np.stack([st[k][beads] for k in "xyz"], 1)
+    q = {"half_turn": np.array([0.0, 0.6, 0.0, 0.8])}.get(kind, rng.normal(size=4))
+    q /= np.linalg.norm(q)
+    w, v = q[0], q[1:]
+    K = np.array([[0, -v[2], v[1]], [v[2], 0, -v[0]], [-v[1], v[0], 0]])
+    R = np.eye(3) if kind == "same" else np.eye(3) + 2 * w * K + 2 * K @ K
+    ref = (x - x.mean(0)) @ R.T + rng.normal(size=3) * 40
+    if kind == "noisy":
+        ref += rng.normal(size=ref.shape) * 3.0
+    elif kind == "unrelated":
+        ref = rng.normal(size=ref.shape) * 20.0
+    elif kind == "mirrored":
+        ref[:, 0] *= -1.0
+    g = e.density(0, 5, (0.0, 0.0, 0.0), 5.0, (40, 40, 40), beads, ref)
+    g.add()
+    rmsd = g.get()[2]
+    a, b = x - x.mean(0), ref - ref.mean(0)
+    U, sv, Vt = np.linalg.svd(a.T @ b)
+    sv[2] *= np.sign(np.linalg.det(Vt.T @ U.T)) or 1.0
+    want = np.sqrt(max(0.0, (a * a).sum() + (b * b).sum() - 2 * sv.sum()) / len(beads))
+    # the reference value cancels its sums: good to sqrt(2^-52) of the spread
+    assert abs(rmsd - want) < 3e-8 * np.sqrt((a * a).sum() / len(beads)) + 1e-9 * want, (rmsd, want)
