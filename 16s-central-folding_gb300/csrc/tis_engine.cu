@@ -320,12 +320,11 @@ void mark(Group *h, cudaStream_t s, int k, bool begin)
 }
 
 // deterministic_forces_MPI (E:2524-2586) in one launch: fixed-point atomics into one sum, the
-// LR sum kept apart.  make_noise: the step's Gaussians and recentring shifts too (launch_move
-// follows)
+// LR sum kept apart.  make_noise: the step's Gaussians too
 void enqueue_forces(Group *h, bool make_noise)
 {
     mark(h, h->stream, 0, true);
-    tis::launch_forces(h->dev, h->stream, make_noise, make_noise);
+    tis::launch_forces(h->dev, h->stream, make_noise);
     mark(h, h->stream, 0, false);
 }
 
@@ -770,12 +769,12 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
     for (int c = 0; c < 9; ++c)
         if ((rc = dupload(O, sd[c], st[c]))) return bail(rc);
     if ((rc = dalloc(O, &d.f, 3 * (size_t)h->P)) || (rc = dalloc(O, &d.flr, 3 * (size_t)h->P)) ||
-        (rc = dalloc(O, &d.gnoise, (size_t)h->R * tis::kNoiseStride)) || (rc = dalloc(O, &d.force_blocks, 1)) || (rc = dalloc(O, &d.cell_of, h->P)) ||
+        (rc = dalloc(O, &d.gnoise, (size_t)h->R * tis::kNoiseStride)) || (rc = dalloc(O, &d.centre, (size_t)h->R * tis::kCentre)) || (rc = dalloc(O, &d.cell_of, h->P)) ||
         (rc = dalloc(O, &d.cell_count, h->C)) || (rc = dalloc(O, &d.cell_start, h->C)) ||
         (rc = dalloc(O, &d.cell_fill, h->C)) || (rc = dalloc(O, &d.cell_list, h->P)) || (rc = dalloc(O, &d.qs, h->P)) ||
         (rc = dalloc(O, &d.n_sr, h->P)) || (rc = dalloc(O, &d.n_lr, h->P)) ||
         (rc = dalloc(O, &d.nbr_sr, (size_t)cap_sr * h->P)) || (rc = dalloc(O, &d.nbr_lr, (size_t)cap_lr * h->P)) ||
-        (rc = dalloc(O, &d.eterm, (size_t)h->R * tis::kNE)) || (rc = dalloc(O, &d.shift, (size_t)h->R * 3)) || 
+        (rc = dalloc(O, &d.eterm, (size_t)h->R * tis::kNE)) || 
         (rc = dalloc(O, &h->d_scalar, 4)) || (rc = dalloc(O, &h->stage, 9 * (size_t)h->npk)) ||
         (rc = dalloc(O, &h->d_e5, 5 * (size_t)h->R)) || (rc = dalloc(O, &h->d_peaks, 2)))
         return bail(rc);
@@ -1398,7 +1397,7 @@ static int grp_full_forces(Group *h)
 static int grp_move_rigid_units(Group *h)
 {
     if (!h) return fail(TIS_ERR_ARG, "null handle");
-    tis::launch_integrate(h->dev, h->stream);
+    tis::launch_move(h->dev, h->stream);
     TIS_CUDA(cudaGetLastError());
     return TIS_OK;
 }
@@ -1469,8 +1468,7 @@ static int grp_profile_stages(Group *h, int64_t n, double *ms)
         TIS_CUDA(cudaEventRecord(ev[3], h->stream));
         tis::launch_topology(d, h->stream, 16, false, true, true);
         TIS_CUDA(cudaEventRecord(ev[4], h->stream));
-        tis::launch_shift(d, h->stream);
-        TIS_CUDA(cudaEventRecord(ev[5], h->stream));
+        TIS_CUDA(cudaEventRecord(ev[5], h->stream));  // the shift is the integrator's
         tis::launch_move(d, h->stream);  // the skin check runs in its last blocks
         TIS_CUDA(cudaEventRecord(ev[6], h->stream));
         tis::launch_cells(d, h->stream);

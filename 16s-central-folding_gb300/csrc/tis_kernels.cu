@@ -6,7 +6,7 @@
 //                 E:1851-1907 every lr_interval steps or after a rebuild), bonded terms
 //                 (polymer_constraints E:2354-2520), stacks by term (E:1911-2141), H-bonds of
 //                 a replica per block with the valence-limited Monte Carlo (E:2145-2350),
-//                 full_forces' Gaussians (E:2590-2611), adjust_box's shift (E:2632-2656)
+//                 full_forces' Gaussians (E:2590-2611)
 //   k_integrate   full_forces (application) + move_rigid_units + leap_frog_move_atom + adjust_box
 //                                             E:2612-2732, E:570-642; its last block per
 //                 replica runs check_shifts      E:1741-1776
@@ -1584,29 +1584,19 @@ __global__ void __launch_bounds__(kHbThreads) k_hbond(Dev d, int do_hb, int make
     hbond_block<D, EN>(d, blockIdx.x, do_hb, make_noise, (int)threadIdx.x, (int)blockDim.x, CtaBar{});
 }
 
-// The recentring shift of adjust_box (E:2632-2656), the centre bead's new position moved
-// to the box centre, of replica r
-template <bool D>
-__device__ __forceinline__ void form_shift(const Dev &d, int r)
-{
-    const RepParams *R = d.rp + r;
-    double xn[3], vn[3];
-    leap_frog<D>(d, R, r, R->center, xn, vn);
-    for (int c = 0; c < 3; ++c) d.shift[3 * r + c] = R->hbox[c] - xn[c];
-}
-
 // deterministic_forces_MPI (E:2524-2586) with the step's Gaussians, of every replica of the
 // group in one launch: blocks [0, R) the H-bonds of a replica each (the longest chain, so
 // first), then the topology blocks, then the pairs, kForceThreads / TS sub-blocks of PB
-// particles per block.  With finish, the group's last block to end forms the recentring
-// shifts, for which every force of the centre beads must be in.
+// particles per block.
 // One launch instead of four on forked streams and one for the shift: a step is a chain of
 // kernels of a few microseconds, so each launch, fork and join in it counts (step of one
 // 346-nt replica 32.1 -> 24.7 us, of one 76-nt replica in FP64 96 -> 35 us), and an LR launch
 // with nothing due waited for room beside the other groups' work (64 replicas: 114 -> 107 us).
+// Blocks end without a word to one another: a count of ended blocks, whose last one formed
+// the recentring shift here, held every block for its fence (the integrator forms it now).
 // Two blocks of 512 threads per SM; FP64 needs the registers of one.
 template <bool D, int PB, int TS>
-__global__ void __launch_bounds__(kForceThreads, D ? 1 : 2) k_forces(Dev d, TopoPlan tp, int noise, int finish)
+__global__ void __launch_bounds__(kForceThreads, D ? 1 : 2) k_forces(Dev d, TopoPlan tp, int noise)
 {
     extern __shared__ __align__(16) unsigned char s_dyn[];
     const int tid = threadIdx.x;
@@ -1621,19 +1611,6 @@ __global__ void __launch_bounds__(kForceThreads, D ? 1 : 2) k_forces(Dev d, Topo
         if (pb * PB < d.P)
             pair_tasks<D, false, true, PB, TS>(d, pb, 1, 1, tid - sub * TS, ((PairSmem<PB> *)s_dyn)[sub],
                                                NamedBar{1 + sub, TS});
-    }
-    if (!finish) return;
-    __shared__ int s_last;
-    __syncthreads();  // every force of this block is issued
-    if (tid == 0) {
-        __threadfence();
-        s_last = atomicAdd(d.force_blocks, 1u) == gridDim.x - 1;
-        if (s_last) *d.force_blocks = 0u;
-    }
-    __syncthreads();
-    if (s_last) {
-        __threadfence();
-        for (int r = tid; r < d.R; r += kForceThreads) form_shift<D>(d, r);
     }
 }
 
@@ -1652,14 +1629,6 @@ __device__ inline bool above(double x, double L) { return __double_as_longlong(x
 __device__ inline bool bounded(double x)
 {
     return ((unsigned)(__double_as_longlong(x) >> 52) & 0x7ffu) < 1023u + 20u;
-}
-
-// the recentring shift alone (the drop-in move_rigid_units, stage timing)
-template <bool D>
-__global__ void k_shift(Dev d)
-{
-    wait_prior_grid();
-    if (threadIdx.x == 0) form_shift<D>(d, blockIdx.x);
 }
 
 // The five Energies-file values of replica r (E:6308-6312: E2_HB, E3_HB, E2_STACK,
@@ -1725,18 +1694,15 @@ __device__ void write_frame(const Dev &d, int r, long long klok, int tid, int nt
     }
 }
 
-// move_rigid_units for particle p of replica r (leap-frog, the recentring shift
-// sh, the ions' periodic wrap, the new fixed-point position, its force sum zeroed);
-// xn, xo: its new position and the old one, moved alike; est: leap_frog's estimate of
-// |xn - xo|^2.  False for a padding slot.
+// move_rigid_units for particle p of replica r after its leap-frog (xn, vn; the recentring
+// shift sh, the ions' periodic wrap, the new fixed-point position, its force sum zeroed);
+// xo: its old position, moved alike.  The centre bead's new state goes to `hold` when given
+// (a replica's place in Dev::centre) instead of the arrays, from which other blocks still
+// form the shift.
 template <bool D>
-__device__ __forceinline__ bool move_particle(const Dev &d, const RepParams *R, int r, int p, const double sh[3],
-                                              double xn[3], double xo[3], float2 *est, int &err)
+__device__ __forceinline__ void move_particle(const Dev &d, const RepParams *R, int p, int4 q, const double sh[3],
+                                              double xn[3], const double vn[3], double xo[3], double *hold, int &err)
 {
-    const int4 qp = d.q[p];
-    if (!((qp.w >> 16) & 1)) return false;
-    double vn[3];
-    leap_frog<D>(d, R, r, p, xn, vn, est);
     xo[0] = d.x[p];
     xo[1] = d.y[p];
     xo[2] = d.z[p];
@@ -1754,18 +1720,76 @@ __device__ __forceinline__ bool move_particle(const Dev &d, const RepParams *R, 
     bool ok = true;
     for (int c = 0; c < 3; ++c) ok = ok && bounded(xn[c]) && bounded(vn[c]);
     if (!ok) err |= kErrNonFinite;
+    q.x = fix_position(R, 0, xn[0]);
+    q.y = fix_position(R, 1, xn[1]);
+    q.z = fix_position(R, 2, xn[2]);
+    if (hold && p == R->center) {
+        for (int c = 0; c < 3; ++c) {
+            hold[c] = xn[c];
+            hold[3 + c] = xo[c];
+            hold[6 + c] = vn[c];
+        }
+        *(int4 *)(hold + 10) = q;
+        return;
+    }
     d.x[p] = xn[0]; d.y[p] = xn[1]; d.z[p] = xn[2];
     d.xo[p] = xo[0]; d.yo[p] = xo[1]; d.zo[p] = xo[2];
     d.vx[p] = vn[0]; d.vy[p] = vn[1]; d.vz[p] = vn[2];
     d.f[p] = 0ull;  // consumed: the next step's force kernels accumulate from zero
     d.f[d.P + p] = 0ull;
     d.f[2 * d.P + p] = 0ull;
-    int4 q = qp;
-    q.x = fix_position(R, 0, xn[0]);
-    q.y = fix_position(R, 1, xn[1]);
-    q.z = fix_position(R, 2, xn[2]);
     d.q[p] = q;
-    return true;
+}
+
+// the centre bead's held state into the arrays, by one thread, once every block has read them
+__device__ __forceinline__ void release_centre(const Dev &d, const RepParams *R, const double *hold)
+{
+    const int p = R->center;
+    double v[9];
+    for (int c = 0; c < 9; ++c) v[c] = __ldcg(hold + c);
+    const int4 q = __ldcg((const int4 *)(hold + 10));
+    d.x[p] = v[0]; d.y[p] = v[1]; d.z[p] = v[2];
+    d.xo[p] = v[3]; d.yo[p] = v[4]; d.zo[p] = v[5];
+    d.vx[p] = v[6]; d.vy[p] = v[7]; d.vz[p] = v[8];
+    d.f[p] = 0ull;
+    d.f[d.P + p] = 0ull;
+    d.f[2 * d.P + p] = 0ull;
+    d.q[p] = q;
+}
+
+// component c of the recentring shift of adjust_box (E:2632-2656), the centre bead's new
+// position moved to the box centre, by lane c of three (all lanes of the warp call): the
+// leap-frog of leap_frog with a lane per component, so that a warp issues a third of it
+template <bool D>
+__device__ __forceinline__ double shift_lane(const Dev &d, const RepParams *R, int r, int lane)
+{
+    const int c = min(lane, 2), p = R->center, P = d.P;
+    const int t = d.q[p].w & 0xff, k = (p - R->p0 + 1) % 1000;
+    const double *xs = c == 0 ? d.x : c == 1 ? d.y : d.z, *os = c == 0 ? d.xo : c == 1 ? d.yo : d.zo,
+                 *vs = c == 0 ? d.vx : c == 1 ? d.vy : d.vz;
+    const double x0 = xs[p], o0 = os[p], v0 = vs[p], g = step_noise(d, r)[k + 1000 * c];
+    double vn, xn;
+    if (D) {
+        double f = total_force<D>(d, p, c);
+        if (d.noise == 0) f = __dadd_rn(f, __dmul_rn(g, R->sigma[t]));
+        vn = __dadd_rn(__dmul_rn(R->k1[t], v0), __dmul_rn(R->k2[t], f));
+    } else {
+        const double kg = d.noise == 0 ? R->k2sig[t] : 0.0;
+        const long long fx = (long long)(__ldcg(d.f + c * P + p) + __ldcg(d.flr + c * P + p));
+        vn = fma(kg, g, fma(R->k2fix[t], fix_to_double(fx), R->k1[t] * v0));
+    }
+    const int hv = __reduce_max_sync(kFull, __double2hiint(vn) & 0x7fffffff);
+    if (hv >= R->vcut[t]) {
+        const double v[3] = {__shfl_sync(kFull, vn, 0), __shfl_sync(kFull, vn, 1), __shfl_sync(kFull, vn, 2)};
+        double vsq = R->vcap[t] * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+        if (vsq > 1.0) {
+            vsq = 1.0 / sqrt(vsq);
+            vn *= vsq;
+        }
+    }
+    if (D) xn = __dadd_rn(__dsub_rn(__dmul_rn(2.0, x0), o0), __dmul_rn(__dsub_rn(vn, v0), R->h));
+    else xn = fma(vn - v0, R->h, x0 + (x0 - o0));
+    return R->hbox[c] - xn;
 }
 
 // |xn - xo|^2 as a bit pattern (non-negative doubles order as integers)
@@ -1780,8 +1804,9 @@ __device__ __forceinline__ unsigned long long shift_bits(const double xn[3], con
 }
 
 // move_rigid_units (E:2660-2731) of one particle per thread, T threads per block: leap-frog,
-// the recentring shift, the periodic wrap of the ions; the replica's last block to
-// finish runs the skin check.
+// the recentring shift, which every block's first warp forms from the centre bead, the
+// periodic wrap of the ions; the replica's last block to finish writes the centre bead and
+// runs the skin check.
 // Bound by the FP64 pipe (a warp instruction takes it 16 cycles or more, 64 issue slots):
 // everything but the update itself runs on integers or FP32.  Of the largest
 // displacement, which check_shifts needs exactly, an FP32 estimate finds the block's
@@ -1789,6 +1814,9 @@ __device__ __forceinline__ unsigned long long shift_bits(const double xn[3], con
 // replicas, 344,903 particles, 51.3 -> 38.9 us; 16 replicas, 782,384 particles, 96 -> 70 us.
 // Handles of few particles for the GPU (Dev::wide) take blocks of 64 threads, so that the
 // FP64 work spreads over more SMs; with more they would only add blocks to schedule.
+// The shift costs a block a twelfth of its FP64 work and the centre bead a detour through
+// Dev::centre; formed at the end of the force launch it held that launch's blocks for a
+// fence and an atomic: step of 64 replicas 95.3 -> 92.7 us, of one 23.7 -> 21.4 us.
 template <bool D, int T>
 __global__ void __launch_bounds__(T) k_integrate(Dev d)
 {
@@ -1798,13 +1826,21 @@ __global__ void __launch_bounds__(T) k_integrate(Dev d)
     const RepParams *R = d.rp + r;
     __shared__ int s_est;
     __shared__ int s_last;
+    __shared__ double s_shift[3];
     if (threadIdx.x == 0) s_est = 0;
-    __syncthreads();
-    const double sh[3] = {d.shift[3 * r], d.shift[3 * r + 1], d.shift[3 * r + 2]};
     int err = 0;
     float2 est = make_float2(0.0f, 0.0f);
-    double xn[3], xo[3];
-    const bool on = move_particle<D>(d, R, r, p, sh, xn, xo, &est, err);
+    double xn[3], vn[3], xo[3];
+    const int4 q = d.q[p];
+    const bool on = (q.w >> 16) & 1;
+    if (on) leap_frog<D>(d, R, r, p, xn, vn, &est);
+    if (threadIdx.x < 32) {
+        const double s = shift_lane<D>(d, R, r, (int)threadIdx.x);
+        if (threadIdx.x < 3) s_shift[threadIdx.x] = s;
+    }
+    __syncthreads();
+    double *hold = d.centre + (size_t)r * kCentre;
+    if (on) move_particle<D>(d, R, p, q, s_shift, xn, vn, xo, hold, err);
     // check_shifts (E:1745-1762): max |x - x_old|^2 over the block (a NaN estimate orders above all)
     const int wm = __reduce_max_sync(kFull, on ? __float_as_int(est.x) & 0x7fffffff : 0);
     if ((threadIdx.x & 31) == 0) atomicMax(&s_est, wm);
@@ -1823,6 +1859,7 @@ __global__ void __launch_bounds__(T) k_integrate(Dev d)
     __syncthreads();
     if (s_last) {
         __threadfence();
+        if (threadIdx.x == 32) release_centre(d, R, hold);  // beside control_step's thread
         control_step(d, r);
         if (d.fr.every > 0) {  // a frame step: this block writes the replica's frame (all its blocks are done)
             __syncthreads();
@@ -2371,13 +2408,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_step_fused(Dev d, int step
         cluster_barrier();
         lap(0);
         ph[6] += lr_now ? 1 : 0;
-        if (tid == 0) {  // adjust_box's shift (E:2632-2656) from the centre bead's new position
-            double xn[3], vn[3];
-            leap_frog<D>(d, R, r, R->center, xn, vn);
-            for (int c = 0; c < 3; ++c) s_shift[c] = R->hbox[c] - xn[c];
-            if (rank == 0)
-                for (int c = 0; c < 3; ++c) d.shift[3 * r + c] = s_shift[c];  // as k_shift leaves it
-            s_max = 0ull;
+        if (warp == 0) {  // adjust_box's shift (E:2632-2656) from the centre bead's new position
+            const double s = shift_lane<D>(d, R, r, lane);
+            if (lane < 3) s_shift[lane] = s;
+            if (lane == 0) s_max = 0ull;
         }
         cluster_barrier();  // no CTA moves the centre bead before every CTA has read it
         lap(2);
@@ -2386,8 +2420,12 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_step_fused(Dev d, int step
             unsigned long long bits = 0ull;
             const int i1 = min(npad, (rank + 1) * per);
             for (int i = rank * per + tid; i < i1; i += kFusedThreads) {
-                double xn[3], xo[3];
-                if (move_particle<D>(d, R, r, p0 + i, sh, xn, xo, nullptr, err)) bits = max(bits, shift_bits(xn, xo));
+                const int4 q = d.q[p0 + i];
+                if (!((q.w >> 16) & 1)) continue;
+                double xn[3], vn[3], xo[3];
+                leap_frog<D>(d, R, r, p0 + i, xn, vn);
+                move_particle<D>(d, R, p0 + i, q, sh, xn, vn, xo, nullptr, err);
+                bits = max(bits, shift_bits(xn, xo));
             }
             for (int o = 16; o > 0; o >>= 1) {
                 const unsigned long long b = __shfl_down_sync(kFull, bits, o);
@@ -2566,24 +2604,24 @@ size_t forces_smem(const Dev &d)
 }
 
 template <bool D, int PB, int TS>
-void launch_forces_t(const Dev &d, cudaStream_t s, bool noise, bool finish)
+void launch_forces_t(const Dev &d, cudaStream_t s, bool noise)
 {
     const TopoPlan tp = topo_plan(d, noise);
     constexpr int per = PB * (kForceThreads / TS);  // particles per pair block
     k_forces<D, PB, TS><<<d.R + tp.blocks() + (d.P + per - 1) / per, kForceThreads, forces_smem<D, PB, TS>(d), s>>>(
-        d, tp, noise ? 1 : 0, finish ? 1 : 0);
+        d, tp, noise ? 1 : 0);
 }
 
 }  // namespace
 
-void launch_forces(const Dev &d, cudaStream_t s, bool noise, bool finish)
+void launch_forces(const Dev &d, cudaStream_t s, bool noise)
 {
     if (d.fp64) {
-        if (d.wide) launch_forces_t<true, 32, 512>(d, s, noise, finish);
-        else launch_forces_t<true, 32, 128>(d, s, noise, finish);
+        if (d.wide) launch_forces_t<true, 32, 512>(d, s, noise);
+        else launch_forces_t<true, 32, 128>(d, s, noise);
     } else {
-        if (d.wide) launch_forces_t<false, 32, 128>(d, s, noise, finish);
-        else launch_forces_t<false, 128, 128>(d, s, noise, finish);
+        if (d.wide) launch_forces_t<false, 32, 128>(d, s, noise);
+        else launch_forces_t<false, 128, 128>(d, s, noise);
     }
 }
 
@@ -2657,12 +2695,6 @@ void launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s, co
     cudaLaunchKernelEx(&cfg, kernel, d);
 }
 
-void launch_shift(const Dev &d, cudaStream_t s)
-{
-    if (d.fp64) launch_pdl(k_shift<true>, d.R, 32, 0, s, d);
-    else launch_pdl(k_shift<false>, d.R, 32, 0, s, d);
-}
-
 void launch_move(const Dev &d, cudaStream_t s)
 {
     if (d.wide) {
@@ -2672,12 +2704,6 @@ void launch_move(const Dev &d, cudaStream_t s)
         if (d.fp64) launch_pdl(k_integrate<true, kBlock>, d.nblk, kBlock, 0, s, d);
         else launch_pdl(k_integrate<false, kBlock>, d.nblk, kBlock, 0, s, d);
     }
-}
-
-void launch_integrate(const Dev &d, cudaStream_t s)
-{
-    launch_shift(d, s);
-    launch_move(d, s);
 }
 
 void launch_cells(const Dev &d, cudaStream_t s)
@@ -2702,7 +2728,7 @@ void launch_force_all_rebuild(const Dev &d, cudaStream_t s) { k_force_rebuild<<<
 
 void launch_rg(const Dev &d, cudaStream_t s, int replica, double *out) { k_rg<<<1, 256, 0, s>>>(d, replica, out); }
 
-// forces (+ Gaussians, recentring shift), integrate (+ skin check), cells, pair search
+// forces (+ Gaussians), integrate (+ recentring shift, skin check), cells, pair search
 int kernel_launches_per_step() { return 4; }
 
 size_t fused_smem(const Dev &d) { return (size_t)max(d.hb_smem, d.cell_smem); }

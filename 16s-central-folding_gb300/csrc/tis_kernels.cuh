@@ -69,14 +69,14 @@ struct Dev {
     int cidx_max, cpos_max;         // largest per-replica ca_cidx and hb_cpos lengths
     int hb_smem;                // dynamic shared bytes of the H-bond kernel (0: its arrays stay in global scratch)
     double *eterm;              // R x kNE (per-term energies, compute_forces only)
-    unsigned *force_blocks;     // force blocks of the running step that have ended
+    double *centre;             // R x kCentre: the centre bead's new state until every block has read the old one
     int wide;                   // 1: few particles for the GPU: force blocks of fewer particles each
-    double *shift;              // R x 3, recentring shift of the current step (adjust_box)
     const int *cell_rep;        // replica of every cell
     int *hb_rec;                // when not null: 1 per H-bond candidate formed after the step's Monte Carlo, else 0
     unsigned long long *fprof;  // when not null: the fused step kernel's phase times, kFusedPhases per replica (ns)
     FrameRing fr;               // frame output from inside the step (fr.every = 0: off)
 };
+constexpr int kCentre = 12;       // doubles of Dev::centre per replica: x, x_old, v, a gap, the packed position
 constexpr int kFusedPhases = 12;  // forces, H-bond chain, shift, move, control, rebuild, steps with LR, rebuild steps,
                                   // and the H-bond chain's restraint terms, Monte Carlo, forces, Gaussians
 
@@ -147,16 +147,14 @@ void launch_ion_counts(const Dev &d, cudaStream_t s, int r, int nrna, int kind, 
 // sr: 1 with the SR lists; lr: the LR lists never (0), of the replicas whose refresh is
 // due (1), of all replicas (2)
 void launch_pair(const Dev &d, cudaStream_t s, bool energies, bool excl_in_list, int sr, int lr);
-// the step's forces in one launch; noise: its Gaussians too; finish: the recentring shifts too
-void launch_forces(const Dev &d, cudaStream_t s, bool noise, bool finish);
+// the step's forces in one launch; noise: its Gaussians too
+void launch_forces(const Dev &d, cudaStream_t s, bool noise);
 void launch_topology(const Dev &d, cudaStream_t s, int mask, bool energies, bool make_noise, bool excl_in_list);
 void launch_noise(const Dev &d, cudaStream_t s);  // the step's Gaussians only
 int configure_kernels(const Dev &d);                  // kernel attributes (shared-memory limits); cudaError_t
-void launch_integrate(const Dev &d, cudaStream_t s);  // recentring shift, then the particles (the drop-in call)
 void launch_rebuild(const Dev &d, cudaStream_t s);  // gated on RepState::rebuild: cells, then pair search
-// the parts of launch_integrate and launch_rebuild, for stage timing
-void launch_shift(const Dev &d, cudaStream_t s);
-void launch_move(const Dev &d, cudaStream_t s);
+void launch_move(const Dev &d, cudaStream_t s);  // move_rigid_units with its recentring shift
+// the parts of launch_rebuild, for stage timing
 void launch_cells(const Dev &d, cudaStream_t s);
 void launch_search(const Dev &d, cudaStream_t s);
 void launch_force_all_rebuild(const Dev &d, cudaStream_t s);

@@ -346,9 +346,9 @@ int tis_profile_stages(tis_handle *h, int64_t n, double *ms);
  * events around each kernel, all groups' graphs replayed concurrently;
  * ms[TIS_N_STAGES] receives each kernel's mean duration per launch (one group,
  * one step), averaged over the steps and groups, with the other groups' work
- * running beside it.  The step runs its forces, Gaussians and recentring shift in
- * one launch: its duration is entry 0, and entries 1 to 4 are 0.  Advances every
- * replica by `steps` steps. */
+ * running beside it.  The step runs its forces and Gaussians in
+ * one launch and the recentring shift in the integrator's: entry 0 is the force launch, and
+ * entries 1 to 4 are 0.  Advances every replica by `steps` steps. */
 int tis_profile_in_step(tis_handle *h, int32_t steps, double *ms);
 
 /* The persistent fused step kernel (tis_run_params.fused_ctas) run for `steps`
