@@ -680,7 +680,7 @@ __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int 
             double ec = 0;
             if constexpr (!D) {
                 const int4 e4 = __ldg((const int4 *)nbr + (size_t)task_chunk(task) * P + p);
-                const int raw[4] = {e4.x, e4.y, e4.z, e4.w};
+                int raw[4] = {e4.x, e4.y, e4.z, e4.w};
                 const int4 qp = sm.q[pl];
                 const int tp = qp.w & 0xff;
                 const bool chp = is_charged((qp.w >> 8) & 0xff);
@@ -689,13 +689,19 @@ __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int 
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
                     if (k < cnt) qj[k] = __ldg(d.q + (raw[k] & kIdxMask));
+                // one copy of the entry's code, the four taking turns in its registers: the roles of
+                // this launch together overrun the instruction cache (64 replicas: 92.7 -> 87.7 us a step)
+#pragma unroll 1
+                for (int k = 0; k < cnt; ++k) {
+                    const float ljw = EX ? (float)(1 - (raw[0] >> kExclShift)) : 1.0f;
+                    pair_entry<false, EN>(d, R, p, qp, tp, chp, raw[0] & kIdxMask, qj[0], ljw, tb, kap, lo, hi, ax, ay, az,
+                                          err, e_lj, ec);
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (k < cnt) {
-                        const float ljw = EX ? (float)(1 - (raw[k] >> kExclShift)) : 1.0f;
-                        pair_entry<false, EN>(d, R, p, qp, tp, chp, raw[k] & kIdxMask, qj[k], ljw, tb, kap, lo, hi, ax,
-                                              ay, az, err, e_lj, ec);
+                    for (int u = 0; u < 3; ++u) {
+                        raw[u] = raw[u + 1];
+                        qj[u] = qj[u + 1];
                     }
+                }
                 if (ax | ay | az) {
                     unsigned long long *out = tlr ? d.flr : d.f;
                     atomic_add_fix(out + p, ax);
