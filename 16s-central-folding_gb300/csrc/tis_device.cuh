@@ -105,14 +105,20 @@ __host__ __device__ inline void philox4x32_10(uint32_t c[4], uint32_t k0, uint32
     }
 }
 
-// Draw k of the rand() stream of a replica: an integer in [1, 2^31-1].
+// A draw of the rand() stream from its Philox word: an integer in [1, 2^31-1].
+__host__ __device__ inline uint32_t rand_word(uint32_t w)
+{
+    const uint32_t v = w >> 1;
+    return v ? v : 1u;
+}
+
+// Draw k of the rand() stream of a replica.
 __host__ __device__ inline uint32_t rand_value(unsigned long long seed, unsigned long long k)
 {
     unsigned long long blk = k >> 2;
     uint32_t c[4] = {(uint32_t)blk, (uint32_t)(blk >> 32), 0u, 0u};
     philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
-    uint32_t v = c[k & 3u] >> 1;
-    return v ? v : 1u;
+    return rand_word(c[k & 3u]);
 }
 
 // v / (2^31 - 1) rounded to nearest double, for 1 <= v <= 2^31 - 1: the reference's

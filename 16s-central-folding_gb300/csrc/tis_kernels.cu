@@ -916,24 +916,50 @@ __device__ inline void leap_frog(const Dev &d, const RepParams *R, int r, int p,
     }
 }
 
-// the Gaussians of full_forces (E:2594-2606) made from draws c and c + 1
+// two Gaussians of full_forces (E:2594-2606) from the draws v1 and v2
 template <bool D>
-__device__ __forceinline__ void noise_pair(const RepParams *R, unsigned long long c, double *out)
+__device__ __forceinline__ double2 gaussians(uint32_t v1, uint32_t v2)
 {
-    const uint32_t v1 = rand_value(R->seed, c), v2 = rand_value(R->seed, c + 1);
     if (D) {  // Box-Muller as the reference forms it (E:2598-2606), in FP64
         const double a = sqrt(-2.0 * log(u31_ratio(v1)));
         const double b = 2.0 * 3.14159265358979323846 * u31_ratio(v2);
         double sn, cs;
         sincos(b, &sn, &cs);
-        out[0] = a * cs;
-        out[1] = a * sn;
-    } else {  // FP32 Box-Muller, radius accurate over the whole uniform range
-        const float a = bm_radius(v1);
-        float sn, cs;
-        sincospif(2.0f * ((float)v2 * (1.0f / 2147483647.0f)), &sn, &cs);
-        out[0] = (double)(a * cs);
-        out[1] = (double)(a * sn);
+        return make_double2(a * cs, a * sn);
+    }
+    // FP32 Box-Muller, radius accurate over the whole uniform range
+    const float a = bm_radius(v1);
+    float sn, cs;
+    sincospif(2.0f * ((float)v2 * (1.0f / 2147483647.0f)), &sn, &cs);
+    return make_double2((double)(a * cs), (double)(a * sn));
+}
+
+// Pairs of Gaussians from draw c0 on, pair k from draws c0 + 2 k and c0 + 2 k + 1: one Philox
+// block holds four draws, so thread j forms the (up to two) pairs of [0, pairs) whose first
+// draw lies in block c0 / 4 + j.  The Monte Carlo takes its draws in twos, so c0 is even and
+// a block's draws suffice; after an odd count the last pair takes one of the next block.
+// A quarter of the Philox blocks of a draw at a time: step of 64 replicas 85.6 -> 85.0 us,
+// the drop-in step 50.8 -> 49.9 us.
+__host__ __device__ constexpr int noise_blocks(int pairs) { return pairs / 2 + 1; }
+template <bool D>
+__device__ __forceinline__ void noise_block(unsigned long long seed, unsigned long long c0, int pairs, int j, double *out)
+{
+    const unsigned long long b = (c0 >> 2) + (unsigned long long)j;
+    uint32_t c[4] = {(uint32_t)b, (uint32_t)(b >> 32), 0u, 0u};
+    philox4x32_10(c, (uint32_t)seed, (uint32_t)(seed >> 32));
+    uint32_t v1 = rand_word(c[0]), v2 = rand_word(c[1]), v3 = rand_word(c[2]), v4 = rand_word(c[3]);
+    if (c0 & 1u) {
+        v1 = v2;
+        v2 = v3;
+        v3 = v4;
+        v4 = rand_value(seed, 4 * b + 4);
+    }
+    int k = 2 * j - (int)((c0 >> 1) & 1u);
+#pragma unroll 1
+    for (int i = 0; i < 2; ++i, ++k) {
+        if (k >= 0 && k < pairs) ((double2 *)out)[k] = gaussians<D>(v1, v2);
+        v1 = v3;
+        v2 = v4;
     }
 }
 
@@ -942,7 +968,7 @@ template <bool D>
 __device__ void gen_noise(const Dev &d, int r, unsigned long long c0, double *out, int tid, int nthr)
 {
     if (d.noise != 0) return;
-    for (int t = tid; t < kNoise / 2; t += nthr) noise_pair<D>(d.rp + r, c0 + 2 * t, out + 2 * t);
+    for (int j = tid; j < noise_blocks(kNoise / 2); j += nthr) noise_block<D>(d.rp[r].seed, c0, kNoise / 2, j, out);
 }
 
 // the step's Gaussians alone (the drop-in full_forces call), one block per replica;
@@ -1229,11 +1255,11 @@ __device__ __forceinline__ void topo_block(const Dev &d, const TopoPlan &tp, int
         return;
     }
     b -= tp.nb;
-    constexpr int kPairs = (kNoise + kNoiseSpare) / 2;
+    constexpr int kPairs = (kNoise + kNoiseSpare) / 2, kPer = noise_blocks(kPairs);
     const int item = b * tp.per + tid;
-    if (tid < tp.per && item < d.R * kPairs) {
-        const int r = item / kPairs, k = item - r * kPairs;
-        noise_pair<D>(d.rp + r, d.rs[r].ctr + 2 * k, d.gnoise + (size_t)r * kNoiseStride + 2 * k);
+    if (tid < tp.per && item < d.R * kPer) {
+        const int r = item / kPer;
+        noise_block<D>(d.rp[r].seed, d.rs[r].ctr, kPairs, item - r * kPer, d.gnoise + (size_t)r * kNoiseStride);
     }
 }
 
@@ -2597,7 +2623,7 @@ TopoPlan topo_plan(const Dev &d, bool noise)
     tp.n3 = (d.nst3 + 63) / 64;
     tp.n2 = (d.nst2 + 127) / 128;
     tp.nb = (d.nbt + tp.per - 1) / tp.per;
-    tp.nn = noise && d.noise == 0 ? (d.R * ((kNoise + kNoiseSpare) / 2) + tp.per - 1) / tp.per : 0;
+    tp.nn = noise && d.noise == 0 ? (d.R * noise_blocks((kNoise + kNoiseSpare) / 2) + tp.per - 1) / tp.per : 0;
     return tp;
 }
 

@@ -58,6 +58,25 @@ def test_fixed_point_to_double_by_integers():
         assert b | ((1 << 63) if v < 0 else 0) == _bits(float(v)), v
 
 
+@pytest.mark.parametrize("c0", [0, 1, 2, 3, 5046, 2 ** 32 - 2, 2 ** 32 + 3])
+@pytest.mark.parametrize("pairs", [1500, 1564])
+def test_noise_pairs_of_philox_blocks(pairs, c0):
+    """noise_block's split: over threads 0 .. pairs / 2 every pair k is formed once, from draws
+    c0 + 2 k and c0 + 2 k + 1, wherever in a block of four the first draw lies."""
+    got = {}
+    for j in range(pairs // 2 + 1):
+        b = (c0 >> 2) + j
+        v = [4 * b, 4 * b + 1, 4 * b + 2, 4 * b + 3]
+        if c0 & 1:
+            v = v[1:] + [4 * b + 4]
+        k = 2 * j - ((c0 >> 1) & 1)
+        for i in range(2):
+            if 0 <= k + i < pairs:
+                assert k + i not in got
+                got[k + i] = (v[2 * i], v[2 * i + 1])
+    assert got == {k: (c0 + 2 * k, c0 + 2 * k + 1) for k in range(pairs)}
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n_cl,n_k", [(0, 0), (27, 1), (27, 2), (261, 406), (261, 407), (261, 408)])
 def test_particle_counts_at_block_edges(n_cl, n_k):
