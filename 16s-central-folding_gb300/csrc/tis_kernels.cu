@@ -1845,7 +1845,7 @@ __device__ __forceinline__ unsigned long long shift_bits(const double xn[3], con
 }
 
 // move_rigid_units (E:2660-2731) of one particle per thread, T threads per block: leap-frog,
-// the recentring shift, which every block's first warp forms from the centre bead, the
+// the recentring shift, which a warp of every block forms from the centre bead, the
 // periodic wrap of the ions; the replica's last block to finish writes the centre bead and
 // runs the skin check.
 // Bound by the FP64 pipe (a warp instruction takes it 16 cycles or more, 64 issue slots):
@@ -1858,11 +1858,15 @@ __device__ __forceinline__ unsigned long long shift_bits(const double xn[3], con
 // The shift costs a block a twelfth of its FP64 work and the centre bead a detour through
 // Dev::centre; formed at the end of the force launch it held that launch's blocks for a
 // fence and an atomic: step of 64 replicas 95.3 -> 92.7 us, of one 23.7 -> 21.4 us.
-template <bool D, int T>
-__global__ void __launch_bounds__(T) k_integrate(Dev d)
+// E: threads of a further warp that forms the shift beside the others' leap-frog (wide handles:
+// the block's FP64 chain is what takes the time; step of one 346-nt replica 19.8 -> 18.8 us, of 7
+// replicas of 203 nt 32.1 -> 31.2 us, FP64 step 32.1 -> 31.2 us).  Full blocks have their first warp
+// do both: a fifth warp takes registers of blocks that would run beside (85.5 against 84.7 us).
+template <bool D, int T, int E>
+__global__ void __launch_bounds__(T + E) k_integrate(Dev d)
 {
     wait_prior_grid();
-    const int p = blockIdx.x * T + threadIdx.x;
+    const int p = blockIdx.x * T + (int)threadIdx.x;
     const int r = d.blk_rep[blockIdx.x * T / kBlock];
     const RepParams *R = d.rp + r;
     __shared__ int s_est;
@@ -1872,12 +1876,14 @@ __global__ void __launch_bounds__(T) k_integrate(Dev d)
     int err = 0;
     float2 est = make_float2(0.0f, 0.0f);
     double xn[3], vn[3], xo[3];
-    const int4 q = d.q[p];
+    int4 q = make_int4(0, 0, 0, 0);
+    if (E == 0 || threadIdx.x < T) q = d.q[p];
     const bool on = (q.w >> 16) & 1;
     if (on) leap_frog<D>(d, R, r, p, xn, vn, &est);
-    if (threadIdx.x < 32) {
-        const double s = shift_lane<D>(d, R, r, (int)threadIdx.x);
-        if (threadIdx.x < 3) s_shift[threadIdx.x] = s;
+    if (E == 0 ? threadIdx.x < 32 : threadIdx.x >= T) {
+        const int lane = (int)threadIdx.x & 31;
+        const double s = shift_lane<D>(d, R, r, lane);
+        if (lane < 3) s_shift[lane] = s;
     }
     __syncthreads();
     double *hold = d.centre + (size_t)r * kCentre;
@@ -2739,11 +2745,11 @@ void launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s, co
 void launch_move(const Dev &d, cudaStream_t s)
 {
     if (d.wide) {
-        if (d.fp64) launch_pdl(k_integrate<true, 64>, d.P / 64, 64, 0, s, d);
-        else launch_pdl(k_integrate<false, 64>, d.P / 64, 64, 0, s, d);
+        if (d.fp64) launch_pdl(k_integrate<true, 64, 32>, d.P / 64, 64 + 32, 0, s, d);
+        else launch_pdl(k_integrate<false, 64, 32>, d.P / 64, 64 + 32, 0, s, d);
     } else {
-        if (d.fp64) launch_pdl(k_integrate<true, kBlock>, d.nblk, kBlock, 0, s, d);
-        else launch_pdl(k_integrate<false, kBlock>, d.nblk, kBlock, 0, s, d);
+        if (d.fp64) launch_pdl(k_integrate<true, kBlock, 0>, d.nblk, kBlock, 0, s, d);
+        else launch_pdl(k_integrate<false, kBlock, 0>, d.nblk, kBlock, 0, s, d);
     }
 }
 
