@@ -83,7 +83,7 @@ struct RepState {
     int rebuild, lr_now, err, n_active;
     double e2hb, e3hb, e2st, e3st;
     double e2st_acc, e3st_acc;   // stacking energies being summed in the current step
-    unsigned blocks_done;        // integrator blocks finished this step (the last one runs the skin check)
+    unsigned blocks_done;        // integrator blocks finished this step (drop-in routine: the last one runs the skin check)
     unsigned pending;            // 1 + the Monte Carlo draws of the step in flight, which control_step books with its Gaussians (0: none)
 };
 

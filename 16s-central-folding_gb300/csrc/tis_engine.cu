@@ -259,7 +259,7 @@ int populate_launch(Group *h)
     // of the step's one (a warp per particle is latency-bound; more warps in flight)
     tis::Dev full = h->dev;
     full.search_warps = h->dev.sm_count * 24;
-    tis::launch_rebuild(full, h->stream);
+    tis::launch_rebuild(full, h->stream, 0);
     TIS_CUDA(cudaMemsetAsync(h->d_peaks, 0, 2 * sizeof(int), h->stream));
     tis::launch_list_peaks(h->dev, h->stream, h->d_peaks);
     TIS_CUDA(cudaGetLastError());
@@ -332,16 +332,17 @@ void enqueue_step(Group *h)
 {
     enqueue_forces(h, true);
     if (!h->pev) {
-        tis::launch_move(h->dev, h->stream);  // last block per replica: skin check
-        tis::launch_rebuild(h->dev, h->stream);
+        tis::launch_move(h->dev, h->stream, 0);
+        tis::launch_rebuild(h->dev, h->stream, 1);  // the skin check first
         return;
     }
     // the same launches with events between them (their programmatic dependent launch
     // then waits for the event nodes like a plain dependency)
-    void (*chain[3])(const tis::Dev &, cudaStream_t) = {tis::launch_move, tis::launch_cells, tis::launch_search};
     for (int k = 0; k < 3; ++k) {
         mark(h, h->stream, 5 + k, true);
-        chain[k](h->dev, h->stream);
+        if (k == 0) tis::launch_move(h->dev, h->stream, 0);
+        else if (k == 1) tis::launch_cells(h->dev, h->stream, 1);
+        else tis::launch_search(h->dev, h->stream);
         mark(h, h->stream, 5 + k, false);
     }
     ++h->pev_next;
@@ -1317,8 +1318,8 @@ static int grp_traj_grad(Group *h, int64_t steps, int K, const double *const *se
             enqueue_forces(h, true);
             h->dev.hb_rec = nullptr;
             tis::launch_adj_record(d, aj, dj, h->stream);
-            tis::launch_move(d, h->stream);
-            tis::launch_rebuild(d, h->stream);
+            tis::launch_move(d, h->stream, 0);
+            tis::launch_rebuild(d, h->stream, 1);
         }
         TIS_CUDA(cudaEventRecord(recorded[b], h->stream));
         TIS_CUDA(cudaStreamWaitEvent(back, recorded[b], 0));
@@ -1397,7 +1398,7 @@ static int grp_full_forces(Group *h)
 static int grp_move_rigid_units(Group *h)
 {
     if (!h) return fail(TIS_ERR_ARG, "null handle");
-    tis::launch_move(h->dev, h->stream);
+    tis::launch_move(h->dev, h->stream, 1);
     TIS_CUDA(cudaGetLastError());
     return TIS_OK;
 }
@@ -1406,7 +1407,7 @@ static int grp_check_shifts(Group *h)
 {
     if (!h) return fail(TIS_ERR_ARG, "null handle");
     // the displacement check itself ran at the end of tis_move_rigid_units
-    tis::launch_rebuild(h->dev, h->stream);
+    tis::launch_rebuild(h->dev, h->stream, 0);
     TIS_CUDA(cudaGetLastError());
     return TIS_OK;
 }
@@ -1469,9 +1470,9 @@ static int grp_profile_stages(Group *h, int64_t n, double *ms)
         tis::launch_topology(d, h->stream, 16, false, true, true);
         TIS_CUDA(cudaEventRecord(ev[4], h->stream));
         TIS_CUDA(cudaEventRecord(ev[5], h->stream));  // the shift is the integrator's
-        tis::launch_move(d, h->stream);  // the skin check runs in its last blocks
+        tis::launch_move(d, h->stream, 0);
         TIS_CUDA(cudaEventRecord(ev[6], h->stream));
-        tis::launch_cells(d, h->stream);
+        tis::launch_cells(d, h->stream, 1);
         TIS_CUDA(cudaEventRecord(ev[7], h->stream));
         tis::launch_search(d, h->stream);
         TIS_CUDA(cudaEventRecord(ev[8], h->stream));

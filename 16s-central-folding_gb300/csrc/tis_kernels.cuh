@@ -152,10 +152,12 @@ void launch_forces(const Dev &d, cudaStream_t s, bool noise);
 void launch_topology(const Dev &d, cudaStream_t s, int mask, bool energies, bool make_noise, bool excl_in_list);
 void launch_noise(const Dev &d, cudaStream_t s);  // the step's Gaussians only
 int configure_kernels(const Dev &d);                  // kernel attributes (shared-memory limits); cudaError_t
-void launch_rebuild(const Dev &d, cudaStream_t s);  // gated on RepState::rebuild: cells, then pair search
-void launch_move(const Dev &d, cudaStream_t s);  // move_rigid_units with its recentring shift
+// gated on RepState::rebuild: cells, then pair search; control: the step's skin check first, which sets it
+void launch_rebuild(const Dev &d, cudaStream_t s, int control);
+// move_rigid_units with its recentring shift; tail: and the skin check, else launch_cells' control has to follow
+void launch_move(const Dev &d, cudaStream_t s, int tail);
 // the parts of launch_rebuild, for stage timing
-void launch_cells(const Dev &d, cudaStream_t s);
+void launch_cells(const Dev &d, cudaStream_t s, int control);
 void launch_search(const Dev &d, cudaStream_t s);
 void launch_force_all_rebuild(const Dev &d, cudaStream_t s);
 void launch_rg(const Dev &d, cudaStream_t s, int replica, double *out);

@@ -118,6 +118,31 @@ def test_small_and_full_blocks_agree(precision, steps):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("copies", [1, 48])
+def test_skin_check_in_either_kernel(copies):
+    """The drop-in loop, whose integrator ends with the skin check, against steps, whose cell
+    kernel begins with it, over list rebuilds: bit for bit in mixed precision."""
+    systems = [load(golden_inputs(), "small", seed=s) for s in (3, 4)] * copies
+    a, b = Engine(systems, precision=PREC_MIXED), Engine(systems, precision=PREC_MIXED)
+    for e in (a, b):
+        e.populate_lists()
+    a.step(150)
+    for _ in range(150):
+        b.deterministic_forces()
+        b.full_forces()
+        b.move_rigid_units()
+        b.check_shifts()
+    for e in (a, b):
+        e.sync()
+    assert max(a.counters(r)[1] for r in range(len(systems))) > 1
+    for r in (0, len(systems) - 1):
+        assert a.counters(r) == b.counters(r)
+        x, y = a.get_state(r), b.get_state(r)
+        for k in STATE_NAMES:
+            assert np.array_equal(x[k], y[k]), k
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("precision", [PREC_MIXED, PREC_FP64])
 @pytest.mark.parametrize("box,full", [(60.0, 1), (60.0, 0), (67.0, 1), (99.5, 1), (101.0, 0), (133.5, 1), (200.0, 0)])
 def test_search_cells_of_any_grid(box, full, precision):
