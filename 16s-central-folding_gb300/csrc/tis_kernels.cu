@@ -1883,7 +1883,9 @@ __global__ void __launch_bounds__(T + E) k_integrate(Dev d, int tail)
     int4 q = make_int4(0, 0, 0, 0);
     if (E == 0 || threadIdx.x < T) q = d.q[p];
     const bool on = (q.w >> 16) & 1;
-    if (on) leap_frog<D>(d, R, r, p, xn, vn, &est);
+    // padding particles too (their state is zero and nothing of it is kept): the loads then
+    // need not wait for the type's (step of 64 replicas 83.9 -> 83.6 us, one 18.0 -> 17.9 us)
+    if (E == 0 || threadIdx.x < T) leap_frog<D>(d, R, r, p, xn, vn, &est);
     if (E == 0 ? threadIdx.x < 32 : threadIdx.x >= T) {
         const int lane = (int)threadIdx.x & 31;
         const double s = shift_lane<D>(d, R, r, lane);
