@@ -60,6 +60,10 @@ struct RepParams {
     float hf;                    // h in FP32
     // floor(x qinv) by integers (fix_position): qinv 2^k in 64 bits, the high word of 2 L, and the shifts
     struct { unsigned long long q; unsigned hi2l; int sh, fb; } qx[3];
+    // positions in fixed units (axis_fix): the high word of 2^(E - 10), 1.01 box as a high word above
+    // it, 2^(E - 40); displacements whose FP32 estimate (squared) is below e2min may be off by e2pad
+    struct { unsigned lo, span; float step; } ax[3];
+    float e2min, e2pad;
     double k2fix[10], k2sig[10];  // K2 * 2^-32 (fixed-point force to velocity), K2 * sigma (noise)
     // pair tables, 1..45 (E:2908-2938); dm = D_LJ - 1.5852
     float dlj2[46], dm[46], flj[46], elj[46], d2min[46], qclb[46];

@@ -849,6 +849,54 @@ __device__ __forceinline__ int fix_position(const RepParams *R, int c, double x)
     return (int)(unsigned)__double2ll_rd(x * R->qinv[c]);
 }
 
+// Sums of positions by integers, rounded as FP64 rounds them.  Full blocks use them, where
+// the FP64 pipe is what the integrator waits for (twelve of its 27 operations per particle
+// become some 200 integer instructions, 56 cycles of issue for 192 of the pipe: step of 16
+// large replicas 194.1 -> 187.6 us, of 64 replicas 83.1 -> 82.5 us); a handle of few particles
+// waits for the chain of one block, which they lengthen (one replica 19.8 -> 20.6 us).
+// x in units of 2^(E - 64) (2^E > 1.02 box), exactly, for 2^(E - 10) <= x < 1.01 box
+__device__ __forceinline__ bool axis_fix(const RepParams *R, int c, double x, unsigned long long &v)
+{
+    const unsigned hi = (unsigned)__double2hiint(x), o = hi - R->ax[c].lo;
+    v = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | (unsigned)__double2loint(x)) << (((o >> 20) + 2u) & 15u);
+    return o < R->ax[c].span;
+}
+
+// the double nearest to v units, ties to even, for v >= 2^54
+__device__ __forceinline__ double axis_value(const RepParams *R, int c, unsigned long long v)
+{
+    const unsigned z = (unsigned)__clz((int)(v >> 32));  // 0 .. 9
+    const unsigned long long w = v << z;
+    const unsigned low = (unsigned)w, up = (low & 0x7ffu) + ((low >> 11) & 1u) > 0x400u;
+    return __longlong_as_double((long long)((w >> 11) + ((unsigned long long)(R->ax[c].lo + (8u << 20) - (z << 20)) << 32) + up));
+}
+
+// a shift s in the same units, rounded to odd, so that its sum with a position rounds as the
+// exact one does; kNoShift when |s| >= 2^(E - 10)
+constexpr long long kNoShift = (long long)0x8000000000000000ull;
+__device__ __forceinline__ long long shift_fix(const RepParams *R, int c, double s)
+{
+    const unsigned hi = (unsigned)__double2hiint(s), a = hi & 0x7fffffffu;
+    if (a >= R->ax[c].lo) return kNoShift;
+    if (s == 0.0) return 0;
+    const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | (unsigned)__double2loint(s)) << 1;
+    const unsigned r = (R->ax[c].lo >> 20) - 1u - (a >> 20);
+    unsigned long long v = r < 64u ? m >> r : 0ull;
+    if (r >= 64u || v << r != m) v |= 1ull;
+    return (int)hi < 0 ? -(long long)v : (long long)v;
+}
+
+// x + s for the shift s = S units of axis c
+template <bool I>
+__device__ __forceinline__ double axis_add(const RepParams *R, int c, double x, double s, long long S)
+{
+    if (!I) return x + s;
+    unsigned long long v;
+    const bool ok = axis_fix(R, c, x, v) && S != kNoShift;
+    v += (unsigned long long)S;
+    return ok && v >= (1ull << 54) ? axis_value(R, c, v) : x + s;
+}
+
 // x as a float, its significand cut to 24 bits (0 below 2^-126, huge from 2^128 on)
 __device__ __forceinline__ float cut_to_float(double x)
 {
@@ -870,7 +918,7 @@ __device__ __forceinline__ const double *step_noise(const Dev &d, int r)
 // same update v' = K1 v + K2 (f + g sigma) as K1 v + (K2 2^-32) f_fix + (K2 sigma) g
 // with fused multiply-adds, and x' = x + (x - x_old) + (v' - v) h; the velocity
 // cap m v'^2 / (300 T) > 1 uses the precomputed m / (300 T) in both modes.
-template <bool D>
+template <bool D, bool I>
 __device__ inline void leap_frog(const Dev &d, const RepParams *R, int r, int p, double xn[3], double vn[3], float2 *e2 = nullptr)
 {
     const int t = d.q[p].w & 0xff;
@@ -904,24 +952,35 @@ __device__ inline void leap_frog(const Dev &d, const RepParams *R, int r, int p,
             for (int c = 0; c < 3; ++c) vn[c] *= vsq;
         }
     }
-    if (D) {
-        for (int c = 0; c < 3; ++c)
-            xn[c] = __dadd_rn(__dsub_rn(__dmul_rn(2.0, x0[c]), o0[c]), __dmul_rn(__dsub_rn(vn[c], v0[c]), R->h));
-    } else {
-        for (int c = 0; c < 3; ++c) xn[c] = fma(vn[c] - v0[c], R->h, x0[c] + (x0[c] - o0[c]));
+    // |x' - x|^2 in FP32, good to 1e-5 unless its two parts cancel (or it all but
+    // vanishes): then nothing (x) and an upper bound (y)
+    float s = 0.0f, parts = 0.0f;
+    for (int c = 0; c < 3; ++c) {
+        // 2 x0 - o0 rounded once, which is also what x0 + (x0 - o0) gives while the difference
+        // is exact: by integers while both are a usual place and the difference below 2^(E - 10)
+        unsigned long long X, O;
+        const bool in = axis_fix(R, c, x0[c], X) & axis_fix(R, c, o0[c], O);
+        const long long dif = (long long)(X - O);
+        X += (unsigned long long)dif;
+        double t;
+        float a;
+        if (I && in && (unsigned long long)(dif + (1ll << 54)) < (1ull << 55) && X >= (1ull << 54)) {
+            t = axis_value(R, c, X);
+            a = (float)(int)(dif >> 24) * R->ax[c].step;
+        } else {
+            const double e = x0[c] - o0[c];
+            t = D ? __dsub_rn(__dmul_rn(2.0, x0[c]), o0[c]) : x0[c] + e;
+            a = cut_to_float(e);
+        }
+        const double dv = vn[c] - v0[c];
+        xn[c] = D ? __dadd_rn(t, __dmul_rn(dv, R->h)) : fma(dv, R->h, t);
+        const float b = cut_to_float(dv) * R->hf, e = a + b;
+        s += e * e;
+        parts += a * a + b * b;
     }
     if (e2) {
-        // |x' - x|^2 in FP32, good to 1e-5 unless its two parts cancel (or it all but
-        // vanishes): then nothing (x) and an upper bound (y)
-        const float h = R->hf;
-        float s = 0.0f, parts = 0.0f;
-        for (int c = 0; c < 3; ++c) {
-            const float a = cut_to_float(x0[c] - o0[c]), b = cut_to_float(vn[c] - v0[c]) * h, e = a + b;
-            s += e * e;
-            parts += a * a + b * b;
-        }
-        const bool bad = s < 1.0e-30f || parts > 64.0f * s;
-        *e2 = make_float2(bad ? 0.0f : s, bad ? 2.1f * parts + 1.0e-30f : s);
+        const bool bad = s < R->e2min || parts > 64.0f * s;
+        *e2 = make_float2(bad ? 0.0f : s, bad ? 2.1f * parts + R->e2pad : s);
     }
 }
 
@@ -1737,20 +1796,21 @@ __device__ void write_frame(const Dev &d, int r, long long klok, int tid, int nt
 }
 
 // move_rigid_units for particle p of replica r after its leap-frog (xn, vn; the recentring
-// shift sh, the ions' periodic wrap, the new fixed-point position, its force sum zeroed);
-// xo: its old position, moved alike.  The centre bead's new state goes to `hold` when given
+// shift sh, shf in fixed units when I, the ions' periodic wrap, the new fixed-point position,
+// its force sum zeroed); xo: its old position, moved alike.  The centre bead's new state goes to `hold` when given
 // (a replica's place in Dev::centre) instead of the arrays, from which other blocks still
 // form the shift.
-template <bool D>
+template <bool D, bool I>
 __device__ __forceinline__ void move_particle(const Dev &d, const RepParams *R, int p, int4 q, const double sh[3],
-                                              double xn[3], const double vn[3], double xo[3], double *hold, int &err)
+                                              const long long shf[3], double xn[3], const double vn[3], double xo[3],
+                                              double *hold, int &err)
 {
     xo[0] = d.x[p];
     xo[1] = d.y[p];
     xo[2] = d.z[p];
     for (int c = 0; c < 3; ++c) {
-        xn[c] = xn[c] + sh[c];
-        xo[c] = xo[c] + sh[c];
+        xn[c] = axis_add<I>(R, c, xn[c], sh[c], shf[c]);
+        xo[c] = axis_add<I>(R, c, xo[c], sh[c], shf[c]);
     }
     if (p - R->p0 >= R->nrna) {  // periodic wrap of the ions (E:2676-2731)
         for (int c = 0; c < 3; ++c) {
@@ -1877,6 +1937,8 @@ __global__ void __launch_bounds__(T + E) k_integrate(Dev d, int tail)
     __shared__ int s_est;
     __shared__ int s_last;
     __shared__ double s_shift[3];
+    __shared__ long long s_shf[3];
+    constexpr bool I = T == kBlock;  // axis_fix
     if (threadIdx.x == 0) s_est = 0;
     int err = 0;
     float2 est = make_float2(0.0f, 0.0f);
@@ -1886,15 +1948,18 @@ __global__ void __launch_bounds__(T + E) k_integrate(Dev d, int tail)
     const bool on = (q.w >> 16) & 1;
     // padding particles too (their state is zero and nothing of it is kept): the loads then
     // need not wait for the type's (step of 64 replicas 83.9 -> 83.6 us, one 18.0 -> 17.9 us)
-    if (E == 0 || threadIdx.x < T) leap_frog<D>(d, R, r, p, xn, vn, &est);
+    if (E == 0 || threadIdx.x < T) leap_frog<D, I>(d, R, r, p, xn, vn, &est);
     if (E == 0 ? threadIdx.x < 32 : threadIdx.x >= T) {
         const int lane = (int)threadIdx.x & 31;
         const double s = shift_lane<D>(d, R, r, lane);
-        if (lane < 3) s_shift[lane] = s;
+        if (lane < 3) {
+            s_shift[lane] = s;
+            if (I) s_shf[lane] = shift_fix(R, lane, s);
+        }
     }
     __syncthreads();
     double *hold = d.centre + (size_t)r * kCentre;
-    if (on) move_particle<D>(d, R, p, q, s_shift, xn, vn, xo, hold, err);
+    if (on) move_particle<D, I>(d, R, p, q, s_shift, s_shf, xn, vn, xo, hold, err);
     // check_shifts (E:1745-1762): max |x - x_old|^2 over the block (a NaN estimate orders above all)
     const int wm = __reduce_max_sync(kFull, on ? __float_as_int(est.x) & 0x7fffffff : 0);
     if ((threadIdx.x & 31) == 0) atomicMax(&s_est, wm);
@@ -2488,8 +2553,8 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_step_fused(Dev d, int step
                 const int4 q = d.q[p0 + i];
                 if (!((q.w >> 16) & 1)) continue;
                 double xn[3], vn[3], xo[3];
-                leap_frog<D>(d, R, r, p0 + i, xn, vn);
-                move_particle<D>(d, R, p0 + i, q, sh, xn, vn, xo, nullptr, err);
+                leap_frog<D, false>(d, R, r, p0 + i, xn, vn);
+                move_particle<D, false>(d, R, p0 + i, q, sh, nullptr, xn, vn, xo, nullptr, err);
                 bits = max(bits, shift_bits(xn, xo));
             }
             for (int o = 16; o > 0; o >>= 1) {

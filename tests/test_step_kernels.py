@@ -46,6 +46,67 @@ def test_position_floor_by_integers(box):
     assert fast > 5000
 
 
+@pytest.mark.parametrize("box", [51.3, 65.0, 200.0, 250.98, 277.5, 350.0, 501.9, 502.0, 511.9, 1000.0, 4096.0])
+def test_position_sums_by_integers(box):
+    """The integrator's integer forms (axis_fix, axis_value, shift_fix; constants as tis_create
+    forms them) of x + s and of x + (x - x_old) against the FP64 operations, over the axis,
+    its ends, neighbours of powers of two, tiny, zero and largest shifts, and ties."""
+    rng = random.Random(int(10 * box))
+    e = math.frexp(1.02 * box)[1]
+    lo, M = (1023 + e - 10) << 20, 2 ** 64 - 1
+    span = (_bits(1.01 * box) >> 32) - lo
+
+    def fix(x):
+        hi = _bits(x) >> 32
+        o = (hi - lo) & 0xFFFFFFFF
+        return o < span, (((((hi & 0xFFFFF) | 0x100000) << 32) | (_bits(x) & 0xFFFFFFFF)) << (((o >> 20) + 2) & 15)) & M
+
+    def value(v):
+        z = 64 - v.bit_length()
+        assert 0 <= z <= 9
+        w = (v << z) & M
+        up = int((w & 0x7FF) + ((w >> 11) & 1) > 0x400)
+        return struct.unpack("<d", struct.pack("<Q", (w >> 11) + ((lo + (8 << 20) - (z << 20)) << 32) + up))[0]
+
+    def shift(s):
+        hi = _bits(s) >> 32
+        a = hi & 0x7FFFFFFF
+        if a >= lo:
+            return None
+        if s == 0.0:
+            return 0
+        m = ((((hi & 0xFFFFF) | 0x100000) << 32) | (_bits(s) & 0xFFFFFFFF)) << 1
+        r = (lo >> 20) - 1 - (a >> 20)
+        v = m >> r if r < 64 else 0
+        if r >= 64 or v << r != m:
+            v |= 1
+        return -v if hi >> 31 else v
+
+    least, fast = 2.0 ** (e - 10), [0, 0]
+    for k in range(20000):
+        x = rng.uniform(0, box) if k % 4 else rng.choice([box, least, 2.0 ** rng.randint(e - 12, e), 1.0099 * box, 0.0, -1.0])
+        x = math.nextafter(x, rng.choice([-1e9, 1e9])) if k % 3 == 0 else x
+        s = rng.choice([0.0, 5e-324, 1.0, rng.uniform(-1, 1), 2.0 ** -rng.randint(1, 70)]) * rng.choice([-1, 1]) * math.nextafter(least, 0)
+        if k % 5 == 0:  # half a unit in the last place of x, and beside it
+            s = math.ulp(x) / 2 * rng.choice([1, -1, 1 + 2.0 ** -52, 1 - 2.0 ** -53])
+        ok, v = fix(x)
+        if ok:
+            assert v == int(math.ldexp(x, 64 - e)) and math.ldexp(x, 64 - e) % 4 == 0
+        S = shift(s)
+        if ok and S is not None and (v + S) & M >= 2 ** 54:
+            fast[0] += 1
+            assert value((v + S) & M) == x + s, (x, s)
+        o = x - s
+        ok2, w = fix(o)
+        d = v - w
+        if ok and ok2 and -2 ** 54 <= d < 2 ** 54 and (v + d) & M >= 2 ** 54:
+            fast[1] += 1
+            assert value((v + d) & M) == x + (x - o) == 2.0 * x - o, (x, o)
+            a = (d >> 24) * 2.0 ** (e - 40)
+            assert abs(a - (x - o)) <= 2.0 ** (e - 40)
+    assert min(fast) > 10000
+
+
 def test_fixed_point_to_double_by_integers():
     """fix_to_double's arithmetic against the conversion, up to the 53 bits it covers."""
     rng = random.Random(7)
