@@ -126,7 +126,9 @@ struct Group {
     int npk = 0;              // particles of the group's replicas (unpadded)
     double *stage = nullptr;  // nine packed arrays of npk values (tis_traj_grad's seeds and state adjoints)
     double *d_e5 = nullptr;   // five energies per replica (tis_get_all_energies)
-    tis::RepState *h_rs = nullptr;  // pinned host copy of the replicas' state (list build checks)
+    tis::RepState *h_rs = nullptr;  // pinned host copy of the replicas' state (error flags, list build checks)
+    char *h_out = nullptr;          // pinned memory for a replica's forces or ion counts, made by the first
+    size_t h_out_bytes = 0;         // call that reads them (pinned_out)
     int *h_peaks = nullptr;         // pinned: largest SR and LR neighbour counts of the last list build
     int *d_peaks = nullptr;
     // parameter-derivative coefficients (tis_param_grad, tis_traj_grad)
@@ -151,6 +153,7 @@ struct Group {
         for (cudaEvent_t e : adj_event)
             if (e) cudaEventDestroy(e);
         if (h_rs) cudaFreeHost(h_rs);
+        if (h_out) cudaFreeHost(h_out);
         if (h_peaks) cudaFreeHost(h_peaks);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -158,13 +161,19 @@ struct Group {
 
 namespace {
 
-int check_flags(Group *h)
+// the replicas' error flags: the copy into pinned memory, and what it says once the group's
+// stream is synchronised.  A caller queues the copy behind its work (of every group) and
+// waits once; a copy to pageable memory would wait by itself.
+int flags_copy(Group *h)
 {
-    std::vector<tis::RepState> rs(h->R);
-    TIS_CUDA(cudaMemcpyAsync(rs.data(), h->dev.rs, sizeof(tis::RepState) * h->R, cudaMemcpyDeviceToHost, h->stream));
-    TIS_CUDA(cudaStreamSynchronize(h->stream));
+    TIS_CUDA(cudaMemcpyAsync(h->h_rs, h->dev.rs, sizeof(tis::RepState) * h->R, cudaMemcpyDeviceToHost, h->stream));
+    return TIS_OK;
+}
+
+int flags_verdict(Group *h)
+{
     for (int r = 0; r < h->R; ++r) {
-        const int e = rs[r].err;
+        const int e = h->h_rs[r].err;
         if (e & tis::kErrCapacity) return fail(TIS_ERR_CAPACITY, "replica %d: neighbour list capacity exceeded", h->base + r);
         if (e & tis::kErrRange) return fail(TIS_ERR_RANGE, "replica %d: a particle left the cell grid's range", h->base + r);
         if (e & tis::kErrNonFinite) return fail(TIS_ERR_NONFINITE, "replica %d: non-finite or runaway force/state", h->base + r);
@@ -172,15 +181,28 @@ int check_flags(Group *h)
     return TIS_OK;
 }
 
-int clear_flags(Group *h)
+int check_flags(Group *h)
 {
-    // err is the 4th int after 4 eight-byte counters and a double; clear via a host round trip
-    std::vector<tis::RepState> rs(h->R);
-    TIS_CUDA(cudaMemcpyAsync(rs.data(), h->dev.rs, sizeof(tis::RepState) * h->R, cudaMemcpyDeviceToHost, h->stream));
+    const int rc = flags_copy(h);
+    if (rc) return rc;
     TIS_CUDA(cudaStreamSynchronize(h->stream));
-    for (auto &s : rs) s.err = 0;
-    TIS_CUDA(cudaMemcpyAsync(h->dev.rs, rs.data(), sizeof(tis::RepState) * h->R, cudaMemcpyHostToDevice, h->stream));
-    TIS_CUDA(cudaStreamSynchronize(h->stream));
+    return flags_verdict(h);
+}
+
+// pinned memory for results of `bytes`, kept with the group (at most a replica's forces)
+int pinned_out(Group *h, size_t bytes, char **out)
+{
+    if (bytes > h->h_out_bytes) {
+        if (h->h_out) cudaFreeHost(h->h_out);
+        h->h_out = nullptr;
+        h->h_out_bytes = 0;
+        if (cudaMallocHost((void **)&h->h_out, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(TIS_ERR_NOMEM, "cudaMallocHost(%zu bytes) failed", bytes);
+        }
+        h->h_out_bytes = bytes;
+    }
+    *out = h->h_out;
     return TIS_OK;
 }
 
@@ -998,14 +1020,14 @@ static int grp_ion_counts(Group *h, int r, int kind, double radius, int32_t *cou
         return fail(TIS_ERR_ARG, "tis_ion_counts: radius %g outside (0, %g] (the SR radius)", radius, h->prm.sr);
     if (!h->lists_built && (rc = populate(h))) return rc;
     const RepHost &hr = h->rep[r];
-    int *d_cnt = nullptr, *d_hit = nullptr;
-    TIS_CUDA(cudaMallocAsync((void **)&d_cnt, sizeof(int) * (hr.nrna + hr.n), h->stream));
-    d_hit = d_cnt + hr.nrna;
+    char *pin = nullptr;
+    if ((rc = pinned_out(h, sizeof(int) * (hr.nrna + hr.n), &pin))) return rc;
+    int *d_cnt = (int *)h->stage, *d_hit = d_cnt + hr.nrna;  // the stage holds nine doubles per particle
     TIS_CUDA(cudaMemsetAsync(d_hit, 0, sizeof(int) * hr.n, h->stream));
     tis::launch_ion_counts(h->dev, h->stream, r, hr.nrna, kind, radius * radius, d_cnt, d_hit);
-    std::vector<int> c(hr.nrna + hr.n);
-    TIS_CUDA(cudaMemcpyAsync(c.data(), d_cnt, sizeof(int) * c.size(), cudaMemcpyDeviceToHost, h->stream));
-    TIS_CUDA(cudaFreeAsync(d_cnt, h->stream));
+    const int *c = (const int *)pin;
+    TIS_CUDA(cudaMemcpyAsync(pin, d_cnt, sizeof(int) * (hr.nrna + hr.n), cudaMemcpyDeviceToHost, h->stream));
+    if ((rc = flags_copy(h))) return rc;
     TIS_CUDA(cudaStreamSynchronize(h->stream));
     int64_t np = 0;
     for (int i = 0; i < hr.nrna; ++i)
@@ -1019,7 +1041,7 @@ static int grp_ion_counts(Group *h, int r, int kind, double radius, int32_t *cou
         for (int j = 0; j < hr.n; ++j) t += c[hr.nrna + j];
         *total = t;
     }
-    return check_flags(h);
+    return flags_verdict(h);
 }
 
 static int grp_get_hb_status(Group *h, int r, int32_t *status, int32_t *excess)
@@ -1040,8 +1062,14 @@ static int grp_compute_forces(Group *h, int r, int mask, double *forces, double 
     int rc = valid_replica(h, r);
     if (rc) return rc;
     if (!h->lists_built && (rc = populate(h))) return rc;
-    if ((rc = clear_flags(h))) return rc;
     const tis::Dev &d = h->dev;
+    const RepHost &hr = h->rep[r];
+    // energies, Rg, then the forces
+    const size_t n3 = forces ? 3 * (size_t)hr.n : 0;
+    char *pin = nullptr;
+    if ((rc = pinned_out(h, sizeof(double) * (tis::kNE + 1 + n3), &pin))) return rc;
+    double *out = (double *)pin;
+    tis::launch_clear_err(d, h->stream);
     TIS_CUDA(cudaMemsetAsync(d.eterm, 0, sizeof(double) * h->R * tis::kNE, h->stream));
     TIS_CUDA(cudaMemsetAsync(d.f, 0, sizeof(unsigned long long) * 3 * h->P, h->stream));
     const int m_sr = mask & TIS_TERM_SR ? 1 : 0, m_lr = mask & TIS_TERM_LR ? 2 : 0;
@@ -1050,42 +1078,22 @@ static int grp_compute_forces(Group *h, int r, int mask, double *forces, double 
     const int tmask = (mask & TIS_TERM_BONDED ? 4 : 0) | (mask & TIS_TERM_STACK ? 8 : 0) | (mask & TIS_TERM_HB ? 16 : 0);
     if (tmask) tis::launch_topology(d, h->stream, tmask, true, false, false);
     tis::launch_rg(d, h->stream, r, h->d_scalar);
+    if (n3) tis::launch_get_forces(d, h->stream, hr.p0, hr.n, h->stage);
     TIS_CUDA(cudaGetLastError());
-    const RepHost &hr = h->rep[r];
-    std::vector<unsigned long long> f(3 * (size_t)hr.n), fl(3 * (size_t)hr.n);
-    for (int c = 0; c < 3; ++c) {
-        TIS_CUDA(cudaMemcpyAsync(f.data() + c * hr.n, d.f + (size_t)c * h->P + hr.p0, 8 * hr.n, cudaMemcpyDeviceToHost, h->stream));
-        TIS_CUDA(cudaMemcpyAsync(fl.data() + c * hr.n, d.flr + (size_t)c * h->P + hr.p0, 8 * hr.n, cudaMemcpyDeviceToHost, h->stream));
-    }
-    double et[tis::kNE], rg = 0;
-    tis::RepState st;
-    TIS_CUDA(cudaMemcpyAsync(et, d.eterm + r * tis::kNE, sizeof et, cudaMemcpyDeviceToHost, h->stream));
-    TIS_CUDA(cudaMemcpyAsync(&rg, h->d_scalar, sizeof rg, cudaMemcpyDeviceToHost, h->stream));
-    TIS_CUDA(cudaMemcpyAsync(&st, d.rs + r, sizeof st, cudaMemcpyDeviceToHost, h->stream));
+    TIS_CUDA(cudaMemcpyAsync(out, d.eterm + r * tis::kNE, sizeof(double) * tis::kNE, cudaMemcpyDeviceToHost, h->stream));
+    TIS_CUDA(cudaMemcpyAsync(out + tis::kNE, h->d_scalar, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    if (n3) TIS_CUDA(cudaMemcpyAsync(out + tis::kNE + 1, h->stage, sizeof(double) * n3, cudaMemcpyDeviceToHost, h->stream));
+    if ((rc = flags_copy(h))) return rc;
     // the step's force kernels accumulate into a zero sum: leave it so
     TIS_CUDA(cudaMemsetAsync(d.f, 0, sizeof(unsigned long long) * 3 * h->P, h->stream));
     TIS_CUDA(cudaMemsetAsync(d.flr, 0, sizeof(unsigned long long) * 3 * h->P, h->stream));
     TIS_CUDA(cudaStreamSynchronize(h->stream));
-    if (forces)
-        for (int i = 0; i < hr.n; ++i)
-            for (int c = 0; c < 3; ++c) {
-                const size_t k = (size_t)c * hr.n + i;
-                double v;
-                if (d.fp64) {
-                    double a, b;
-                    memcpy(&a, &f[k], 8);
-                    memcpy(&b, &fl[k], 8);
-                    v = a + b;
-                } else {
-                    v = (double)(long long)(f[k] + fl[k]) / tis::kFixScale;
-                }
-                forces[3 * i + c] = v;
-            }
+    if (n3) memcpy(forces, out + tis::kNE + 1, sizeof(double) * n3);
     if (energies) {
-        for (int k = 0; k < tis::kNE; ++k) energies[k] = et[k];
-        energies[TIS_E_RG] = rg;
+        for (int k = 0; k < tis::kNE; ++k) energies[k] = out[k];
+        energies[TIS_E_RG] = out[tis::kNE];
     }
-    return check_flags(h);
+    return flags_verdict(h);
 }
 
 // ---------------------------------------------------------------------------
@@ -1129,7 +1137,7 @@ static int grp_param_grad(Group *h, double *out)
 {
     int rc;
     if (!h->lists_built && (rc = populate(h))) return rc;
-    if ((rc = clear_flags(h))) return rc;
+    tis::launch_clear_err(h->dev, h->stream);
     AdjMem M;
     tis::AdjDev a = adj_base(h);
     if ((rc = M.alloc(h, &a.dth, (size_t)h->R * tis::kNParams)) || (rc = M.alloc(h, &a.rhb, (size_t)h->nhb_all)))
@@ -1185,7 +1193,7 @@ static int grp_traj_grad(Group *h, int64_t steps, int K, const double *const *se
                          double *const *dstate0)
 {
     int rc;
-    if ((rc = clear_flags(h))) return rc;
+    tis::launch_clear_err(h->dev, h->stream);
     if ((rc = populate(h))) return rc;  // the run starts with populate_lists (E:6237): lists and LR force fresh
     const tis::Dev &d = h->dev;
     const size_t P = h->P, R = h->R;
@@ -1496,12 +1504,6 @@ static int grp_profile_stages(Group *h, int64_t n, double *ms)
     for (auto &e : ev) cudaEventDestroy(e);
     for (int k = 0; k < kS; ++k) ms[k] = acc[k] / (double)n;
     h->launches += n * tis::kernel_launches_per_step();
-    return check_flags(h);
-}
-
-static int grp_sync(Group *h)
-{
-    if (!h) return fail(TIS_ERR_ARG, "null handle");
     return check_flags(h);
 }
 
@@ -2658,9 +2660,12 @@ int tis_sync(tis_handle *h)
 {
     if (!h) return fail(TIS_ERR_ARG, "null handle");
     TIS_CUDA(cudaStreamSynchronize(h->stream));
+    int rc;
+    for (Group *g : h->groups)
+        if ((rc = flags_copy(g))) return rc;
     for (Group *g : h->groups) {
-        const int rc = grp_sync(g);
-        if (rc) return rc;
+        TIS_CUDA(cudaStreamSynchronize(g->stream));
+        if ((rc = flags_verdict(g))) return rc;
     }
     return TIS_OK;
 }

@@ -2640,6 +2640,14 @@ __global__ void k_ion_counts(Dev d, int r, int kind, double r2cut, int *count, i
     if (lane == 0) count[i] = c;
 }
 
+// the total force of particles p0 .. p0 + n - 1 as (x, y, z) triples
+__global__ void k_get_forces(Dev d, int p0, int n, double *out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    for (int c = 0; c < 3; ++c) out[3 * i + c] = d.fp64 ? total_force<true>(d, p0 + i, c) : total_force<false>(d, p0 + i, c);
+}
+
 // clears every replica's device-side error flags
 __global__ void k_clear_err(Dev d)
 {
@@ -2688,6 +2696,11 @@ void launch_get_state(const Dev &d, cudaStream_t s, double *stage, int n, unsign
 }
 
 void launch_energies(const Dev &d, cudaStream_t s, double *out) { k_energies<<<d.R, 256, 0, s>>>(d, out); }
+
+void launch_get_forces(const Dev &d, cudaStream_t s, int p0, int n, double *out)
+{
+    k_get_forces<<<(n + 127) / 128, 128, 0, s>>>(d, p0, n, out);
+}
 
 void launch_clear_err(const Dev &d, cudaStream_t s) { k_clear_err<<<1, 256, 0, s>>>(d); }
 

@@ -133,6 +133,7 @@ __host__ __device__ inline HbLayout hb_layout(int hb_nmax, int ca_nmax, int k_nm
 void launch_quantize(const Dev &d, cudaStream_t s);
 // the group's state packed (replicas end to end, n values per array, nine arrays) <-> device
 void launch_put_state(const Dev &d, cudaStream_t s, const double *stage, int n);
+void launch_get_forces(const Dev &d, cudaStream_t s, int p0, int n, double *out);
 void launch_get_state(const Dev &d, cudaStream_t s, double *stage, int n, unsigned mask);
 void launch_energies(const Dev &d, cudaStream_t s, double *out);  // 5 values per replica
 void launch_clear_err(const Dev &d, cudaStream_t s);              // RepState::err = 0 for every replica

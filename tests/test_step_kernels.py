@@ -179,6 +179,26 @@ def test_small_and_full_blocks_agree(precision, steps):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("precision", [PREC_MIXED, PREC_FP64])
+def test_forces_of_one_replica_among_others(precision):
+    """Force terms and ion counts of replicas of different sizes in one handle, read in turn,
+    against each replica alone: the results' pinned and device staging holds the largest."""
+    systems = [load(golden_inputs(), "small", seed=3, n_mg=1 if n else 0, n_cl=n, n_k=n) for n in (27, 0, 261, 28)]
+    many, ones = Engine(systems, precision=precision), [Engine([s], precision=precision) for s in systems]
+    for r, one in enumerate(ones):
+        for mask in (31, 2):
+            f, en = many.forces(r, mask)
+            # a call evaluates every replica of its handle and takes its Monte Carlo draws
+            g, eg = [e.forces(0, mask) for e in ones][r]
+            if precision == PREC_MIXED:
+                assert np.array_equal(f, g)
+            assert np.abs(f - g).max() <= 1e-9 * np.abs(g).max()  # FP64 sums run in any order
+            assert all(abs(en[k] - eg[k]) <= 1e-9 * max(1.0, abs(eg[k])) for k in en), mask
+        a, b = many.ion_counts(r, 5, 10.0), one.ion_counts(0, 5, 10.0)
+        assert np.array_equal(a[0], b[0]) and a[1] == b[1]
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("copies", [1, 48])
 def test_skin_check_in_either_kernel(copies):
     """The drop-in loop, whose integrator ends with the skin check, against steps, whose cell
