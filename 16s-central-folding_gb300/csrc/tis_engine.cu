@@ -765,6 +765,14 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
         d.search_warps = std::max(4, sms * (h->P >= 100000 ? 16 : 8));
         d.sm_count = std::max(1, sms);
         d.wide = total_blocks <= 4 * d.sm_count;
+        // a block of 1024 threads takes a whole SM's registers, so each step waits for an SM that
+        // runs nothing else; one of 512 fits beside a force block, but bins a replica more slowly.
+        // 1024 / 512 / 256 threads: 64 replicas of 5,400 particles 8.12 / 7.98 / 8.09 ms (100 steps),
+        // their list build and 20 steps 2.32 / 2.27 / 2.30 ms, 16 of 48,900 7.43 / 7.49 / - ms (40);
+        // between the two sizes nothing was measured
+        int npad_max = 0;
+        for (auto &Q : rp) npad_max = std::max(npad_max, Q.npad);
+        d.cell_threads = npad_max <= 20000 ? 512 : 1024;
         int nc_max = 1;
         for (auto &Q : rp) nc_max = std::max(nc_max, Q.nc);
         d.nc_max = nc_max;

@@ -2855,8 +2855,8 @@ void launch_move(const Dev &d, cudaStream_t s, int tail)
 
 void launch_cells(const Dev &d, cudaStream_t s, int control)
 {
-    if (d.fp64) launch_pdl(k_cells<true>, d.R, kCellThreads, d.cell_smem, s, d, control);
-    else launch_pdl(k_cells<false>, d.R, kCellThreads, d.cell_smem, s, d, control);
+    if (d.fp64) launch_pdl(k_cells<true>, d.R, d.cell_threads, d.cell_smem, s, d, control);
+    else launch_pdl(k_cells<false>, d.R, d.cell_threads, d.cell_smem, s, d, control);
 }
 
 void launch_search(const Dev &d, cudaStream_t s)

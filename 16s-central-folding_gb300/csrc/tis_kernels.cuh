@@ -70,6 +70,7 @@ struct Dev {
     int hb_smem;                // dynamic shared bytes of the H-bond kernel (0: its arrays stay in global scratch)
     double *eterm;              // R x kNE (per-term energies, compute_forces only)
     double *centre;             // R x kCentre: the centre bead's new state until every block has read the old one
+    int cell_threads;           // threads of the cell kernel's blocks
     int wide;                   // 1: few particles for the GPU: force blocks of fewer particles each
     const int *cell_rep;        // replica of every cell
     int *hb_rec;                // when not null: 1 per H-bond candidate formed after the step's Monte Carlo, else 0
