@@ -158,8 +158,9 @@ class ClockSampler:
 
 
 def fp32_roofline(device, clocks, entries_per_launch, launch_ms):
-    """The SR pair kernel against the FP32 roofline: its algorithmic FLOPs per launch
-    (FLOP_PER_SR_ENTRY per list entry) over its in-step duration, and the GPU's FP32
+    """The SR pairs against the FP32 roofline: their algorithmic FLOPs per launch
+    (FLOP_PER_SR_ENTRY per list entry) over the in-step duration of the force launch,
+    which holds the other force stages too, and the GPU's FP32
     peak at the SM clock sampled during the timed region (SMs x 128 lanes x 2)."""
     import torch
     sms = torch.cuda.get_device_properties(device).multi_processor_count
@@ -214,13 +215,13 @@ def stage_bytes(n, sr, lr, lr_frac, nreb, nrna, items, nhb, nrep):
 
 
 # DRAM bytes per replica of each step kernel's launch: dram__bytes_read.sum +
-# dram__bytes_write.sum of one launch over a group of 8 replicas (about 43k
-# particles; cold L2, serialised) divided by 8, from ncu captures of
-# `python bench.py --steps 40 --warmup 3 --no-extras --groups 8` with --clock-control
-# none, --kernel-name-base mangled and -k set to the kernel (None: no capture of a
-# stepping launch).  Scaled to the batch by the number of replicas.
-NCU_DRAM_BYTES_PER_REPLICA = {"pair_sr": 3.04e6 / 8, "pair_lr": None, "bonded": 1.24e6 / 8, "hbond": 0.479e6 / 8,
-                              "shift": 0.04e6 / 8, "integrate": 5.35e6 / 8, "cells": 0.03e6 / 8, "search": None}
+# dram__bytes_write.sum of one launch over a group of 5 or 6 replicas (28.7k particles;
+# cold L2, serialised) divided by 64 / 12, from the capture of profiles/ncu_step_kernels.md
+# ("pair_sr": the force launch, which holds the stages without an entry).  Scaled to the
+# batch by the number of replicas.
+NCU_DRAM_BYTES_PER_REPLICA = {"pair_sr": 3.24e6 * 12 / 64, "pair_lr": None, "bonded": None, "hbond": None,
+                              "shift": None, "integrate": 3.59e6 * 12 / 64, "cells": 0.095e6 * 12 / 64,
+                              "search": 0.063e6 * 12 / 64}
 
 
 # Algorithmic FP32 work of the SR pair kernel per list entry evaluated: the distance
@@ -230,11 +231,10 @@ NCU_DRAM_BYTES_PER_REPLICA = {"pair_sr": 3.04e6 / 8, "pair_lr": None, "bonded": 
 FLOP_PER_SR_ENTRY = 26
 
 
-# FP32 (FMA) pipe and issue-slot use of each kernel from its committed ncu capture
-# (`--set full`, one launch over a group of 8 replicas; profiles/ncu_full_*.md):
+# FP32 (FMA) pipe and issue-slot use of each kernel from the same capture:
 # sm__pipe_fma_cycles_active and smsp__issue_active as fractions of their peaks.
-NCU_FMA_PIPE = {"pair_sr": 0.0371, "hbond": 0.0621, "search": 0.0526, "bonded": 0.0632}
-NCU_ISSUE_ACTIVE = {"pair_sr": 0.1469, "hbond": 0.1379, "search": 0.1452, "bonded": 0.1523}
+NCU_FMA_PIPE = {"pair_sr": 0.0558, "integrate": 0.0226, "cells": 0.0107, "search": 0.0143}
+NCU_ISSUE_ACTIVE = {"pair_sr": 0.189, "integrate": 0.0998, "cells": 0.0479, "search": 0.0693}
 
 
 def cpu_sample(files, specs, steps, workers):

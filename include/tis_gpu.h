@@ -337,7 +337,7 @@ int tis_replica_size(tis_handle *h, int replica, int *n_particles);
  * between them, on each group's stream; ms[TIS_N_STAGES] receives the mean
  * duration per step, summed over the replica groups, of: SR pair forces, LR pair
  * forces, bonded + stacking terms, H-bonds + the step's Gaussians, recentring
- * shift, integrator (+ skin check), cell binning, pair search. */
+ * shift, integrator, cell binning (+ skin check), pair search. */
 #define TIS_N_STAGES 8
 int tis_profile_stages(tis_handle *h, int64_t n, double *ms);
 
