@@ -10,7 +10,7 @@ import pytest
 
 from oracle_bridge import Oracle
 from systems import golden_inputs, load
-from tis_gb300 import PREC_FP64, PREC_MIXED, STATE_NAMES, Engine
+from tis_gb300 import PREC_FP64, PREC_MIXED, STATE_NAMES, Engine, System
 
 
 def _bits(x):
@@ -196,6 +196,51 @@ def test_forces_of_one_replica_among_others(precision):
             assert all(abs(en[k] - eg[k]) <= 1e-9 * max(1.0, abs(eg[k])) for k in en), mask
         a, b = many.ion_counts(r, 5, 10.0), one.ion_counts(0, 5, 10.0)
         assert np.array_equal(a[0], b[0]) and a[1] == b[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [PREC_MIXED, PREC_FP64])
+@pytest.mark.parametrize("copies", [5, 6, 8])
+def test_monte_carlo_draws_around_the_spare_gaussians(copies, precision):
+    """Steps whose Monte Carlo draws fewer and more numbers than the Gaussians made beside it
+    leave room for (128): every H-bond candidate several times over and valences of one.  Draw
+    counts against the oracle's; states against its (FP64, 1e-7 A) or the drop-in loop's, which
+    draws its Gaussians after the Monte Carlo (bit for bit)."""
+    sd = load(golden_inputs(), "small").to_dict()
+    n, off, co, ci = len(sd["hb_E"]), sd["hb_atom_off"], sd["hba_cand_off"], sd["hba_cand_idx"]
+    for k in ("hb_E", "hb_dhs", "hb_dode", "hb_idx", "hb_native", "hb_atom_idx"):
+        sd[k] = np.tile(sd[k], copies)
+    sd["hb_atom_off"] = np.concatenate([off[:-1] + k * off[-1] for k in range(copies)] + [[copies * off[-1]]]).astype(np.int32)
+    sd["hba_cand_off"] = (copies * co).astype(np.int32)
+    sd["hba_cand_idx"] = np.concatenate([ci[co[a]:co[a + 1]] + k * n for a in range(len(co) - 1) for k in range(copies)]).astype(np.int32)
+    sd["hba_valence"] = np.minimum(sd["hba_valence"], 1).astype(np.int32)
+    s = System.from_arrays(sd)
+    o = Oracle(s.to_dict(), seed=3)
+    a, b = Engine([s], precision=precision), Engine([s], precision=precision)
+    for e in (o, a, b):
+        e.populate_lists()
+    drawn = []
+    for _ in range(20):
+        before = o.draws()
+        o.step(1)
+        drawn.append(o.draws() - before - 3000)
+        a.step(1)
+        a.sync()
+        if precision == PREC_FP64:
+            assert a.counters(0)[2] == o.draws()
+    assert max(drawn) <= 128 if copies == 5 else max(drawn) > 128
+    for _ in range(20):
+        b.deterministic_forces()
+        b.full_forces()
+        b.move_rigid_units()
+        b.check_shifts()
+    b.sync()
+    x, y, z = a.get_state(0), b.get_state(0), o.get_state()
+    assert a.counters(0) == b.counters(0)
+    for k in STATE_NAMES:
+        assert np.array_equal(x[k], y[k]) if precision == PREC_MIXED else np.abs(x[k] - y[k]).max() < 1e-9, k
+    if precision == PREC_FP64:
+        assert max(np.abs(x[k] - z[k]).max() for k in "xyz") < 1e-7
 
 
 @pytest.mark.gpu
