@@ -468,7 +468,8 @@ struct PairTables {
 
 // The force of one list entry (partner j, packed position qj, ljw: the weight of its LJ
 // term) on the particle p of type tp: mixed precision, added to (ax, ay, az) in fixed
-// point.  An LR entry (LR known, or lr set) is farther than any LJ range and charged.
+// point.  An LR entry has no LJ term (LR_interactions_lists, E:1851-1907), however far its
+// pair is: LR known, or a weight of zero.
 template <bool LR, bool EN>
 __device__ __forceinline__ void pair_entry(const Dev &d, const RepParams *R, int p, const int4 &qp, int tp, bool chp,
                                            int j, const int4 &qj, float ljw, const PairTables &tb, float kap, float lo,
@@ -711,7 +712,7 @@ __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int 
                 // this launch together overrun the instruction cache (64 replicas: 92.7 -> 87.7 us a step)
 #pragma unroll 1
                 for (int k = 0; k < cnt; ++k) {
-                    const float ljw = EX ? (float)(1 - (raw[0] >> kExclShift)) : 1.0f;
+                    const float ljw = tlr ? 0.0f : EX ? (float)(1 - (raw[0] >> kExclShift)) : 1.0f;
                     pair_entry<false, EN>(d, R, p, qp, tp, chp, raw[0] & kIdxMask, qj[0], ljw, tb, kap, lo, hi, ax, ay, az,
                                           err, e_lj, ec);
 #pragma unroll
@@ -729,7 +730,7 @@ __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int 
             } else {
                 const int raw = __ldg(nbr + nb_idx(task_chunk(task), p, P));
                 const int wp = sm.q[pl].w;
-                const double ljw = EX ? (double)(1 - (raw >> kExclShift)) : 1.0;
+                const double ljw = tlr ? 0.0 : EX ? (double)(1 - (raw >> kExclShift)) : 1.0;
                 double ax = 0, ay = 0, az = 0;
                 pair_entry<false, EN>(d, R, p, wp & 0xff, is_charged((wp >> 8) & 0xff), raw & kIdxMask,
                                       __ldg(&d.q[raw & kIdxMask].w), ljw, ax, ay, az, e_lj, ec);

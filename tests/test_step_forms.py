@@ -1,0 +1,55 @@
+"""What the step's kernels and the calls around them hold to in every form they take: which
+terms a list entry has, the order of FP64 sums, the memory a call leaves behind."""
+import numpy as np
+import pytest
+
+from oracle_bridge import Oracle
+from systems import golden_inputs, load, rel_err
+from tis_gb300 import PREC_FP64, PREC_MIXED, STATE_NAMES, TERM_LR, Engine
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,tol", [(PREC_MIXED, 1e-5), (PREC_FP64, 1e-10)])
+def test_lr_entries_inside_the_contact_distance(precision, tol):
+    """An SR list radius (4 A) below the contact distances of phosphate and K+ (4.76 A): the pairs
+    between the two are LR entries and feel Coulomb alone (E:1851-1907).  The LR term against the
+    oracle's (the per-term bounds), one step against the oracle's in FP64 (1e-7 A) and against the
+    persistent kernel's in mixed precision (bit for bit)."""
+    s = load(golden_inputs(), "small")
+    e = Engine([s], precision=PREC_FP64)
+    e.populate_lists()
+    e.step(300)
+    e.sync()
+    st = e.get_state(0)
+    o = Oracle(s.to_dict(), seed=3, sr=3.0, skin=1.0)
+    o.set_state(st)
+    o.populate_lists()
+    sd = s.to_dict()
+    i, j = np.asarray(o.pairs(1)).reshape(-1, 2).T
+    dv = np.stack([st[k][i] - st[k][j] for k in "xyz"], 1)
+    r = np.sqrt(((dv - 200.0 * np.round(dv / 200.0)) ** 2).sum(1))
+    typ, rlj = sd["type"], sd["rlj"]
+    assert (r < np.where(np.maximum(typ[i], typ[j]) <= 6, 3.2, rlj[typ[i] - 1] + rlj[typ[j] - 1])).sum() > 0
+    ref = o.terms()
+    a = Engine([s], precision=precision, sr=3.0, skin=1.0)
+    a.set_state(0, st)
+    a.populate_lists()
+    f, en = a.forces(0, TERM_LR)
+    assert rel_err(f, ref["F_lr"]) < tol and en["E_lj"] == 0.0
+    assert en["E_coul_lr"] == pytest.approx(ref["E_coul_lr"], rel=tol)
+    a.step(1)
+    a.sync()
+    x = a.get_state(0)
+    if precision == PREC_FP64:
+        o.step(1)
+        y = o.get_state()
+        assert max(np.abs(x[k] - y[k]).max() for k in "xyz") < 1e-7
+        return
+    b = Engine([s], precision=precision, sr=3.0, skin=1.0, fused_ctas=1)
+    b.set_state(0, st)
+    b.populate_lists()
+    b.step(1)
+    b.sync()
+    y = b.get_state(0)
+    for k in STATE_NAMES:
+        assert np.array_equal(x[k], y[k]), k
