@@ -636,11 +636,65 @@ struct NamedBar {
 };
 
 
-template <int PB>
+template <bool D, int PB>
 struct PairSmem {
     float dlj2[46], dm[46], flj[46], qclb[46];
     int4 q[PB];          // packed positions of the particles
     TaskSmem<PB> tasks;
+};
+template <int PB>
+struct PairSmem<true, PB> : PairSmem<false, PB> {
+    double f[3][kPairTasks];  // the forces of the window's tasks
+};
+
+// FP64 sums of the tasks' forces in an order that the lists alone set, so that the same state
+// gives the same force, whatever the handle's other replicas and the launch's shape: one
+// thread sums a particle's SR entries in list order, four its LR entries, entry k by
+// thread k % 4.  One task is one entry here, and a particle's are numbered end to end, SR first.
+template <int PB>
+struct OrderedSums {
+    double sr[3] = {0, 0, 0}, lr[3] = {0, 0, 0};
+    // the tasks win .. win + nt - 1, between barriers
+    __device__ __forceinline__ void window(const PairSmem<true, PB> &sm, int tid, int win, int nt)
+    {
+        if (tid < PB) {
+            int lo, ns, nl;
+            place(sm, tid, win, lo, ns, nl);
+            for (int k = max(lo, 0), e = min(lo + ns, nt); k < e; ++k)
+                for (int c = 0; c < 3; ++c) sr[c] += sm.f[c][k];
+        }
+        if (tid < 4 * PB) {
+            int lo, ns, nl;
+            place(sm, tid >> 2, win, lo, ns, nl);
+            lo += ns;
+            const int e = min(lo + nl, nt), j = tid & 3;
+            for (int k = lo + (lo < 0 ? ((-lo - j + 3) & ~3) : 0) + j; k < e; k += 4)
+                for (int c = 0; c < 3; ++c) lr[c] += sm.f[c][k];
+        }
+    }
+    // a particle's first task, counted from the window's first, and its list lengths
+    static __device__ __forceinline__ void place(const PairSmem<true, PB> &sm, int pl, int win, int &lo, int &ns, int &nl)
+    {
+        const int4 at = sm.tasks.at[pl];
+        lo = at.x - win;
+        for (int v = 0; v < (pl >> 5); ++v) lo += sm.tasks.cnt[v].x;
+        ns = at.z;
+        nl = at.w;
+    }
+    __device__ __forceinline__ void store(const Dev &d, int p0, int tid, bool do_lr) const
+    {
+        double *f = (double *)d.f, *flr = (double *)d.flr;
+        const int P = d.P;
+        if (tid < PB && (sr[0] != 0 || sr[1] != 0 || sr[2] != 0))  // beside the other terms' atomics
+            for (int c = 0; c < 3; ++c) atomicAdd(f + c * P + p0 + tid, sr[c]);
+        if (do_lr && tid < 4 * PB)
+            for (int c = 0; c < 3; ++c) {
+                double v = lr[c];
+                v += __shfl_xor_sync(kFull, v, 1);
+                v += __shfl_xor_sync(kFull, v, 2);
+                if ((tid & 3) == 0) flr[c * P + p0 + (tid >> 2)] = v;
+            }
+    }
 };
 
 // Pair forces of PB particles (sub-block pb) by the TS threads of one sub-block, over
@@ -649,14 +703,14 @@ struct PairSmem {
 //
 // Their list entries are dealt out as tasks (tis_tasks.cuh): a thread per particle took one
 // dependent load after another for as long as its warp's longest list.  FP64 tasks hold
-// one entry: FP64 latency and the narrow FP64 pipe bound them.
+// one entry: FP64 latency and the narrow FP64 pipe bound them; their sums keep an order (OrderedSums).
 // Alone, SR lists of 5 replicas of a 346-nt chain: 22.3 -> 11.9 us; one 76-nt replica in
 // FP64: 52 -> 15 us.
 template <bool D, bool EN, bool EX, int PB, int TS, class Bar>
-__device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int do_lr, int tid, PairSmem<PB> &sm, Bar bar)
+__device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int do_lr, int tid, PairSmem<D, PB> &sm, Bar bar)
 {
     constexpr int U = D ? 1 : 4;  // entries per task
-    static_assert(TS >= PB, "a thread per particle");
+    static_assert(TS >= (D ? 4 * PB : PB), "a thread per particle; for FP64 sums four");
     const int p0 = pb * PB, r = d.blk_rep[p0 / kBlock], P = d.P;
     const RepParams *R = d.rp + r;
     const bool lr = do_lr == 2 || (do_lr == 1 && d.rs[r].lr_now);
@@ -676,14 +730,15 @@ __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int 
         sm.q[tid] = qp;
         const bool act = (qp.w >> 16) & 1;
         const int ns = act && do_sr ? d.n_sr[p] : 0, nl = act && lr ? d.n_lr[p] : 0;
-        if (lr)  // the LR force is kept for the MTS interval: started again here, its tasks add to it
-            for (int c = 0; c < 3; ++c) d.flr[c * P + p] = 0ull;  // FP64 mode: 0.0 has the same bits
+        if (!D && lr)  // the LR force is kept for the MTS interval: started again here, its tasks add to it
+            for (int c = 0; c < 3; ++c) d.flr[c * P + p] = 0ull;
         tasks_count<PB, U>(sm.tasks, tid, ns, nl);
     }
     bar();
     const int total = tasks_total(sm.tasks);
     int err = 0;
     double e_lj = 0, e_c = 0, e_cl = 0;
+    typename std::conditional<D, OrderedSums<PB>, int>::type sums{};
     for (int win = 0; win < total; win += kPairTasks) {
         if (win) bar();  // the previous window's tasks are done
         if (tid < PB) tasks_window<PB, U>(sm.tasks, tid, win);
@@ -734,19 +789,21 @@ __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int 
                 double ax = 0, ay = 0, az = 0;
                 pair_entry<false, EN>(d, R, p, wp & 0xff, is_charged((wp >> 8) & 0xff), raw & kIdxMask,
                                       __ldg(&d.q[raw & kIdxMask].w), ljw, ax, ay, az, e_lj, ec);
-                if (ax != 0 || ay != 0 || az != 0) {
-                    double *out = (double *)(tlr ? d.flr : d.f);
-                    atomicAdd(out + p, ax);
-                    atomicAdd(out + P + p, ay);
-                    atomicAdd(out + 2 * P + p, az);
-                }
+                sm.f[0][t] = ax;
+                sm.f[1][t] = ay;
+                sm.f[2][t] = az;
             }
             if (EN) {
                 if (tlr) e_cl += ec;
                 else e_c += ec;
             }
         }
+        if constexpr (D) {
+            bar();
+            sums.window(sm, tid, win, nt);
+        }
     }
+    if constexpr (D) sums.store(d, p0, tid, lr);
     if (EN) {
         for (int o = 16; o > 0; o >>= 1) {
             e_lj += __shfl_down_sync(kFull, e_lj, o);
@@ -769,7 +826,7 @@ constexpr int kPairAlone = 128;
 template <bool D, bool EN, bool EX>
 __global__ void __launch_bounds__(kPairAlone) k_pair(Dev d, int do_sr, int do_lr)
 {
-    __shared__ PairSmem<32> sm;
+    __shared__ PairSmem<D, 32> sm;
     pair_tasks<D, EN, EX, 32, kPairAlone>(d, blockIdx.x, do_sr, do_lr, (int)threadIdx.x, sm, CtaBar{});
 }
 
@@ -1714,7 +1771,7 @@ __global__ void __launch_bounds__(kForceThreads, D ? 1 : 2) k_forces(Dev d, Topo
         constexpr int kSub = kForceThreads / TS;
         const int sub = tid / TS, pb = (b - tp.blocks()) * kSub + sub;
         if (pb * PB < d.P)
-            pair_tasks<D, false, true, PB, TS>(d, pb, 1, 1, tid - sub * TS, ((PairSmem<PB> *)s_dyn)[sub],
+            pair_tasks<D, false, true, PB, TS>(d, pb, 1, 1, tid - sub * TS, ((PairSmem<D, PB> *)s_dyn)[sub],
                                                NamedBar{1 + sub, TS});
     }
 }
@@ -2767,7 +2824,7 @@ void launch_pdl(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s, co
 template <bool D, int PB, int TS>
 size_t forces_smem(const Dev &d)
 {
-    const size_t pair = sizeof(PairSmem<PB>) * (kForceThreads / TS), topo = sizeof(Real<D>) * 16 * 32;
+    const size_t pair = sizeof(PairSmem<D, PB>) * (kForceThreads / TS), topo = sizeof(Real<D>) * 16 * 32;
     size_t m = pair > topo ? pair : topo;
     return m > (size_t)d.hb_smem ? m : (size_t)d.hb_smem;
 }

@@ -5,7 +5,7 @@ import pytest
 
 from oracle_bridge import Oracle
 from systems import golden_inputs, load, rel_err
-from tis_gb300 import PREC_FP64, PREC_MIXED, STATE_NAMES, TERM_LR, Engine
+from tis_gb300 import PREC_FP64, PREC_MIXED, STATE_NAMES, TERM_LR, TERM_SR, Engine
 
 
 @pytest.mark.gpu
@@ -53,3 +53,36 @@ def test_lr_entries_inside_the_contact_distance(precision, tol):
     y = b.get_state(0)
     for k in STATE_NAMES:
         assert np.array_equal(x[k], y[k]), k
+
+
+@pytest.mark.gpu
+def test_fp64_pair_forces_keep_an_order():
+    """FP64 SR and held LR forces are the same bits on every evaluation, and in a handle large
+    enough for full blocks: each particle's entries are summed in an order its list alone sets.
+    Also against the oracle's terms (1e-10, the FP64 bound)."""
+    s = load(golden_inputs(), "small")
+    e, many = Engine([s], precision=PREC_FP64), Engine([s] * 96, precision=PREC_FP64)
+    e.populate_lists()
+    e.step(300)
+    e.sync()
+    st = e.get_state(0)
+    e.set_state(0, st)
+    e.populate_lists()
+    o = Oracle(s.to_dict(), seed=3)
+    o.set_state(st)
+    o.populate_lists()
+    ref = o.terms()
+    for term, name in ((TERM_SR, "F_sr"), (TERM_LR, "F_lr")):
+        f = e.forces(0, term)[0]
+        assert rel_err(f, ref[name]) < 1e-10
+        for _ in range(20):
+            assert np.array_equal(f, e.forces(0, term)[0])
+    # ions feel SR and LR forces alone: one thread's sum of each, in both launch shapes
+    many.set_states({k: np.tile(st[k], 96) for k in STATE_NAMES})
+    many.populate_lists()
+    ions = slice(3 * int(s["n_rna"][0]), None)
+    for h in (e, many):
+        h.deterministic_forces()
+    f = e.current_forces(0)[ions]
+    for r in (0, 41, 95):
+        assert np.array_equal(f, many.current_forces(r)[ions])
