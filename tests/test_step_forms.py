@@ -86,3 +86,30 @@ def test_fp64_pair_forces_keep_an_order():
     f = e.current_forces(0)[ions]
     for r in (0, 41, 95):
         assert np.array_equal(f, many.current_forces(r)[ions])
+
+
+@pytest.mark.gpu
+def test_gradient_memory_of_a_handle_of_groups():
+    """What a trajectory gradient leaves reserved for the next call does not grow with the number of
+    replica groups, which take it in turn: six groups of one replica hold less than twice what
+    one replica alone does (and 64 MiB, the allocator's rounding); closing the handle gives it back."""
+    import torch
+    s = load(golden_inputs(), "small")
+
+    def held(replicas):
+        e = Engine([s] * replicas, precision=PREC_MIXED, groups=replicas)
+        e.populate_lists()
+        e.sync()
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        for _ in range(2):
+            e.traj_grad(80, 40, {"x": np.ones(sum(e.n))})
+        torch.cuda.synchronize()
+        left = free - torch.cuda.mem_get_info()[0]
+        e.close()
+        return left, torch.cuda.mem_get_info()[0] - free
+
+    held(1)  # modules loaded
+    one, six = held(1), held(6)
+    assert six[0] < 2 * one[0] + (64 << 20), (one, six)
+    assert min(one[1], six[1]) >= 0  # the handle's own memory came back too
