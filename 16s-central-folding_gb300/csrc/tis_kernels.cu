@@ -944,15 +944,35 @@ __device__ __forceinline__ long long shift_fix(const RepParams *R, int c, double
     return (int)hi < 0 ? -(long long)v : (long long)v;
 }
 
-// x + s for the shift s = S units of axis c
+// the recentring shift: s, and where positions are summed by integers (I) the same as fix units
 template <bool I>
-__device__ __forceinline__ double axis_add(const RepParams *R, int c, double x, double s, long long S)
+struct Shift {
+    double s[3];
+    __device__ __forceinline__ void set(const RepParams *, int c, double v) { s[c] = v; }
+};
+template <>
+struct Shift<true> {
+    double s[3];
+    long long fix[3];
+    __device__ __forceinline__ void set(const RepParams *R, int c, double v)
+    {
+        s[c] = v;
+        fix[c] = shift_fix(R, c, v);
+    }
+};
+
+// x + the shift of axis c
+template <bool I>
+__device__ __forceinline__ double axis_add(const RepParams *R, int c, double x, const Shift<I> &sh)
 {
-    if (!I) return x + s;
-    unsigned long long v;
-    const bool ok = axis_fix(R, c, x, v) && S != kNoShift;
-    v += (unsigned long long)S;
-    return ok && v >= (1ull << 54) ? axis_value(R, c, v) : x + s;
+    if constexpr (!I) return x + sh.s[c];
+    else {
+        unsigned long long v;
+        const long long S = sh.fix[c];
+        const bool ok = axis_fix(R, c, x, v) && S != kNoShift;
+        v += (unsigned long long)S;
+        return ok && v >= (1ull << 54) ? axis_value(R, c, v) : x + sh.s[c];
+    }
 }
 
 // x as a float, its significand cut to 24 bits (0 below 2^-126, huge from 2^128 on)
@@ -1857,21 +1877,20 @@ __device__ void write_frame(const Dev &d, int r, long long klok, int tid, int nt
 }
 
 // move_rigid_units for particle p of replica r after its leap-frog (xn, vn; the recentring
-// shift sh, shf in fixed units when I, the ions' periodic wrap, the new fixed-point position,
+// shift sh, the ions' periodic wrap, the new fixed-point position,
 // its force sum zeroed); xo: its old position, moved alike.  The centre bead's new state goes to `hold` when given
 // (a replica's place in Dev::centre) instead of the arrays, from which other blocks still
 // form the shift.
 template <bool D, bool I>
-__device__ __forceinline__ void move_particle(const Dev &d, const RepParams *R, int p, int4 q, const double sh[3],
-                                              const long long shf[3], double xn[3], const double vn[3], double xo[3],
-                                              double *hold, int &err)
+__device__ __forceinline__ void move_particle(const Dev &d, const RepParams *R, int p, int4 q, const Shift<I> &sh,
+                                              double xn[3], const double vn[3], double xo[3], double *hold, int &err)
 {
     xo[0] = d.x[p];
     xo[1] = d.y[p];
     xo[2] = d.z[p];
     for (int c = 0; c < 3; ++c) {
-        xn[c] = axis_add<I>(R, c, xn[c], sh[c], shf[c]);
-        xo[c] = axis_add<I>(R, c, xo[c], sh[c], shf[c]);
+        xn[c] = axis_add<I>(R, c, xn[c], sh);
+        xo[c] = axis_add<I>(R, c, xo[c], sh);
     }
     if (p - R->p0 >= R->nrna) {  // periodic wrap of the ions (E:2676-2731)
         for (int c = 0; c < 3; ++c) {
@@ -1997,9 +2016,8 @@ __global__ void __launch_bounds__(T + E) k_integrate(Dev d, int tail)
     const RepParams *R = d.rp + r;
     __shared__ int s_est;
     __shared__ int s_last;
-    __shared__ double s_shift[3];
-    __shared__ long long s_shf[3];
     constexpr bool I = T == kBlock;  // axis_fix
+    __shared__ Shift<I> s_shift;
     if (threadIdx.x == 0) s_est = 0;
     int err = 0;
     float2 est = make_float2(0.0f, 0.0f);
@@ -2013,14 +2031,11 @@ __global__ void __launch_bounds__(T + E) k_integrate(Dev d, int tail)
     if (E == 0 ? threadIdx.x < 32 : threadIdx.x >= T) {
         const int lane = (int)threadIdx.x & 31;
         const double s = shift_lane<D>(d, R, r, lane);
-        if (lane < 3) {
-            s_shift[lane] = s;
-            if (I) s_shf[lane] = shift_fix(R, lane, s);
-        }
+        if (lane < 3) s_shift.set(R, lane, s);
     }
     __syncthreads();
     double *hold = d.centre + (size_t)r * kCentre;
-    if (on) move_particle<D, I>(d, R, p, q, s_shift, s_shf, xn, vn, xo, hold, err);
+    if (on) move_particle<D, I>(d, R, p, q, s_shift, xn, vn, xo, hold, err);
     // check_shifts (E:1745-1762): max |x - x_old|^2 over the block (a NaN estimate orders above all)
     const int wm = __reduce_max_sync(kFull, on ? __float_as_int(est.x) & 0x7fffffff : 0);
     if ((threadIdx.x & 31) == 0) atomicMax(&s_est, wm);
@@ -2607,7 +2622,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_step_fused(Dev d, int step
         cluster_barrier();  // no CTA moves the centre bead before every CTA has read it
         lap(2);
         {
-            const double sh[3] = {s_shift[0], s_shift[1], s_shift[2]};
+            const Shift<false> sh = {{s_shift[0], s_shift[1], s_shift[2]}};
             unsigned long long bits = 0ull;
             const int i1 = min(npad, (rank + 1) * per);
             for (int i = rank * per + tid; i < i1; i += kFusedThreads) {
@@ -2615,7 +2630,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_step_fused(Dev d, int step
                 if (!((q.w >> 16) & 1)) continue;
                 double xn[3], vn[3], xo[3];
                 leap_frog<D, false>(d, R, r, p0 + i, xn, vn);
-                move_particle<D, false>(d, R, p0 + i, q, sh, nullptr, xn, vn, xo, nullptr, err);
+                move_particle<D, false>(d, R, p0 + i, q, sh, xn, vn, xo, nullptr, err);
                 bits = max(bits, shift_bits(xn, xo));
             }
             for (int o = 16; o > 0; o >>= 1) {
