@@ -451,15 +451,12 @@ __global__ void __launch_bounds__(kBlock) k_get_state(Dev d, double *stage, int 
 // ---------------------------------------------------------------------------
 // pair forces over the full (both-direction) neighbour lists
 // ---------------------------------------------------------------------------
-// Loads of data that the fused step kernel rewrites while it runs (positions,
-// lists) go through L2, the coherent path; the step's separate kernels read them
-// through the read-only path.
-template <bool CO, class T>
-__device__ __forceinline__ T ld_in(const T *ptr)
-{
-    if (CO) return __ldcg(ptr);
-    return __ldg(ptr);
-}
+// Loads of data that the fused step kernel rewrites while it runs (positions, lists) go
+// through L2 (__ldcg).  The step's separate kernels use plain loads: the read-only path
+// (__ldg) is for data that nothing writes while the kernel exists, and theirs, launched
+// while its predecessor drains, may exist before the last write has landed.  No
+// difference in time: step of one 346-nt replica 17.60 and 17.61 us, of 64 replicas 79.33 and
+// 79.37 us, of 16 large ones 186.0 and 185.8 us.
 
 // the replica's FP32 pair tables as the pair code reads them (shared memory copies)
 struct PairTables {
@@ -584,11 +581,11 @@ __device__ __forceinline__ void pair_particle(const Dev &d, const RepParams *R, 
     const float lo = R->rc2f * (1.0f - kBand), hi = R->rc2f * (1.0f + kBand);
     const float kap = R->kappaf;
     for (int k = lane4; k < cnt; k += L) {
-        const int raw = ld_in<true>(nbr + nb_idx(k, p, P));
+        const int raw = __ldcg(nbr + nb_idx(k, p, P));
         const int j = raw & kIdxMask;
         if constexpr (!D) {
             const float ljw = LR ? 1.0f : (float)(1 - (raw >> kExclShift));
-            pair_entry<LR, false>(d, R, p, qp, tp, chp, j, ld_in<true>(d.q + j), ljw, tb, kap, lo, hi, ax, ay, az, err,
+            pair_entry<LR, false>(d, R, p, qp, tp, chp, j, __ldcg(d.q + j), ljw, tb, kap, lo, hi, ax, ay, az, err,
                                   e0, e1);
         } else {
             const double ljw = LR ? 1.0 : (double)(1 - (raw >> kExclShift));
@@ -753,7 +750,7 @@ __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int 
             const int *nbr = tlr ? d.nbr_lr : d.nbr_sr;
             double ec = 0;
             if constexpr (!D) {
-                const int4 e4 = __ldg((const int4 *)nbr + (size_t)task_chunk(task) * P + p);
+                const int4 e4 = ((const int4 *)nbr)[(size_t)task_chunk(task) * P + p];
                 int raw[4] = {e4.x, e4.y, e4.z, e4.w};
                 const int4 qp = sm.q[pl];
                 const int tp = qp.w & 0xff;
@@ -762,7 +759,7 @@ __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int 
                 int4 qj[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    if (k < cnt) qj[k] = __ldg(d.q + (raw[k] & kIdxMask));
+                    if (k < cnt) qj[k] = d.q[raw[k] & kIdxMask];
                 // one copy of the entry's code, the four taking turns in its registers: the roles of
                 // this launch together overrun the instruction cache (64 replicas: 92.7 -> 87.7 us a step)
 #pragma unroll 1
@@ -783,12 +780,12 @@ __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int 
                     atomic_add_fix(out + 2 * P + p, az);
                 }
             } else {
-                const int raw = __ldg(nbr + nb_idx(task_chunk(task), p, P));
+                const int raw = nbr[nb_idx(task_chunk(task), p, P)];
                 const int wp = sm.q[pl].w;
                 const double ljw = tlr ? 0.0 : EX ? (double)(1 - (raw >> kExclShift)) : 1.0;
                 double ax = 0, ay = 0, az = 0;
                 pair_entry<false, EN>(d, R, p, wp & 0xff, is_charged((wp >> 8) & 0xff), raw & kIdxMask,
-                                      __ldg(&d.q[raw & kIdxMask].w), ljw, ax, ay, az, e_lj, ec);
+                                      d.q[raw & kIdxMask].w, ljw, ax, ay, az, e_lj, ec);
                 sm.f[0][t] = ax;
                 sm.f[1][t] = ay;
                 sm.f[2][t] = az;
@@ -2527,7 +2524,7 @@ __global__ void __launch_bounds__(128) k_pair_search(Dev d)
 //   move     each CTA integrates its share of the particles; max |x - x_old|^2
 //   control  check_shifts and the LR gate (control_step) by the first CTA
 //   rebuild  when due: cell binning by the first CTA, pair search by every warp
-// Data the kernel rewrites while it runs is read through L2 (ld_in<true>, __ldcg).
+// Data the kernel rewrites while it runs is read through L2 (__ldcg).
 constexpr int kFusedThreads = 512;
 constexpr int kFusedHbThreads = 256;
 constexpr int kFusedWarps = kFusedThreads / 32;
