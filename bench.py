@@ -159,9 +159,9 @@ class ClockSampler:
 
 def fp32_roofline(device, clocks, entries_per_launch, launch_ms):
     """The SR pairs against the FP32 roofline: their algorithmic FLOPs per launch
-    (FLOP_PER_SR_ENTRY per list entry) over the in-step duration of the force launch,
-    which holds the other force stages too, and the GPU's FP32
-    peak at the SM clock sampled during the timed region (SMs x 128 lanes x 2)."""
+    (FLOP_PER_SR_ENTRY per list entry) over the duration of a launch of the SR pairs
+    alone (in the step they share the force launch), and the GPU's FP32 peak at the SM
+    clock sampled during the timed region (SMs x 128 lanes x 2)."""
     import torch
     sms = torch.cuda.get_device_properties(device).multi_processor_count
     mhz = (clocks or {}).get("sm_mhz") or 2070.0
@@ -170,7 +170,6 @@ def fp32_roofline(device, clocks, entries_per_launch, launch_ms):
     ach = flops / (launch_ms * 1e-3) / 1e12 if launch_ms > 0 else None
     return {"kernel": "pair_sr", "alg_flops_per_launch": flops, "achieved_tflops": ach, "peak_tflops": peak,
             "unit": "TFLOP/s", "frac": ach / peak if ach is not None else None,
-            "ncu_fma_pipe_frac": NCU_FMA_PIPE.get("pair_sr"),
             "model": f"{FLOP_PER_SR_ENTRY} FLOP per SR list entry; peak at the sampled SM clock"}
 
 
@@ -214,14 +213,30 @@ def stage_bytes(n, sr, lr, lr_frac, nreb, nrna, items, nhb, nrep):
     }
 
 
+# The four kernels of a step and the stages each runs (tis_profile_stages' names).
+STEP_KERNELS = {"forces": ("pair_sr", "pair_lr", "bonded", "hbond"), "integrate": ("shift", "integrate"),
+                "cells": ("cells",), "search": ("search",)}
+
+
+def step_kernels(alg, alone, in_step, groups):
+    """Per kernel of the step: its time per launch in the step and alone (its stages one after
+    another), its algorithmic bytes per launch (one replica group, one step) and the rate
+    they give; and the name of the kernel that takes the most time in the step."""
+    out = {}
+    for name, stages in STEP_KERNELS.items():
+        us = 1000 * sum(in_step[k] for k in stages)
+        b = sum(alg[k] for k in stages) / groups
+        out[name] = {"in_step_us": us, "alone_us_per_group": 1000 * sum(alone[k] for k in stages) / groups,
+                     "alg_bytes_per_launch": b, "achieved_gbs": b / (us * 1e-6) / 1e9 if us > 0 else None}
+    return out, max(out, key=lambda k: out[k]["in_step_us"])
+
+
 # DRAM bytes per replica of each step kernel's launch: dram__bytes_read.sum +
 # dram__bytes_write.sum of one launch over a group of 5 or 6 replicas (28.7k particles;
-# cold L2, serialised) divided by 64 / 12, from the capture of profiles/ncu_step_kernels.md
-# ("pair_sr": the force launch, which holds the stages without an entry).  Scaled to the
-# batch by the number of replicas.
-NCU_DRAM_BYTES_PER_REPLICA = {"pair_sr": 3.24e6 * 12 / 64, "pair_lr": None, "bonded": None, "hbond": None,
-                              "shift": None, "integrate": 3.59e6 * 12 / 64, "cells": 0.095e6 * 12 / 64,
-                              "search": 0.063e6 * 12 / 64}
+# cold L2, serialised) divided by 64 / 12, from the capture of profiles/ncu_step_kernels.md.
+# Scaled to the batch by the number of replicas.
+NCU_DRAM_BYTES_PER_REPLICA = {"forces": 3.24e6 * 12 / 64, "integrate": 3.59e6 * 12 / 64,
+                              "cells": 0.095e6 * 12 / 64, "search": 0.063e6 * 12 / 64}
 
 
 # Algorithmic FP32 work of the SR pair kernel per list entry evaluated: the distance
@@ -233,8 +248,8 @@ FLOP_PER_SR_ENTRY = 26
 
 # FP32 (FMA) pipe and issue-slot use of each kernel from the same capture:
 # sm__pipe_fma_cycles_active and smsp__issue_active as fractions of their peaks.
-NCU_FMA_PIPE = {"pair_sr": 0.0558, "integrate": 0.0226, "cells": 0.0107, "search": 0.0143}
-NCU_ISSUE_ACTIVE = {"pair_sr": 0.189, "integrate": 0.0998, "cells": 0.0479, "search": 0.0693}
+NCU_FMA_PIPE = {"forces": 0.0558, "integrate": 0.0226, "cells": 0.0107, "search": 0.0143}
+NCU_ISSUE_ACTIVE = {"forces": 0.189, "integrate": 0.0998, "cells": 0.0479, "search": 0.0693}
 
 
 def cpu_sample(files, specs, steps, workers):
@@ -538,32 +553,21 @@ def gpu_arm(args):
         items = (len(sd["bt_kind"]) + len(sd["st3_E"]) + len(sd["st2_E"])) * N_REPLICAS
         nhb = len(sd["hb_E"]) * N_REPLICAS
         alg = stage_bytes(n_part, sr, lr, 0.1 + reb_rep / N_REPLICAS, nreb, nrna, items, nhb, N_REPLICAS)
-        inside = [k for k in in_step if not in_step[k] > 0]  # stages that run in the force launch ("pair_sr")
-        alg["pair_sr"] += sum(alg[k] for k in inside)
-        for k in inside:
-            alg[k] = 0.0
-        per_stage = {}
-        for k in in_step:
-            b = alg[k] / groups  # one launch = one replica group's kernel in one step
-            per_stage[k] = {"in_step_us": 1000 * in_step[k], "alone_us_per_group": 1000 * stages[k] / groups,
-                            "alg_bytes_per_launch": b,
-                            "achieved_gbs": b / (in_step[k] * 1e-3) / 1e9 if in_step[k] > 0 else None}
-        dom = max((k for k in stages if in_step[k] > 0), key=stages.get)  # the most time of its own (timed alone)
-        ach = per_stage[dom]["achieved_gbs"]
+        per_kernel, dom = step_kernels(alg, stages, in_step, groups)
+        ach = per_kernel[dom]["achieved_gbs"]
         traffic = NCU_DRAM_BYTES_PER_REPLICA.get(dom)
         roofline = {"bound": "latency", "axis": "hbm", "kernel": dom, "achieved": ach, "peak": peak, "unit": "GB/s",
                     "frac": ach / peak, "peak_source": peak_kind,
                     "traffic": traffic * N_REPLICAS / groups if traffic is not None else None,
-                    "alg_bytes_per_launch": per_stage[dom]["alg_bytes_per_launch"],
-                    "launch_us_in_step": per_stage[dom]["in_step_us"],
+                    "alg_bytes_per_launch": per_kernel[dom]["alg_bytes_per_launch"],
+                    "launch_us_in_step": per_kernel[dom]["in_step_us"],
                     "fp32_pipe_frac": NCU_FMA_PIPE.get(dom), "issue_active_frac": NCU_ISSUE_ACTIVE.get(dom),
-                    "fp32_pair_sr": fp32_roofline(local, clocks, sr * n_part / groups, in_step.get("pair_sr", 0.0)),
-                    "mean_neighbours": {"sr": sr, "lr": lr}, "stages": per_stage, "in_step_source": in_step_src,
+                    "fp32_pair_sr": fp32_roofline(local, clocks, sr * n_part / groups, stages["pair_sr"] / groups),
+                    "mean_neighbours": {"sr": sr, "lr": lr}, "kernels": per_kernel, "in_step_source": in_step_src,
                     "step": {"alg_bytes": sum(alg.values()),
                              "achieved_gbs": sum(alg.values()) / (ms_per_step * 1e-3) / 1e9,
                              "frac": sum(alg.values()) / (ms_per_step * 1e-3) / 1e9 / peak},
-                    "note": "kernel with the most execution time of its own (each stage timed alone, "
-                            "tis_profile_stages), timed inside the step (tis_profile_in_step: event pairs around "
+                    "note": "kernel with the most time in the step (tis_profile_in_step: event pairs around "
                             "each kernel inside the concurrently replayed graphs of all groups); one launch = one "
                             "replica group (1/" + str(groups) + " of the batch) for one step; achieved = its "
                             "algorithmic bytes / its in-step duration; bound: the kernels are latency bound "
