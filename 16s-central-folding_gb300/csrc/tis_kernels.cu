@@ -204,7 +204,7 @@ __device__ __forceinline__ void bond_apply(const BondGeom<D> &g, Acc<D> &A, int 
 // theta) / sin theta; this is the same vector, 2 k0 (theta0 - theta) d theta/dx,
 // with d theta/dx1 = a x w / (|a|^2 |w|), d theta/dx3 = -b x w / (|b|^2 |w|),
 // w = a x b, which keeps FP32 accurate where sin theta is small.
-template <bool D>
+template <bool D, bool ROLL = true>
 __device__ __forceinline__ void angle_apply(const AngleGeom<D> &g, Acc<D> &A, int i1, int i2, int i3, Real<D> k0,
                                             Real<D> th0, bool clamp)
 {
@@ -215,9 +215,11 @@ __device__ __forceinline__ void angle_apply(const AngleGeom<D> &g, Acc<D> &A, in
     const V3<R> g1 = (s / g.aa) * cross(g.a, g.w);
     const V3<R> g3 = (-s / g.bb) * cross(g.b, g.w);
     // a loop, so that the beads share one copy of the fixed-point sum's code (instruction cache:
-    // step of one 346-nt replica 19.5 -> 19.2 us, drop-in 50.6 -> 48.9 us, with the dihedral's)
+    // step of one 346-nt replica 19.5 -> 19.2 us, drop-in 50.6 -> 48.9 us, with the dihedral's);
+    // ROLL false, a copy each, in the persistent kernel's six-term restraints (six_force: one
+    // 60-nt replica on one CTA 98.4 -> 93.1 us a step, 64 of 203 nt 301 -> 293 us)
     V3<R> f = g1, f2 = R(-1) * (g1 + g3), f3 = g3;
-#pragma unroll 1
+#pragma unroll (ROLL ? 1 : 3)
     for (int k = 0; k < 3; ++k) {
         A.add(i1, f);
         f = f2; f2 = f3;
@@ -231,7 +233,7 @@ __device__ __forceinline__ void angle_apply(const AngleGeom<D> &g, Acc<D> &A, in
 // d psi/dx1 = -|v2| m / |m|^2, d psi/dx4 = |v2| n / |n|^2,
 // d psi/dx2 = -(1 + v1.v2/|v2|^2) d psi/dx1 + (v3.v2/|v2|^2) d psi/dx4,
 // which has no 1/sin psi and so no FP32 cancellation at planar (psi ~ 0, pi) geometry.
-template <bool D>
+template <bool D, bool ROLL = true>
 __device__ __forceinline__ void dihedral_apply(const DihedralGeom<D> &g, Acc<D> &A, int i1, int i2, int i3, int i4,
                                                Real<D> k0, Real<D> psi0)
 {
@@ -242,7 +244,7 @@ __device__ __forceinline__ void dihedral_apply(const DihedralGeom<D> &g, Acc<D> 
     const V3<R> g4 = (c * g.l2 / g.nn) * g.n;
     const V3<R> g2 = (R(-1) - g.p) * g1 + g.q * g4;
     V3<R> f = g1, f2 = g2, f3 = R(-1) * (g1 + g2 + g4), f4 = g4;
-#pragma unroll 1
+#pragma unroll (ROLL ? 1 : 4)
     for (int k = 0; k < 4; ++k) {
         A.add(i1, f);
         f = f2; f2 = f3; f3 = f4;
@@ -256,16 +258,16 @@ __device__ void bond_force(const Pos<D> &P, Acc<D> &A, int i1, int i2, Real<D> k
     bond_apply<D>(bond_geom<D>(P, i1, i2), A, i1, i2, k0, r0);
 }
 
-template <bool D>
+template <bool D, bool ROLL = true>
 __device__ void angle_force(const Pos<D> &P, Acc<D> &A, int i1, int i2, int i3, Real<D> k0, Real<D> th0, bool clamp)
 {
-    angle_apply<D>(angle_geom<D>(P, i1, i2, i3), A, i1, i2, i3, k0, th0, clamp);
+    angle_apply<D, ROLL>(angle_geom<D>(P, i1, i2, i3), A, i1, i2, i3, k0, th0, clamp);
 }
 
-template <bool D>
+template <bool D, bool ROLL = true>
 __device__ void dihedral_force(const Pos<D> &P, Acc<D> &A, int i1, int i2, int i3, int i4, Real<D> k0, Real<D> psi0)
 {
-    dihedral_apply<D>(dihedral_geom<D>(P, i1, i2, i3, i4), A, i1, i2, i3, i4, k0, psi0);
+    dihedral_apply<D, ROLL>(dihedral_geom<D>(P, i1, i2, i3, i4), A, i1, i2, i3, i4, k0, psi0);
 }
 
 // native dihedral imaged to within pi of the current one (E:1999-2019): branch -1/0/+1
@@ -311,11 +313,11 @@ __device__ void six_force(const Pos<D> &P, Acc<D> &A, const int *k, const double
     using R = Real<D>;
     int b0 = code % 3 - 1, b1 = (code / 3) % 3 - 1, b2 = code / 9 - 1;
     bond_force<D>(P, A, k[1], k[4], R(5) * w, (R)nat[0]);
-    angle_force<D>(P, A, k[0], k[1], k[4], R(1.5) * w, (R)nat[1], true);
-    angle_force<D>(P, A, k[3], k[4], k[1], R(1.5) * w, (R)nat[2], true);
-    dihedral_force<D>(P, A, k[0], k[1], k[4], k[3], R(0.15) * w, psi_shift<R>((R)nat[3], b0));
-    dihedral_force<D>(P, A, k[4], k[1], k[0], k[2], R(0.15) * w, psi_shift<R>((R)nat[4], b1));
-    dihedral_force<D>(P, A, k[1], k[4], k[3], k[5], R(0.15) * w, psi_shift<R>((R)nat[5], b2));
+    angle_force<D, false>(P, A, k[0], k[1], k[4], R(1.5) * w, (R)nat[1], true);
+    angle_force<D, false>(P, A, k[3], k[4], k[1], R(1.5) * w, (R)nat[2], true);
+    dihedral_force<D, false>(P, A, k[0], k[1], k[4], k[3], R(0.15) * w, psi_shift<R>((R)nat[3], b0));
+    dihedral_force<D, false>(P, A, k[4], k[1], k[0], k[2], R(0.15) * w, psi_shift<R>((R)nat[4], b1));
+    dihedral_force<D, false>(P, A, k[1], k[4], k[3], k[5], R(0.15) * w, psi_shift<R>((R)nat[5], b2));
 }
 
 // The beads of term s of the six-term restraint, as places in its six (1-2: an angle's
@@ -466,7 +468,9 @@ struct PairTables {
 // The force of one list entry (partner j, packed position qj, ljw: the weight of its LJ
 // term) on the particle p of type tp: mixed precision, added to (ax, ay, az) in fixed
 // point.  An LR entry has no LJ term (LR_interactions_lists, E:1851-1907), however far its
-// pair is: LR known, or a weight of zero.
+// pair is: LR known, or a weight of zero.  Each term takes its own root: leaving before a
+// common one where neither applies cost the persistent kernel up to 8% (FP64, one 76-nt
+// replica on one CTA: 399 -> 436 us a step) and gave the force launch nothing.
 template <bool LR, bool EN>
 __device__ __forceinline__ void pair_entry(const Dev &d, const RepParams *R, int p, const int4 &qp, int tp, bool chp,
                                            int j, const int4 &qj, float ljw, const PairTables &tb, float kap, float lo,
@@ -482,10 +486,9 @@ __device__ __forceinline__ void pair_entry(const Dev &d, const RepParams *R, int
     const bool lj = !LR && ljw != 0.0f && r2 <= tb.dlj2[J];
     bool cou = (LR || (chp && is_charged(kj))) && r2 <= hi;
     if (cou && !(r2 <= lo)) cou = exact_r2(d, R, p, j) <= R->rc2;
-    if (!lj && !cou) return;
-    const float rr = sqrtf(r2);
     float F = 0.0f;
     if (lj) {  // LJ_FORCE (E:801-821)
+        const float rr = sqrtf(r2);
         const float dr = rr - tb.dm[J];
         const float s = 1.5852f / dr;
         const float s2 = s * s, s4 = s2 * s2, s8 = s4 * s4, s14 = s8 * s4 * s2;
@@ -501,6 +504,7 @@ __device__ __forceinline__ void pair_entry(const Dev &d, const RepParams *R, int
         }
     }
     if (cou) {  // COULOMB_TRUNCATED_FORCE (E:841-855)
+        const float rr = sqrtf(r2);
         if (kap == 0.0f) {
             F += tb.qclb[J] / (r2 * rr);
             if (EN) e_c += 0.5 * (double)(tb.qclb[J] / rr);
@@ -529,10 +533,9 @@ __device__ __forceinline__ void pair_entry(const Dev &d, const RepParams *R, int
     const double r2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
     const bool lj = !LR && ljw != 0.0 && r2 <= R->dlj2_d[J];
     const bool cou = (LR || (chp && is_charged(kj))) && r2 <= R->rc2;
-    if (!lj && !cou) return;
-    const double rr = sqrt(r2);
     double F = 0.0;
     if (lj) {
+        const double rr = sqrt(r2);
         const double dr = rr + kSig0 - R->dlj_d[J];
         const double s = kSig0 / dr;
         const double s2 = s * s, s4 = s2 * s2, s8 = s4 * s4, s14 = s8 * s4 * s2;
@@ -548,6 +551,7 @@ __device__ __forceinline__ void pair_entry(const Dev &d, const RepParams *R, int
         }
     }
     if (cou) {
+        const double rr = sqrt(r2);
         if (R->kappa == 0.0) {
             F += R->qclb_d[J] / (rr * r2);
             if (EN) e_c += 0.5 * R->qclb_d[J] / rr;
