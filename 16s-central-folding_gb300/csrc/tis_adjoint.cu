@@ -22,6 +22,7 @@
 // C kappa^3 exp(-kappa r) / r with kappa = 1 / lambda_D; both vanish unscreened).
 #include <cstdio>
 
+#include "tis_fixed.cuh"
 #include "tis_kernels.cuh"
 #include "tis_tasks.cuh"
 
@@ -342,38 +343,6 @@ __device__ void block_reduce(double (&v)[NV], double *smem /* NV * 32 */)
 // and sums in FP64; comparisons and conversions between FP32 and FP64 run on integers, with
 // the same results.  Measured, 16 replicas of 5,003 particles, one reverse step: with a thread per
 // particle and ten parameter sums per pair 240 + 94 us, now 93; dU/dtheta of 64: 5.4 -> 0.44 ms.
-__device__ __forceinline__ bool le_pos(double a, double b)  // a <= b for a, b >= 0 or NaN a
-{
-    return __double_as_longlong(a) <= __double_as_longlong(b);
-}
-
-// round-to-nearest conversions by integers where both values are normal numbers
-__device__ __forceinline__ float to_float(double x)
-{
-    const int hi = __double2hiint(x), m = hi & 0x7fffffff;
-    if ((unsigned)(m - 0x38100000) < 0x0fd00000u) {  // 2^-126 <= |x| < 2^127
-        const unsigned lo = (unsigned)__double2loint(x);
-        unsigned f = __funnelshift_l(lo, (unsigned)(m - 0x38000000), 3);
-        const unsigned rest = lo & 0x1fffffffu;  // below FP32's last place; half of it is 2^28
-        f += rest > 0x10000000u || (rest == 0x10000000u && (f & 1u)) ? 1u : 0u;
-        return __uint_as_float(f | ((unsigned)hi & 0x80000000u));
-    }
-    return (float)x;
-}
-__device__ __forceinline__ double to_double(float x)
-{
-    const unsigned b = __float_as_uint(x), m = b & 0x7fffffffu;
-    if (m - 0x00800000u < 0x7f000000u) return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(b << 29));
-    return (double)x;
-}
-template <class T>
-__device__ __forceinline__ T to_real(double x)
-{
-    if constexpr (sizeof(T) == 4) return to_float(x);
-    else return x;
-}
-__device__ __forceinline__ double to_double(double x) { return x; }
-
 template <int PB, int MODE>
 struct AdjSmem {
     double x[3][PB], t[MODE ? 6 : 1][PB];  // positions; the SR and LR tangents

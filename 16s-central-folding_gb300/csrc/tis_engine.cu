@@ -11,6 +11,7 @@
 #include "tis_host.h"
 #include <nvtx3/nvToolsExt.h>
 
+#include "tis_fixed.cuh"
 #include "tis_kernels.cuh"
 
 using tis::fail;
@@ -441,32 +442,7 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
         if (rc < prm.sr) return bail(fail(TIS_ERR_ARG, "replica %d: Coulomb cutoff %g below the SR radius %g", base + r, rc, prm.sr));
         for (int k = 0; k < 3; ++k) {
             const double L = box->as<double>()[k];
-            R.box[k] = L;
-            R.hbox[k] = 0.5 * L;
-            R.qinv[k] = 4294967296.0 / L;
-            R.qstep[k] = (float)(L / 4294967296.0);
-            {
-                int e2l, eq;  // 2 L < 2^e2l, qinv < 2^eq
-                std::frexp(2.0 * L, &e2l);
-                std::frexp(R.qinv[k], &eq);
-                uint64_t bits;
-                const double l2 = 2.0 * L;
-                memcpy(&bits, &l2, 8);
-                R.qx[k].q = (unsigned long long)std::ldexp(R.qinv[k], 64 - eq);
-                R.qx[k].hi2l = (unsigned)(bits >> 32);
-                R.qx[k].sh = 1022 + e2l;
-                R.qx[k].fb = 64 - eq - e2l - 1;
-                int e;  // 1.02 L < 2^e
-                std::frexp(1.02 * L, &e);
-                const double top = 1.01 * L;
-                memcpy(&bits, &top, 8);
-                R.ax[k].lo = (unsigned)(1023 + e - 10) << 20;
-                R.ax[k].span = (unsigned)(bits >> 32) - R.ax[k].lo;
-                R.ax[k].step = std::ldexp(1.0f, e - 40);
-                const float u2 = R.ax[k].step * R.ax[k].step;
-                R.e2min = std::max(k ? R.e2min : 0.0f, 1.3e11f * u2);
-                R.e2pad = std::max(k ? R.e2pad : 1.0e-30f, 1.0e3f * u2);
-            }
+            tis::set_axis(R, k, L);
             R.mc[k] = (int)(L / (rc + prm.skin));  // E:1484-1490
             if (R.mc[k] < 1) return bail(fail(TIS_ERR_ARG, "replica %d: box smaller than the LR list radius", base + r));
             R.lcell[k] = L / R.mc[k];

@@ -13,6 +13,7 @@
 //   rebuild       populate_lists + separate_in_cells E:1461-1737, gated per replica
 #include <cstdio>
 
+#include "tis_fixed.cuh"
 #include "tis_kernels.cuh"
 #include "tis_tasks.cuh"
 
@@ -876,115 +877,6 @@ __device__ inline double total_force(const Dev &d, int p, int c)
     return (double)t * (1.0 / kFixScale);
 }
 
-// (double)v by integer operations while v fits the 53 bits of a double's significand
-// (GB300 has 64-bit conversions and FP64 arithmetic at 1/64 of its integer rate)
-__device__ __forceinline__ double fix_to_double(long long v)
-{
-    const unsigned long long m = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
-    if (m >> 53) return (double)v;
-    const int z = __clzll((long long)m);  // 11 .. 64
-    unsigned long long b = ((m << z) << 1) >> 12;  // the significand below its leading one
-    b |= (unsigned long long)(unsigned)(1086 - z) << 52;
-    if (m == 0) b = 0;
-    return __longlong_as_double((long long)(b | ((unsigned long long)v & 0x8000000000000000ull)));
-}
-
-// floor(x qinv) modulo 2^32 of axis c, as __double2ll_rd(x * qinv[c]) gives it.  For
-// 0 <= x < 2 L by integers: X = x 2^(63 - B) (2 L <= 2^B) times qinv 2^k, of which the
-// high word has fb = k - B - 1 fraction bits (28 to 30).  It lies below the exact product
-// by less than 2^-26; the FP64 product is rounded by at most 2^-21, which can only move
-// its floor when the fraction lies within 2^-20 of one: those, and other x, take the FP64 form.
-__device__ __forceinline__ int fix_position(const RepParams *R, int c, double x)
-{
-    const int hi = __double2hiint(x);
-    if ((unsigned)hi < R->qx[c].hi2l) {
-        const int s = R->qx[c].sh - (hi >> 20);
-        const unsigned long long m = ((unsigned long long)(unsigned)((hi & 0xfffff) | 0x100000) << 32 | (unsigned)__double2loint(x)) << 10;
-        const unsigned long long v = __umul64hi(s < 64 ? m >> s : 0ull, R->qx[c].q);
-        const int fb = R->qx[c].fb;
-        const unsigned fr = (unsigned)v & ((1u << fb) - 1u);
-        if (fr < (1u << fb) - (1u << (fb - 20))) return (int)(unsigned)(v >> fb);
-    }
-    return (int)(unsigned)__double2ll_rd(x * R->qinv[c]);
-}
-
-// Sums of positions by integers, rounded as FP64 rounds them.  Full blocks use them, where
-// the FP64 pipe is what the integrator waits for (twelve of its 27 operations per particle
-// become some 200 integer instructions, 56 cycles of issue for 192 of the pipe: step of 16
-// large replicas 194.1 -> 187.6 us, of 64 replicas 83.1 -> 82.5 us); a handle of few particles
-// waits for the chain of one block, which they lengthen (one replica 19.8 -> 20.6 us).
-// x in units of 2^(E - 64) (2^E > 1.02 box), exactly, for 2^(E - 10) <= x < 1.01 box
-__device__ __forceinline__ bool axis_fix(const RepParams *R, int c, double x, unsigned long long &v)
-{
-    const unsigned hi = (unsigned)__double2hiint(x), o = hi - R->ax[c].lo;
-    v = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | (unsigned)__double2loint(x)) << (((o >> 20) + 2u) & 15u);
-    return o < R->ax[c].span;
-}
-
-// the double nearest to v units, ties to even, for v >= 2^54
-__device__ __forceinline__ double axis_value(const RepParams *R, int c, unsigned long long v)
-{
-    const unsigned z = (unsigned)__clz((int)(v >> 32));  // 0 .. 9
-    const unsigned long long w = v << z;
-    const unsigned low = (unsigned)w, up = (low & 0x7ffu) + ((low >> 11) & 1u) > 0x400u;
-    return __longlong_as_double((long long)((w >> 11) + ((unsigned long long)(R->ax[c].lo + (8u << 20) - (z << 20)) << 32) + up));
-}
-
-// a shift s in the same units, rounded to odd, so that its sum with a position rounds as the
-// exact one does; kNoShift when |s| >= 2^(E - 10)
-constexpr long long kNoShift = (long long)0x8000000000000000ull;
-__device__ __forceinline__ long long shift_fix(const RepParams *R, int c, double s)
-{
-    const unsigned hi = (unsigned)__double2hiint(s), a = hi & 0x7fffffffu;
-    if (a >= R->ax[c].lo) return kNoShift;
-    if (s == 0.0) return 0;
-    const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | (unsigned)__double2loint(s)) << 1;
-    const unsigned r = (R->ax[c].lo >> 20) - 1u - (a >> 20);
-    unsigned long long v = r < 64u ? m >> r : 0ull;
-    if (r >= 64u || v << r != m) v |= 1ull;
-    return (int)hi < 0 ? -(long long)v : (long long)v;
-}
-
-// the recentring shift: s, and where positions are summed by integers (I) the same as fix units
-template <bool I>
-struct Shift {
-    double s[3];
-    __device__ __forceinline__ void set(const RepParams *, int c, double v) { s[c] = v; }
-};
-template <>
-struct Shift<true> {
-    double s[3];
-    long long fix[3];
-    __device__ __forceinline__ void set(const RepParams *R, int c, double v)
-    {
-        s[c] = v;
-        fix[c] = shift_fix(R, c, v);
-    }
-};
-
-// x + the shift of axis c
-template <bool I>
-__device__ __forceinline__ double axis_add(const RepParams *R, int c, double x, const Shift<I> &sh)
-{
-    if constexpr (!I) return x + sh.s[c];
-    else {
-        unsigned long long v;
-        const long long S = sh.fix[c];
-        const bool ok = axis_fix(R, c, x, v) && S != kNoShift;
-        v += (unsigned long long)S;
-        return ok && v >= (1ull << 54) ? axis_value(R, c, v) : x + sh.s[c];
-    }
-}
-
-// x as a float, its significand cut to 24 bits (0 below 2^-126, huge from 2^128 on)
-__device__ __forceinline__ float cut_to_float(double x)
-{
-    const int hi = __double2hiint(x), a = hi & 0x7fffffff;
-    const int f = __funnelshift_l((unsigned)__double2loint(x), (unsigned)(a - 0x38000000), 3);
-    const float m = a < 0x38100000 ? 0.0f : a >= 0x47f00000 ? 3.0e38f : __int_as_float(f);
-    return hi < 0 ? -m : m;
-}
-
 // the step's 3000 Gaussians of replica r (RepState::pending)
 __device__ __forceinline__ const double *step_noise(const Dev &d, int r)
 {
@@ -1035,22 +927,8 @@ __device__ inline void leap_frog(const Dev &d, const RepParams *R, int r, int p,
     // vanishes): then nothing (x) and an upper bound (y)
     float s = 0.0f, parts = 0.0f;
     for (int c = 0; c < 3; ++c) {
-        // 2 x0 - o0 rounded once, which is also what x0 + (x0 - o0) gives while the difference
-        // is exact: by integers while both are a usual place and the difference below 2^(E - 10)
-        unsigned long long X, O;
-        const bool in = axis_fix(R, c, x0[c], X) & axis_fix(R, c, o0[c], O);
-        const long long dif = (long long)(X - O);
-        X += (unsigned long long)dif;
-        double t;
         float a;
-        if (I && in && (unsigned long long)(dif + (1ll << 54)) < (1ull << 55) && X >= (1ull << 54)) {
-            t = axis_value(R, c, X);
-            a = (float)(int)(dif >> 24) * R->ax[c].step;
-        } else {
-            const double e = x0[c] - o0[c];
-            t = D ? __dsub_rn(__dmul_rn(2.0, x0[c]), o0[c]) : x0[c] + e;
-            a = cut_to_float(e);
-        }
+        const double t = axis_ahead<D, I>(R, c, x0[c], o0[c], a);
         const double dv = vn[c] - v0[c];
         xn[c] = D ? __dadd_rn(t, __dmul_rn(dv, R->h)) : fma(dv, R->h, t);
         const float b = cut_to_float(dv) * R->hf, e = a + b;
