@@ -734,15 +734,20 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
         // particles, few enough that the blocks of the steps without a rebuild cost little.
         // 4 / 8 / 16 per SM: 7 replicas of 3,000 particles 1.25 / 1.22 / 1.20 ms (33 steps), 64
         // of 5,400 in 12 groups 9.72 / 9.53 / 9.54 ms (100), 16 of 48,900 in 3 groups 9.6 / 8.6 /
-        // 8.2 ms (40); 64 replicas' list builds and 20 steps 2.64 / 2.66 / 2.69 ms
-        d.search_warps = std::max(4, sms * (h->P >= 100000 ? 16 : 8));
+        // 8.2 ms (40); 64 replicas' list builds and 20 steps 2.64 / 2.66 / 2.69 ms.  8 / 16 by the
+        // group's particles, a step: 32,000 (64 replicas, 12 groups) 83.9 / 84.7 us, 40,000 (40, 8)
+        // 83.4 / 84.1, 51,000 (16, 3) 66.0 / 63.7, 57,000 (5, 1) 47.1 / 45.5, 94,000 (12, 3) 93.9 / 89.6,
+        // 118,000 (8, 2) 100.6 / 94.7
+        d.search_warps = std::max(4, sms * (h->P >= 50000 ? 16 : 8));
         d.sm_count = std::max(1, sms);
         d.wide = total_blocks <= 4 * d.sm_count;
         // a block of 1024 threads takes a whole SM's registers, so each step waits for an SM that
         // runs nothing else; one of 512 fits beside a force block, but bins a replica more slowly.
         // 1024 / 512 / 256 threads: 64 replicas of 5,400 particles 8.12 / 7.98 / 8.09 ms (100 steps),
-        // their list build and 20 steps 2.32 / 2.27 / 2.30 ms, 16 of 48,900 7.43 / 7.49 / - ms (40);
-        // between the two sizes nothing was measured
+        // their list build and 20 steps 2.32 / 2.27 / 2.30 ms, 16 of 48,900 7.43 / 7.49 / - ms (40).
+        // 1024 / 512 between the two: step of 16 replicas of 7,900 57.7 / 56.8 us, of 10,200 65.9 / 66.1,
+        // of 19,600 95.8 / 96.2, of 12 of 23,600 95.3 / 96.5; list build of 24 replicas of 11,500
+        // 501 / 474 us, of 16 of 19,600 554 / 569, of 12 of 23,600 476 / 490
         int npad_max = 0;
         for (auto &Q : rp) npad_max = std::max(npad_max, Q.npad);
         d.cell_threads = npad_max <= 20000 ? 512 : 1024;
