@@ -275,8 +275,8 @@ int populate_launch(Group *h)
 {
     tis::launch_clear_err(h->dev, h->stream);
     tis::launch_force_all_rebuild(h->dev, h->stream);
-    // every replica rebuilds: the search gets six blocks of four warps per SM instead
-    // of the step's one (a warp per particle is latency-bound; more warps in flight)
+    // every replica rebuilds: the search gets six blocks of four warps per SM instead of
+    // the step's two or four (a warp per particle is latency-bound; more warps in flight)
     tis::Dev full = h->dev;
     full.search_warps = h->dev.sm_count * 24;
     tis::launch_rebuild(full, h->stream, 0);
@@ -1059,7 +1059,7 @@ static int grp_compute_forces(Group *h, int r, int mask, double *forces, double 
     TIS_CUDA(cudaMemsetAsync(d.eterm, 0, sizeof(double) * h->R * tis::kNE, h->stream));
     TIS_CUDA(cudaMemsetAsync(d.f, 0, sizeof(unsigned long long) * 3 * h->P, h->stream));
     const int m_sr = mask & TIS_TERM_SR ? 1 : 0, m_lr = mask & TIS_TERM_LR ? 2 : 0;
-    if (m_sr || m_lr) tis::launch_pair(d, h->stream, true, false, m_sr, m_lr);
+    if (m_sr || m_lr) tis::launch_pair(d, h->stream, true, m_sr, m_lr);
     if (!m_lr) TIS_CUDA(cudaMemsetAsync(d.flr, 0, sizeof(unsigned long long) * 3 * h->P, h->stream));
     const int tmask = (mask & TIS_TERM_BONDED ? 4 : 0) | (mask & TIS_TERM_STACK ? 8 : 0) | (mask & TIS_TERM_HB ? 16 : 0);
     if (tmask) tis::launch_topology(d, h->stream, tmask, true, false, false);
@@ -1478,9 +1478,9 @@ static int grp_profile_stages(Group *h, int64_t n, double *ms)
     const tis::Dev &d = h->dev;
     for (int64_t s = 0; s < n; ++s) {
         TIS_CUDA(cudaEventRecord(ev[0], h->stream));
-        tis::launch_pair(d, h->stream, false, true, 1, 0);
+        tis::launch_pair(d, h->stream, false, 1, 0);
         TIS_CUDA(cudaEventRecord(ev[1], h->stream));
-        tis::launch_pair(d, h->stream, false, true, 0, 1);
+        tis::launch_pair(d, h->stream, false, 0, 1);
         TIS_CUDA(cudaEventRecord(ev[2], h->stream));
         tis::launch_topology(d, h->stream, 4 | 8, false, false, true);
         TIS_CUDA(cudaEventRecord(ev[3], h->stream));

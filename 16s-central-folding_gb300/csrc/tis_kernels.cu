@@ -8,8 +8,11 @@
 //                 a replica per block with the valence-limited Monte Carlo (E:2145-2350),
 //                 full_forces' Gaussians (E:2590-2611)
 //   k_integrate   full_forces (application) + move_rigid_units + leap_frog_move_atom + adjust_box
-//                                             E:2612-2732, E:570-642; its last block per
-//                 replica runs check_shifts      E:1741-1776
+//                                             E:2612-2732, E:570-642
+//   k_cells       check_shifts' skin check   E:1741-1766 (the drop-in move_rigid_units, after
+//                 which a caller may look at anything, ends with it in k_integrate), the
+//                 replica's frame, and of a rebuilding replica separate_in_cells E:1461-1542
+//                 and the H-bond candidates' status E:1698-1736
 //   rebuild       populate_lists + separate_in_cells E:1461-1737, gated per replica
 #include <cstdio>
 
@@ -823,13 +826,14 @@ __device__ __forceinline__ void pair_tasks(const Dev &d, int pb, int do_sr, int 
     if (err) atomicOr(&d.rs[r].err, err);
 }
 
-// the pair forces alone (tis_compute_forces, stage timing)
+// the pair forces alone: with energies each bonded pair's LJ counts, as the reference's terms have
+// it (tis_compute_forces); without, as the step leaves it out (stage timing)
 constexpr int kPairAlone = 128;
-template <bool D, bool EN, bool EX>
+template <bool D, bool EN>
 __global__ void __launch_bounds__(kPairAlone) k_pair(Dev d, int do_sr, int do_lr)
 {
     __shared__ PairSmem<D, 32> sm;
-    pair_tasks<D, EN, EX, 32, kPairAlone>(d, blockIdx.x, do_sr, do_lr, (int)threadIdx.x, sm, CtaBar{});
+    pair_tasks<D, EN, !EN, 32, kPairAlone>(d, blockIdx.x, do_sr, do_lr, (int)threadIdx.x, sm, CtaBar{});
 }
 
 // ---------------------------------------------------------------------------
@@ -2666,17 +2670,15 @@ void launch_ion_counts(const Dev &d, cudaStream_t s, int r, int nrna, int kind, 
     k_ion_counts<<<(nrna + 3) / 4, 128, 0, s>>>(d, r, kind, r2cut, count, hit);
 }
 
-void launch_pair(const Dev &d, cudaStream_t s, bool en, bool ex, int sr, int lr)
+void launch_pair(const Dev &d, cudaStream_t s, bool en, int sr, int lr)
 {
     const int nb = d.P / 32;
     if (d.fp64) {
-        if (en) k_pair<true, true, false><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
-        else if (ex) k_pair<true, false, true><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
-        else k_pair<true, false, false><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
+        if (en) k_pair<true, true><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
+        else k_pair<true, false><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
     } else {
-        if (en) k_pair<false, true, false><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
-        else if (ex) k_pair<false, false, true><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
-        else k_pair<false, false, false><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
+        if (en) k_pair<false, true><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
+        else k_pair<false, false><<<nb, kPairAlone, 0, s>>>(d, sr, lr);
     }
 }
 

@@ -6,10 +6,10 @@
 
 namespace tis {
 
-// Frames written from inside the step (tis_frames_start): every `every` steps the
-// integrator's last block of each replica writes the replica's positions, its five
-// Energies-file values and then its step number into a ring of `depth` slots in
-// pinned, device-mapped host memory (every = 0: off).
+// Frames written from inside the step (tis_frames_start): every `every` steps each
+// replica's block of the cell kernel (the integrator's last one in the drop-in routine) writes
+// the replica's positions, its five Energies-file values and then its step number into a
+// ring of `depth` slots in pinned, device-mapped host memory (every = 0: off).
 struct FrameRing {
     double *pos;        // depth slots of 3 x n_total doubles: x, y, z of every replica end to end
     double *en;         // depth slots of 5 x R_total doubles
@@ -146,9 +146,9 @@ void launch_ion_counts(const Dev &d, cudaStream_t s, int r, int nrna, int kind, 
 // does not subtract it in the bonded kernel (the reference's net force, without
 // the cancellation of two large equal terms); false gives the reference's
 // per-term split (tis_compute_forces).
-// sr: 1 with the SR lists; lr: the LR lists never (0), of the replicas whose refresh is
-// due (1), of all replicas (2)
-void launch_pair(const Dev &d, cudaStream_t s, bool energies, bool excl_in_list, int sr, int lr);
+// launch_pair: with energies the latter, else the former; sr: 1 with the SR lists; lr: the LR
+// lists never (0), of the replicas whose refresh is due (1), of all replicas (2)
+void launch_pair(const Dev &d, cudaStream_t s, bool energies, int sr, int lr);
 // the step's forces in one launch; noise: its Gaussians too
 void launch_forces(const Dev &d, cudaStream_t s, bool noise);
 void launch_topology(const Dev &d, cudaStream_t s, int mask, bool energies, bool make_noise, bool excl_in_list);

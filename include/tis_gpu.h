@@ -285,7 +285,7 @@ int tis_density_destroy(tis_density *g);
 /* Frames written from inside the step (the reference writes its output every
  * 10^6 steps from the run loop, E:6276-6376, stopping the run to do it).  After
  * tis_frames_start, every `every` steps (step numbers, klok, that are multiples of
- * it) the step's own integrator kernel writes each replica's positions, its five
+ * it) the step's own cell kernel writes each replica's positions, its five
  * Energies-file values (E2_HB, E3_HB, E2_STACK, E3_STACK, Rg) and then the step
  * number into a ring of `depth` (>= 2) slots of pinned host memory that the GPU
  * writes directly; it adds no launch and no synchronisation to the run, graphs
@@ -337,7 +337,9 @@ int tis_replica_size(tis_handle *h, int replica, int *n_particles);
  * between them, on each group's stream; ms[TIS_N_STAGES] receives the mean
  * duration per step, summed over the replica groups, of: SR pair forces, LR pair
  * forces, bonded + stacking terms, H-bonds + the step's Gaussians, recentring
- * shift, integrator, cell binning (+ skin check), pair search. */
+ * shift (0: part of the integrator), integrator, cell binning (+ skin check), pair
+ * search.  The first four are launches of their own here; the step runs them in one,
+ * whose time tis_profile_in_step gives. */
 #define TIS_N_STAGES 8
 int tis_profile_stages(tis_handle *h, int64_t n, double *ms);
 
