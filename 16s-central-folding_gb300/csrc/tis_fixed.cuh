@@ -167,9 +167,10 @@ __device__ __forceinline__ double axis_ahead(const RepParams *R, int c, double x
     return D ? __dsub_rn(__dmul_rn(2.0, x0), o0) : x0 + e;
 }
 
-__device__ __forceinline__ bool le_pos(double a, double b)  // a <= b for a, b >= 0 or NaN a
+// a <= b for b >= 0 and an a that is not negative or is NaN, of either sign
+__device__ __forceinline__ bool le_pos(double a, double b)
 {
-    return __double_as_longlong(a) <= __double_as_longlong(b);
+    return (unsigned long long)__double_as_longlong(a) <= (unsigned long long)__double_as_longlong(b);
 }
 
 // round-to-nearest conversions by integers where both values are normal numbers

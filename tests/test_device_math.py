@@ -150,3 +150,43 @@ def test_integer_forms_give_the_bits_of_the_fp64_operations(tmp_path):
     out = subprocess.run([exe] + [str(b) for b in BOXES], check=True, capture_output=True, text=True).stdout.split()
     assert dict(zip(FUNCTIONS, map(int, out))) == dict.fromkeys(FUNCTIONS, 0)
     assert int(out[-1]) > 64 * 64 * 256 * len(BOXES) // 3  # sums taken by integers
+
+
+NAN_PROGRAM = r"""
+#include <cstdio>
+#include "tis_fixed.cuh"
+
+// b[i]: with each b, NaNs of both signs, quiet and signalling, and the one inf - inf gives
+__global__ void check(const double *b, int n, double inf, int *le)
+{
+    const unsigned long long bits[4] = {0x7ff8000000000000ull, 0xfff8000000000000ull, 0x7ff0000000000001ull, 0xffffffffffffffffull};
+    for (int i = 0; i < n; ++i) {
+        for (int k = 0; k < 4; ++k) *le += tis::le_pos(__longlong_as_double((long long)bits[k]), b[i]);
+        *le += tis::le_pos(inf - inf, b[i]);
+    }
+}
+
+int main()
+{
+    const double b[6] = {0.0, 4.9e-324, 1.0, 900.0, 1.7976931348623157e308, 1.0 / 0.0};
+    double *d;
+    int *le, h = -1;
+    if (cudaMalloc(&d, sizeof b) != cudaSuccess || cudaMalloc(&le, sizeof h) != cudaSuccess) return 1;
+    cudaMemcpy(d, b, sizeof b, cudaMemcpyHostToDevice);
+    cudaMemset(le, 0, sizeof h);
+    check<<<1, 1>>>(d, 6, 1.0 / 0.0, le);
+    if (cudaMemcpy(&h, le, sizeof h, cudaMemcpyDeviceToHost) != cudaSuccess) return 2;
+    printf("%d\n", h);
+    return 0;
+}
+"""
+
+
+@pytest.mark.gpu
+def test_a_distance_that_is_no_number_is_within_no_cutoff(tmp_path):
+    src, exe = str(tmp_path / "t.cu"), str(tmp_path / "t")
+    with open(src, "w") as f:
+        f.write(NAN_PROGRAM)
+    subprocess.run([build.NVCC, "-std=c++17", "-O3", *build.ARCH, "-I", build.CSRC, src, "-o", exe], check=True,
+                   capture_output=True, text=True)
+    assert subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split() == ["0"]
