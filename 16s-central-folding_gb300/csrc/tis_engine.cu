@@ -93,6 +93,7 @@ int64_t scalar_i64(const tis_system *s, const char *name, int64_t def)
 }
 
 int round_up(int v, int m) { return (v + m - 1) / m * m; }
+inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 // an NVTX range around one API call (header-only NVTX; no cost without a profiler)
 struct Range {
@@ -127,10 +128,12 @@ struct Group {
     int npk = 0;              // particles of the group's replicas (unpadded)
     double *stage = nullptr;  // nine packed arrays of npk values (tis_traj_grad's seeds and state adjoints)
     double *d_e5 = nullptr;   // five energies per replica (tis_get_all_energies)
-    tis::RepState *h_rs = nullptr;  // pinned host copy of the replicas' state (error flags, list build checks)
-    char *h_out = nullptr;          // pinned memory for a replica's forces or ion counts, made by the first
-    size_t h_out_bytes = 0;         // call that reads them (pinned_out)
-    int *h_peaks = nullptr;         // pinned: largest SR and LR neighbour counts of the last list build
+    // pinned host memory, one allocation (h_rs is its start): the replicas' state (error flags, list
+    // build checks), the largest SR and LR neighbour counts of the last list build, and a
+    // replica's energies and forces or its ion counts
+    tis::RepState *h_rs = nullptr;
+    int *h_peaks = nullptr;
+    double *h_out = nullptr;
     int *d_peaks = nullptr;
     // parameter-derivative coefficients (tis_param_grad, tis_traj_grad)
     double *a_st2_dss = nullptr, *a_hb_dhs = nullptr;
@@ -151,8 +154,6 @@ struct Group {
         for (cudaEvent_t e : adj_event)
             if (e) cudaEventDestroy(e);
         if (h_rs) cudaFreeHost(h_rs);
-        if (h_out) cudaFreeHost(h_out);
-        if (h_peaks) cudaFreeHost(h_peaks);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -185,23 +186,6 @@ int check_flags(Group *h)
     if (rc) return rc;
     TIS_CUDA(cudaStreamSynchronize(h->stream));
     return flags_verdict(h);
-}
-
-// pinned memory for results of `bytes`, kept with the group (at most a replica's forces)
-int pinned_out(Group *h, size_t bytes, char **out)
-{
-    if (bytes > h->h_out_bytes) {
-        if (h->h_out) cudaFreeHost(h->h_out);
-        h->h_out = nullptr;
-        h->h_out_bytes = 0;
-        if (cudaMallocHost((void **)&h->h_out, bytes) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(TIS_ERR_NOMEM, "cudaMallocHost(%zu bytes) failed", bytes);
-        }
-        h->h_out_bytes = bytes;
-    }
-    *out = h->h_out;
-    return TIS_OK;
 }
 
 void enqueue_step(Group *h);
@@ -888,9 +872,18 @@ static int grp_create(const tis_system *const *systems, int n_replicas, const ti
         d.hb_smem = smem <= 160 * 1024 ? (int)smem : 0;
     }
     if (tis::configure_kernels(d) != 0) return bail(fail(TIS_ERR_CUDA, "cudaFuncSetAttribute failed"));
-    if (cudaMallocHost((void **)&h->h_rs, sizeof(tis::RepState) * h->R) != cudaSuccess ||
-        cudaMallocHost((void **)&h->h_peaks, 2 * sizeof(int)) != cudaSuccess)
-        return bail(fail(TIS_ERR_NOMEM, "cudaMallocHost failed"));
+    {
+        int n_max = 0;
+        for (const RepHost &hr : h->rep) n_max = std::max(n_max, hr.n);
+        const size_t rs_bytes = align256(sizeof(tis::RepState) * h->R), peaks = align256(2 * sizeof(int));
+        const size_t out = sizeof(double) * (tis::kNE + 1 + 3 * (size_t)n_max);  // ion counts: at most two ints per particle
+        char *pin = nullptr;
+        if (cudaMallocHost((void **)&pin, rs_bytes + peaks + out) != cudaSuccess)
+            return bail(fail(TIS_ERR_NOMEM, "cudaMallocHost failed"));
+        h->h_rs = (tis::RepState *)pin;
+        h->h_peaks = (int *)(pin + rs_bytes);
+        h->h_out = (double *)(pin + rs_bytes + peaks);
+    }
     // the allocations' memsets and the pageable uploads above run on the legacy
     // default stream, which the group's non-blocking streams do not wait for
     if (cudaDeviceSynchronize() != cudaSuccess) return bail(fail(TIS_ERR_CUDA, "device synchronisation failed"));
@@ -1006,13 +999,11 @@ static int grp_ion_counts(Group *h, int r, int kind, double radius, int32_t *cou
         return fail(TIS_ERR_ARG, "tis_ion_counts: radius %g outside (0, %g] (the SR radius)", radius, h->prm.sr);
     if (!h->lists_built && (rc = populate(h))) return rc;
     const RepHost &hr = h->rep[r];
-    char *pin = nullptr;
-    if ((rc = pinned_out(h, sizeof(int) * (hr.nrna + hr.n), &pin))) return rc;
     int *d_cnt = (int *)h->stage, *d_hit = d_cnt + hr.nrna;  // the stage holds nine doubles per particle
     TIS_CUDA(cudaMemsetAsync(d_hit, 0, sizeof(int) * hr.n, h->stream));
     tis::launch_ion_counts(h->dev, h->stream, r, hr.nrna, kind, radius * radius, d_cnt, d_hit);
-    const int *c = (const int *)pin;
-    TIS_CUDA(cudaMemcpyAsync(pin, d_cnt, sizeof(int) * (hr.nrna + hr.n), cudaMemcpyDeviceToHost, h->stream));
+    const int *c = (const int *)h->h_out;
+    TIS_CUDA(cudaMemcpyAsync(h->h_out, d_cnt, sizeof(int) * (hr.nrna + hr.n), cudaMemcpyDeviceToHost, h->stream));
     if ((rc = flags_copy(h))) return rc;
     TIS_CUDA(cudaStreamSynchronize(h->stream));
     int64_t np = 0;
@@ -1052,9 +1043,7 @@ static int grp_compute_forces(Group *h, int r, int mask, double *forces, double 
     const RepHost &hr = h->rep[r];
     // energies, Rg, then the forces
     const size_t n3 = forces ? 3 * (size_t)hr.n : 0;
-    char *pin = nullptr;
-    if ((rc = pinned_out(h, sizeof(double) * (tis::kNE + 1 + n3), &pin))) return rc;
-    double *out = (double *)pin;
+    double *out = h->h_out;
     tis::launch_clear_err(d, h->stream);
     TIS_CUDA(cudaMemsetAsync(d.eterm, 0, sizeof(double) * h->R * tis::kNE, h->stream));
     TIS_CUDA(cudaMemsetAsync(d.f, 0, sizeof(unsigned long long) * 3 * h->P, h->stream));
@@ -1167,8 +1156,6 @@ std::vector<std::pair<void *, size_t>> step_state(const Group *h)
     v.emplace_back(d.hb_active, 4 * (size_t)h->nhb_all);
     return v;
 }
-
-inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 constexpr size_t kAdjKeep = (size_t)4 << 30;    // memory a handle keeps between tis_traj_grad calls, at most
 constexpr size_t kAdjSecond = (size_t)8 << 30;  // recorded steps of one segment up to which a second set is taken
