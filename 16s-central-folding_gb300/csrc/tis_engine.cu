@@ -1160,24 +1160,29 @@ std::vector<std::pair<void *, size_t>> step_state(const Group *h)
 constexpr size_t kAdjKeep = (size_t)4 << 30;    // memory a handle keeps between tis_traj_grad calls, at most
 constexpr size_t kAdjSecond = (size_t)8 << 30;  // recorded steps of one segment up to which a second set is taken
 
-// The device memory of one group's part of a tis_traj_grad call, from the handle's pool: the
-// groups run one after another, so each takes the memory of the one before it, and what
-// the pool keeps between calls is bounded (kAdjKeep) and, unused, the driver's to take back
+// The device memory of one group's part of a tis_traj_grad call.  Up to kAdjKeep it comes from the
+// handle's pool: the groups run one after another, so each takes the memory of the one before
+// it, and what the pool keeps between calls is bounded and, unused, the driver's to take back
 // for another allocation of the process (measured: 2 GiB more with 1 GiB free).  40 steps of 12
-// replicas of 5,003 particles (3.5 GiB) take 10.0 ms, 16 when the pool is new; with memory taken
-// and freed by each call 12.0 ms.
+// replicas of 5,003 particles (3.5 GiB) take 10.0 ms, 13.5 when the pool is new (it maps 1.2 GiB
+// a ms); with memory taken and freed by each call 12.0 ms.  A larger block, of which nothing is
+// kept, comes from cudaMalloc and goes back by cudaFree, 0.15 and 1.3 ms for 3.5 GiB where the pool's
+// take 2.9 and 5.2 ms: 200 steps of 16 replicas (5 GiB) 59.0 -> 50.6 ms.
 struct AdjBlock {
     Group *h;
     cudaMemPool_t pool;
     char *mem = nullptr;
+    bool pooled = true;
     AdjBlock(Group *g, cudaMemPool_t p) : h(g), pool(p) {}
     AdjBlock(const AdjBlock &) = delete;
     cudaError_t take(size_t bytes)
     {
+        pooled = bytes <= kAdjKeep;
         uint64_t held = 0;
         cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held);
-        if (held < bytes) cudaMemPoolTrimTo(pool, 0);  // nothing too small is held beside it
-        const cudaError_t e = cudaMallocFromPoolAsync((void **)&mem, bytes, pool, h->stream);
+        if (!pooled || held < bytes) cudaMemPoolTrimTo(pool, 0);  // nothing too small is held beside it
+        const cudaError_t e = pooled ? cudaMallocFromPoolAsync((void **)&mem, bytes, pool, h->stream)
+                                     : cudaMalloc((void **)&mem, bytes);
         if (e == cudaSuccess) return e;
         mem = nullptr;
         cudaGetLastError();
@@ -1187,8 +1192,9 @@ struct AdjBlock {
     {
         if (!mem) return;
         for (cudaStream_t s : h->adj_stream) cudaStreamSynchronize(s);
-        cudaFreeAsync(mem, h->stream);
-        cudaStreamSynchronize(h->stream);  // more than kAdjKeep goes back here
+        if (pooled) cudaFreeAsync(mem, h->stream);
+        cudaStreamSynchronize(h->stream);
+        if (!pooled) cudaFree(mem);
     }
 };
 
