@@ -1167,7 +1167,7 @@ constexpr size_t kAdjSecond = (size_t)8 << 30;  // recorded steps of one segment
 // replicas of 5,003 particles (3.5 GiB) take 10.0 ms, 13.5 when the pool is new (it maps 1.2 GiB
 // a ms); with memory taken and freed by each call 12.0 ms.  A larger block, of which nothing is
 // kept, comes from cudaMalloc and goes back by cudaFree, 0.15 and 1.3 ms for 3.5 GiB where the pool's
-// take 2.9 and 5.2 ms: 200 steps of 16 replicas (5 GiB) 59.0 -> 50.6 ms.
+// take 2.9 and 5.2 ms: 200 steps of 16 of them 59.0 -> 50.6 ms.
 struct AdjBlock {
     Group *h;
     cudaMemPool_t pool;

@@ -235,8 +235,8 @@ def step_kernels(alg, alone, in_step, groups):
 # dram__bytes_write.sum of one launch over a group of 5 or 6 replicas (28.7k particles;
 # cold L2, serialised) divided by 64 / 12, from the capture of profiles/ncu_step_kernels.md.
 # Scaled to the batch by the number of replicas.
-NCU_DRAM_BYTES_PER_REPLICA = {"forces": 3.24e6 * 12 / 64, "integrate": 3.59e6 * 12 / 64,
-                              "cells": 0.095e6 * 12 / 64, "search": 0.063e6 * 12 / 64}
+NCU_DRAM_BYTES_PER_REPLICA = {"forces": 2.98e6 * 12 / 64, "integrate": 3.58e6 * 12 / 64,
+                              "cells": 0.091e6 * 12 / 64, "search": 0.058e6 * 12 / 64}
 
 
 # Algorithmic FP32 work of the SR pair kernel per list entry evaluated: the distance
@@ -248,8 +248,8 @@ FLOP_PER_SR_ENTRY = 26
 
 # FP32 (FMA) pipe and issue-slot use of each kernel from the same capture:
 # sm__pipe_fma_cycles_active and smsp__issue_active as fractions of their peaks.
-NCU_FMA_PIPE = {"forces": 0.0558, "integrate": 0.0226, "cells": 0.0107, "search": 0.0143}
-NCU_ISSUE_ACTIVE = {"forces": 0.189, "integrate": 0.0998, "cells": 0.0479, "search": 0.0693}
+NCU_FMA_PIPE = {"forces": 0.0574, "integrate": 0.0225, "cells": 0.0100, "search": 0.0130}
+NCU_ISSUE_ACTIVE = {"forces": 0.195, "integrate": 0.1006, "cells": 0.0461, "search": 0.0663}
 
 
 def cpu_sample(files, specs, steps, workers):
